@@ -33,7 +33,7 @@ def build() -> str:
 def build_reference() -> bool:
     """Compiles the reference's software backend from its own sources into
     oracle/_ref (only where the reference checkout exists)."""
-    if not os.path.isdir(REFERENCE_SRC):
+    if not os.path.isdir(os.path.join(REFERENCE_SRC, "src")):
         return False
     r = subprocess.run(["make", "-s", "-j8", "-C", os.path.join(HERE, "ref"),
                         f"REF={REFERENCE_SRC}"], capture_output=True, text=True)
