@@ -229,9 +229,14 @@ constexpr int kShortSpan = 4;
 // gradient stops a warp stages in shared memory (longer gradients are read
 // from global memory)
 constexpr int kStagedStops = 16;
-// shared memory of one compositor warp: its tile row, then the staged stops
+// shared memory of one compositor warp: its tile row, padded to 16 bytes (a
+// tile may be any number of pixels wide, the stop colours are read as
+// float4), then the staged stops
+__host__ __device__ constexpr size_t CompRowBytes(uint32_t chunk) {
+  return ((size_t)chunk * 4 + 15) & ~(size_t)15;
+}
 __host__ __device__ constexpr size_t CompWarpSmem(uint32_t chunk) {
-  return (size_t)chunk * 4 + kStagedStops * (16 + 4);
+  return CompRowBytes(chunk) + kStagedStops * (16 + 4);
 }
 
 template <bool kAll>
@@ -256,7 +261,7 @@ __global__ void __launch_bounds__(32 * kCompWarps, kCompMinBlocks)
   const int wib = threadIdx.x >> 5;
   uint8_t* mine = reg_smem + (size_t)wib * CompWarpSmem(chunk);
   uint32_t* row = (uint32_t*)mine;
-  float4* stage_colors = (float4*)(mine + (size_t)chunk * 4);
+  float4* stage_colors = (float4*)(mine + CompRowBytes(chunk));
   float* stage_offsets = (float*)(stage_colors + kStagedStops);
   if (!counter) {
     const uint32_t task = blockIdx.x * kCompWarps + wib;
