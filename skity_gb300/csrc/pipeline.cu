@@ -2106,7 +2106,7 @@ SKITY_CUDA_API int32_t skity_cuda_canvas_flush(skity_cuda_canvas canvas) {
   }
   sv.matrices = canvas->any_matrix ? canvas->matrices.data() : nullptr;
   skc::DeviceBatch& db = canvas->db;
-  db.hb = skc::HostBatch();
+  db.Reset();  // other draws than the last flush's: their passes are uploaded again
   int32_t rc = skc::AddStreamCanvas(db.hb, sv);
   if (rc) return rc;
   rc = skc::UploadBatch(ctx, db);
