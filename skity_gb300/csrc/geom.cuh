@@ -99,25 +99,45 @@ SKC_HD Fixed FixedDivWide(int32_t numer, int32_t denom) {
   if (q > kMaxS32) q = kMaxS32;
   return (Fixed)q;
 }
+SKC_HD uint32_t umulhi_(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
 // The same quotient without a 64-bit division (which the GPU runs as a long
-// called routine): for |denom| < 2^24, floor(|numer| 2^16 / |denom|) is
-// built from three 32-bit divisions giving 16 + 8 + 8 quotient bits
-// (a = q1 b + r1, 2^8 r1 = q2 b + r2, 2^8 r2 = q3 b + r3, so the quotient
-// is q1 2^16 + q2 2^8 + q3 and every partial dividend stays below 2^32),
-// then signed as C's division truncates; larger divisors take the 64-bit
-// path.  Equal to FixedDivWide for every input with denom != 0.
+// called routine): for b = |denom| < 2^24, floor(|numer| 2^16 / b) is built
+// from three digits of 16 + 8 + 8 quotient bits (a = q1 b + r1, 2^8 r1 =
+// q2 b + r2, 2^8 r2 = q3 b + r3, so the quotient is q1 2^16 + q2 2^8 + q3
+// and every partial dividend t stays below 2^32), then signed as C's division
+// truncates; larger divisors take the 64-bit path.  One division serves the
+// three digits (Barrett reduction): with v = floor((2^32 - 1) / b), t v / 2^32
+// is above t / b - 1, so its floor is t's digit or one less.  Equal to
+// FixedDivWide for every input with denom != 0.
 SKC_HD Fixed FixedDiv(int32_t numer, int32_t denom) {
   const uint32_t a = numer < 0 ? 0u - (uint32_t)numer : (uint32_t)numer;
   const uint32_t b = denom < 0 ? 0u - (uint32_t)denom : (uint32_t)denom;
-  if (b >= (1u << 24)) return FixedDivWide(numer, denom);
-  const uint32_t q1 = a / b, r1 = a - q1 * b;
-  const uint32_t t2 = r1 << 8, q2 = t2 / b, r2 = t2 - q2 * b;
-  const uint32_t q3 = (r2 << 8) / b;
-  const uint64_t u = ((uint64_t)q1 << 16) + ((uint64_t)q2 << 8) + q3;
-  int64_t q = ((numer < 0) != (denom < 0)) ? -(int64_t)u : (int64_t)u;
-  if (q < kMinS32) q = kMinS32;
-  if (q > kMaxS32) q = kMaxS32;
-  return (Fixed)q;
+  if (SKC_COLD(b >= (1u << 24))) return FixedDivWide(numer, denom);
+  const uint32_t v = 0xFFFFFFFFu / b;
+  auto digit = [&](uint32_t t, uint32_t* r) {
+    uint32_t q = umulhi_(t, v);
+    *r = t - q * b;
+    if (*r >= b) {
+      *r -= b;
+      ++q;
+    }
+    return q;
+  };
+  uint32_t r1, r2, r3;
+  const uint32_t q1 = digit(a, &r1);
+  const uint32_t q2 = digit(r1 << 8, &r2);
+  const uint32_t q3 = digit(r2 << 8, &r3);
+  const bool neg = (numer ^ denom) < 0;
+  // q1 2^16 + q2 2^8 + q3 clamped to what a Fixed holds
+  if (q1 >= (1u << 15)) return neg ? kMinS32 : kMaxS32;
+  const int32_t u = (int32_t)((q1 << 16) + (q2 << 8) + q3);
+  return neg ? -u : u;
 }
 SKC_HD int FDot6Round(FDot6 x) { return (x + 32) >> 6; }
 SKC_HD FDot6 ScalarToFDot6(float x) { return (FDot6)(x * 64); }

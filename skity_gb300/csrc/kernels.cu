@@ -105,6 +105,13 @@ __device__ __forceinline__ void FinishOverlapped(unsigned int* done) {
   }
 }
 
+// What bounds it: instruction issue.  With a step's coverage made inside the
+// step, the kernel was 140 KB of unrolled code, and instruction fetch held it
+// at 26-34 % of the issue slots; walk and emission as two short loops that
+// take turns (regsweep.cuh), one copy of each part and no unrolling are 54 KB
+// and issue 53 %, with fewer instructions a span (105 -> 73).  64 canvases of
+// 50-2,000 paths: 38 -> 15.3 ms; 256 of them: 149 -> 68.  Register caps for
+// more warps (96, 80, 64 registers) are slower: 18.9, 22.7, 27.6 ms.
 template <int M, int kForm>
 __global__ void __launch_bounds__(32 * kRegWarpsMax) k_sweep_reg(DevBatch b) {
   extern __shared__ __align__(16) uint8_t reg_smem[];

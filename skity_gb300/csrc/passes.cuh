@@ -287,6 +287,7 @@ struct PoolSinkT : SinkBase<kRawCapable> {
     if (c + chunk > cap) dead = true;
     if (!dead) {
       L.sync();
+#pragma unroll 1
       for (uint64_t i = L.lane; i < have; i += Lanes::n) pool[c + i] = pool[row_start + i];
       L.sync();
     }
@@ -296,6 +297,38 @@ struct PoolSinkT : SinkBase<kRawCapable> {
     return cur;
   }
   SKC_HD uint2* span_ptr(uint64_t i) { return dead ? nullptr : pool + i; }
+  // One span per lane (`kept`), rows in increasing order over the lanes, of
+  // `len` pixels each: appended in lane order, every row that ends among them
+  // entered in the row table, the last one left open.
+  SKC_HD void put_rows(const Lanes& L, bool kept_, uint2 v, int y, unsigned len) {
+    const unsigned km = L.ballot(kept_);
+    if (!km) return;
+    const uint32_t cnt = (uint32_t)Lanes::popc(km);
+    const uint64_t at = reserve(L, 0, cnt);
+    const unsigned below = km & L.lt_mask();
+    const uint32_t rank = (uint32_t)Lanes::popc(below);
+    uint2* dst = span_ptr(at + rank);
+    if (kept_ && dst) *dst = v;
+    const int py = LaneBcast(L, y, below ? 31 - clz_(below) : L.lane);
+    const unsigned heads = L.ballot(kept_ && (below ? py : cur_row) != y);
+    if (heads) {
+      const int first = Lanes::ffs(heads) - 1;
+      const uint64_t end = at + (uint32_t)Lanes::popc(km & ((1u << first) - 1u));
+      if (!dead) {
+        if (L.lane == first && end > row_start && cur_row >= row0 && cur_row < row1)
+          rows[cur_row - row0] = make_uint2((uint32_t)row_start, (uint32_t)(end - row_start));
+        const unsigned later = heads & ~((2u << L.lane) - 1u);
+        if (((heads >> L.lane) & 1u) && later) {
+          const uint32_t next = (uint32_t)Lanes::popc(km & ((1u << (Lanes::ffs(later) - 1)) - 1u));
+          rows[y - row0] = make_uint2((uint32_t)(at + rank), next - rank);
+        }
+      }
+      const int last = 31 - clz_(heads);
+      cur_row = LaneBcast(L, y, last);
+      row_start = at + (uint32_t)Lanes::popc(km & ((1u << last) - 1u));
+    }
+    commit(L, cnt, kept_ ? len : 0u);
+  }
   // n: spans appended (warp-uniform); f: this lane's share of their
   // fragments (the shares are summed once, when the pass finishes)
   SKC_HD void commit(const Lanes&, uint32_t n, unsigned long long f) {
@@ -303,113 +336,6 @@ struct PoolSinkT : SinkBase<kRawCapable> {
     kept += n;
     frags += f;
   }
-  // Sparse form of acc_row; returns false (nothing read, nothing written)
-  // when the row has more than ev_cap nonzero entries.
-  SKC_HD bool acc_row_sparse(const Lanes& L, int y, int32_t* diff, int left, int lo, int hi,
-                             int32_t* ev, int ev_cap) {
-    constexpr int V = 4;
-    constexpr int kNone = 0x7fffffff;
-    const bool vec = ((uintptr_t)diff & 15) == 0;
-    int ne = 0;
-    for (int base = vec ? (lo & ~(V - 1)) : lo; base < hi; base += Lanes::n * V) {
-      const int i0 = base + L.lane * V;
-      int32_t d[V];
-      if (vec && i0 + V <= hi) {
-        const int4 q = *(const int4*)(diff + i0);
-        d[0] = q.x;
-        d[1] = q.y;
-        d[2] = q.z;
-        d[3] = q.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < V; ++j) d[j] = i0 + j < hi ? diff[i0 + j] : 0;
-      }
-      int cnt = 0;
-#pragma unroll
-      for (int j = 0; j < V; ++j) cnt += d[j] != 0 ? 1 : 0;
-      if (!L.ballot(cnt != 0)) continue;
-      const int32_t incl = LaneScanIncl(L, cnt);
-      const int total = LaneBcast(L, incl, Lanes::n - 1);
-      if (SKC_COLD(ne + total > ev_cap)) return false;
-      int at = ne + incl - cnt;
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        if (d[j] != 0) {
-          ev[2 * at] = i0 + j;
-          ev[2 * at + 1] = d[j];
-          at++;
-        }
-      }
-      ne += total;
-    }
-    L.sync();
-    int open_start = -1;  // warp-uniform: the run still open after a step
-    int32_t open_v = 0;
-    int32_t carry = 0, prev_sat = 0;
-    for (int eb = 0; eb < ne; eb += Lanes::n) {
-      const int e = eb + L.lane;
-      const bool valid = e < ne;
-      int pos = kNone;
-      int32_t v = 0;
-      if (valid) {
-        pos = ev[2 * e];
-        v = ev[2 * e + 1];
-        diff[pos] = 0;
-      }
-      const int32_t incl = LaneScanIncl(L, v) + carry;
-      const int32_t sat = incl > 255 ? 255 : incl;
-      int32_t before = LaneBcast(L, sat, L.lane > 0 ? L.lane - 1 : 0);
-      if (L.lane == 0) before = prev_sat;
-      const bool start = valid && sat != before;
-      const unsigned starts = L.ballot(start);
-      const unsigned later = starts & ~((2u << L.lane) - 1u);
-      int next = (int)L.shfl((uint32_t)pos, later ? Lanes::ffs(later) - 1 : L.lane);
-      if (!later) next = kNone;
-      uint2 out[2];
-      int cnt = 0;
-      unsigned long long fr = 0;
-      auto put = [&](int s0, int w, int32_t a) {
-        int x = left + s0, len = w;
-        if (keep(x, y, len, (uint8_t)a)) {
-          out[cnt++] = pack(x, len, (uint32_t)a);
-          fr += (unsigned)len;
-        }
-      };
-      if (starts && open_start >= 0 && L.lane == Lanes::ffs(starts) - 1)
-        put(open_start, pos - open_start, open_v);
-      if (start && next != kNone && sat != 0) put(pos, next - pos, sat);
-      if (starts) {
-        const int src = 31 - clz_(starts);
-        const int32_t lv = LaneBcast(L, sat, src);
-        const int lp = LaneBcast(L, pos, src);
-        open_start = lv != 0 ? lp : -1;
-        open_v = lv;
-      }
-      const int32_t ci = LaneScanIncl(L, cnt);
-      const uint32_t total = (uint32_t)LaneBcast(L, ci, Lanes::n - 1);
-      if (total) {
-        const uint64_t at = reserve(L, 0, total);
-        uint2* dst = span_ptr(at + (uint32_t)(ci - cnt));
-        if (dst) {
-          for (int i = 0; i < cnt; ++i) dst[i] = out[i];
-        }
-        commit(L, total, fr);
-      }
-      carry = LaneBcast(L, incl, Lanes::n - 1);
-      prev_sat = LaneBcast(L, sat, Lanes::n - 1);
-    }
-    if (open_start >= 0) {
-      int x = left + open_start, len = hi - open_start;
-      if (keep(x, y, len, (uint8_t)open_v)) {
-        const uint64_t at = reserve(L, 0, 1);
-        if (!dead && L.leader())
-          pool[at] = pack(x, len, (uint32_t)open_v);
-        commit(L, 1, L.leader() ? (unsigned)len : 0u);
-      }
-    }
-    return true;
-  }
-
   // The accumulated spans of a row follow its direct spans (the reference
   // flushes a row's accumulator only after leaving the row,
   // SpanBuilder::Flush, sw_raster.cc:103-136): the runs of equal nonzero
@@ -423,17 +349,9 @@ struct PoolSinkT : SinkBase<kRawCapable> {
   // start), the lane with the chunk's first start also closes the run left
   // open by earlier chunks, and the chunk's spans are written after one
   // prefix sum.  Every entry read is reset to zero.
-  //
-  // With an event scratch (ev, room for ev_cap (position, value) pairs) the
-  // nonzero entries are first gathered in x order -- a difference array has
-  // two per accumulated span, usually far fewer than the row is wide -- and
-  // the runs are found over that list, 32 entries per step, with the same
-  // rules; a row with more nonzero entries than ev_cap takes the dense path.
-  SKC_HD bool acc_row(const Lanes& L, int y, int32_t* diff, int left, int lo, int hi,
-                      int32_t* ev = nullptr, int ev_cap = 0) {
+  SKC_HD bool acc_row(const Lanes& L, int y, int32_t* diff, int left, int lo, int hi) {
     if (y < row0 || y >= row1) return false;
     row_begin(L, y);
-    if (ev && Lanes::n == 32 && acc_row_sparse(L, y, diff, left, lo, hi, ev, ev_cap)) return true;
     constexpr int V = Lanes::n == 32 ? 4 : 1;
     constexpr int kNone = 0x7fffffff;
     int open_start = -1;   // warp-uniform: the run still open after a chunk
@@ -660,9 +578,10 @@ SKC_HD int RunRegSweep(const DevBatch& b, uint32_t p, const PassGeom& g, Sink* s
   L.compute(pd.cap, sizeof(Edge));
   const Edge* S = (const Edge*)(b.scratch + pd.slice_off + L.off[13]);
   const int n = g.n_edges;
-  SweepMem Mm = SweepMemAt(b.sweepmem + sw.work_off, n, g.acc_width);
-  for (int i = lanes.lane; i < n; i += Lanes::n) Mm.W[i] = S[i];
-  int32_t* diff = g.acc_width + 1 <= sdiff_cap ? sdiff : Mm.diff;
+  int32_t* diff = g.acc_width + 1 <= sdiff_cap
+                      ? sdiff
+                      : SweepMemAt(b.sweepmem + sw.work_off, n, g.acc_width).diff;
+#pragma unroll 1
   for (int i = lanes.lane; i <= g.acc_width; i += Lanes::n) diff[i] = 0;
   lanes.sync();
   AccState as;
@@ -672,13 +591,9 @@ SKC_HD int RunRegSweep(const DevBatch& b, uint32_t p, const PassGeom& g, Sink* s
   as.y = kNaN32;
   as.lo = 0x7fffffff;
   as.hi = -1;
-  as.ev = sh->u.ev;
-  as.ev_cap = RegSharedT<M>::kFlushEvents;
-  if (!RegWalk(lanes, *sh, Mm.W, n, sink, as, g.scan_top, (pd.flags & kPassEvenOdd) != 0,
-               g.start_y, g.stop_y, g.left_bound, g.right_bound))
-    return 0;
-  AccFlush(lanes, as, sink);
-  return 1;
+  as.flushing = false;
+  return RegWalk(lanes, *sh, S, n, sink, as, g.scan_top, (pd.flags & kPassEvenOdd) != 0,
+                 g.start_y, g.stop_y, g.left_bound, g.right_bound);
 }
 
 // Which sweep form takes pass p: the register form for up to 32, 64 or 128
@@ -714,6 +629,7 @@ SKC_HD bool SweepPassReg(const DevBatch& b, uint32_t p, const Lanes& lanes, RegS
   }
   // rows the sweep leaves without spans read as empty
   uint2* rows = b.rowspan + b.sweep[p].rbase;
+#pragma unroll 1
   for (int r = lanes.lane; r < g.row1 - g.row0; r += Lanes::n) rows[r] = make_uint2(0, 0);
   lanes.sync();
   PoolSinkReg sink;

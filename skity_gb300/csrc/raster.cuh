@@ -89,32 +89,26 @@ SKC_HD bool UpdateQuad(Edge* e) {  // sw_edge.cc:233-292
   Fixed dx = e->qdx, dy = e->qdy;
   Fixed newx = 0, newy = 0, nsx = 0, nsy = 0;
   int shift = e->curve_shift;
+  // the reference's three ways to a piece's end (a long piece, a short one,
+  // the last one) with one slope division between them
+#pragma unroll 1
   do {
-    Fixed slope;
+    bool far = false;
     if (--count > 0) {
       newx = wadd(oldx, dx >> shift);
       newy = wadd(oldy, dy >> shift);
-      if (iabs_(dy >> shift) >= kFixed1 * 2) {
-        FDot6 diffY = FixedToFDot6(wsub(newy, e->snapped_y));
-        slope = diffY ? FixedDiv(FixedToFDot6(wsub(newx, e->snapped_x)), diffY) : kMaxS32;
-        nsy = min_<Fixed>(e->q_last_y, FixedRoundToFixed(newy));
-        nsx = wsub(newx, FixedMul(slope, wsub(newy, nsy)));
-      } else {
-        nsy = min_<Fixed>(e->q_last_y, SnapY(newy));
-        nsx = newx;
-        FDot6 diffY = FixedToFDot6(wsub(nsy, e->snapped_y));
-        slope = diffY ? FixedDiv(FixedToFDot6(wsub(newx, e->snapped_x)), diffY) : kMaxS32;
-      }
+      far = iabs_(dy >> shift) >= kFixed1 * 2;
+      nsy = min_<Fixed>(e->q_last_y, far ? FixedRoundToFixed(newy) : SnapY(newy));
       dx = wadd(dx, e->qddx);
       dy = wadd(dy, e->qddy);
     } else {
       newx = e->q_last_x;
       newy = e->q_last_y;
       nsy = newy;
-      nsx = newx;
-      FDot6 diffY = wsub(newy, e->snapped_y) >> 10;
-      slope = diffY ? FixedDiv(wsub(newx, e->snapped_x) >> 10, diffY) : kMaxS32;
     }
+    const FDot6 diffY = FixedToFDot6(wsub(far ? newy : nsy, e->snapped_y));
+    const Fixed slope = diffY ? FixedDiv(FixedToFDot6(wsub(newx, e->snapped_x)), diffY) : kMaxS32;
+    nsx = far ? wsub(newx, FixedMul(slope, wsub(newy, nsy))) : newx;
     if (slope < kMaxS32) success = UpdateLine(e, e->snapped_x, e->snapped_y, nsx, nsy, slope);
     oldx = newx;
     oldy = newy;

@@ -1,136 +1,98 @@
 // The sweep of sweep.cuh with the active edges held in registers.
 //
 // Same per-step restatement of WalkEdges (src/render/sw/sw_raster.cc:546-677)
-// as LaneSweep, but the state that the generic form keeps in per-pass global
-// arrays lives on chip:
-//   * list position p of the active list is slot p / 32 of lane p % 32; a
-//     slot holds the edge's index, x, dx, dy, lower_y, winding and curve
-//     count in registers, and in the 32-edge form its quad-piece state too
-//     (the larger forms keep that in the pass's edge copy in global memory,
-//     touched only when a piece ends);
-//   * the per-position values an interval reads (x before the step, after
-//     GoY and after the update, dx, dy) and the interval endpoints are
-//     exchanged through a per-warp shared-memory block;
-//   * the reorder of the survivors is a compaction when their new x are
-//     already non-decreasing in list order (no crossing in the step), and
-//     the rank computation of LaneSweep otherwise;
-//   * each step's intervals, the one left open by a culled right edge
-//     included, are blitted in one pass after the reorder has been decided.
+// as LaneSweep, split into two loops that take turns:
+//
+//   the walk (RegWalk) advances the active list step by step and only logs,
+//   per step, one record per coverage interval -- its two edges' x before
+//   and after the step and their dy -- into a shared-memory buffer;
+//
+//   the emission (RegEmit), run whenever the buffer is full, turns the
+//   logged intervals of several rows into spans: a lane per interval for the
+//   set-up (blit_trapezoid_row), then a lane per span.
+//
+// Each loop is short (the sweep was bound by instruction fetch and latency
+// when a step's coverage was made inside the step), and the emission's lanes
+// are filled by the spans of many rows instead of one row's.
+//
+// The walk's state:
+//   * list position p of the active list is slot p / 32 of lane p % 32: x,
+//     dx, dy, lower_y and a packed word (winding, curve count and shift,
+//     quad slot) in registers; the quad-piece state an edge needs when a
+//     piece ends sits in shared memory at the edge's quad slot, so a reorder
+//     does not move it;
+//   * what depends on the list alone -- which edges open and close
+//     intervals, the nearest end of a piece -- is kept from step to step and
+//     recomputed only when the list or a piece changes;
+//   * windings are +-1, so their prefix sums are population counts of two
+//     ballots.
 // A path whose active list would exceed M edges (the form's size) is not swept here
-// (RegWalk returns 0 before touching its sink's output for the first time
-// at that size) and goes to LaneSweep.
+// (RegWalk returns 0) and goes to LaneSweep.
 #pragma once
 #include "sweep.cuh"
 
 namespace skc {
 
 constexpr int kRegMaxM = 128;  // the largest active list held in registers
-// intervals of one step with at most M active edges: one per pair of them,
-// plus the one left open by a culled right edge
-SKC_HD constexpr int RegIntervals(int M) { return M / 2 + 4; }
+// Interval records the walk logs before they are emitted: a step with at
+// most M active edges logs at most M / 2 + 1.
+SKC_HD constexpr int RegRecords(int M) { return M == 32 ? 64 : M; }
 
-// TrapRow set-ups of a step's intervals, one array per field.
-template <int N>
-struct TrapRowSoA {
-  int32_t ul[N], ur[N], ll[N], lr[N], ldy[N], rdy[N];
-  uint32_t meta[N];  // full | real << 8
-  SKC_HD void put(int i, const TrapRow& t) {
-    ul[i] = t.ul;
-    ur[i] = t.ur;
-    ll[i] = t.ll;
-    lr[i] = t.lr;
-    ldy[i] = t.lDY;
-    rdy[i] = t.rDY;
-    meta[i] = (uint32_t)t.full | (t.real ? 0x100u : 0u);
-  }
-  SKC_HD TrapRow get(int i) const {
-    TrapRow t;
-    t.ul = ul[i];
-    t.ur = ur[i];
-    t.ll = ll[i];
-    t.lr = lr[i];
-    t.lDY = ldy[i];
-    t.rDY = rdy[i];
-    t.full = (uint8_t)(meta[i] & 0xFF);
-    t.real = (meta[i] & 0x100u) != 0;
-    return t;
-  }
-};
+// The packed word of an active edge: winding (2 bits, +-1), a flag for the
+// edges a step has just inserted, curve count, curve shift, quad slot.
+SKC_HD int32_t MakeWc(int winding, int count, int shift, int slot) {
+  return (winding & 3) | ((count & 0x7F) << 8) | ((shift & 0xFF) << 16) |
+         (int32_t)((uint32_t)slot << 24);
+}
+constexpr int32_t kWcNew = 4;
+SKC_HD int WcWinding(int32_t wc) { return 2 - (wc & 3); }  // 1 -> 1, 3 -> -1
+SKC_HD int WcCount(int32_t wc) { return (wc >> 8) & 0x7F; }
+SKC_HD int WcShift(int32_t wc) { return (wc >> 16) & 0xFF; }
+SKC_HD int WcSlot(int32_t wc) { return (int)((uint32_t)wc >> 24); }
 
-// The quad-piece state of an active edge that UpdateQuad reads besides the
-// edge's line (x, dx, dy, lower_y, winding, curve count): forward-difference
-// position, steps and second differences, the last point, the shift.  The
-// 32-edge form holds it in registers beside the rest of the edge (one slot
-// per lane), so a piece change is a register update; the larger forms, with
-// two or four slots per lane, keep it in the pass's edge copy in memory.
-constexpr int kRegQuadWords = 9;
-SKC_HD constexpr bool RegQuadHeld(int M) { return M == 32; }
-struct RegQuad {
-  int32_t w[kRegQuadWords];  // qx, qy, qdx, qdy, qddx, qddy, q_last_x, q_last_y, curve_shift
-  SKC_HD void load(const Edge& e) {
-    w[0] = e.qx;
-    w[1] = e.qy;
-    w[2] = e.qdx;
-    w[3] = e.qdy;
-    w[4] = e.qddx;
-    w[5] = e.qddy;
-    w[6] = e.q_last_x;
-    w[7] = e.q_last_y;
-    w[8] = e.curve_shift;
-  }
-  SKC_HD void put(Edge& e) const {
-    e.qx = w[0];
-    e.qy = w[1];
-    e.qdx = w[2];
-    e.qdy = w[3];
-    e.qddx = w[4];
-    e.qddy = w[5];
-    e.q_last_x = w[6];
-    e.q_last_y = w[7];
-    e.curve_shift = (uint8_t)w[8];
-  }
+// The flags of a logged interval beside its row (high 16 bits) and the
+// step's alpha (low 8 bits).
+enum : uint32_t {
+  kRecClose = 0x100,     // the right edge is too close to its successor (full steps),
+                         // or a trailing interval's precomputed test
+  kRecFirst = 0x200,     // the step's first interval
+  kRecTrailing = 0x400,  // left open by a culled right edge: no test against its neighbours
+  kRecReal = 0x800       // after the set-up: spans are direct, not accumulated
 };
 
 // Per-warp shared block of the register sweep for active lists of up to
 // M edges.
 template <int M>
 struct RegSharedT {
-  static constexpr int kIntervals = RegIntervals(M);
-  static constexpr int kFlushEvents = 2 * M;  // nonzero accumulator entries a flush gathers
-  int32_t xo[M];   // x before the step, by list position
-  int32_t xg[M];   //   after GoY
-  int32_t xf[M];   //   after the quad-piece update
-  int32_t dxo[M];  // dx before the step
-  int32_t dyo[M];  // dy before the step
-  int32_t dxf[M];  // dx after the update
-  int32_t ia[M];   // interval k: left position
-  int32_t ib[M];   //   right position
-  int32_t ax[M];   // active x at insertion; new rank by list position in the reorder
-  // edge state by new list position (reorder and insertion)
-  int32_t p_idx[M], p_x[M], p_dx[M], p_dy[M];
-  int32_t p_low[M], p_wc[M];
-  // the quad-piece state of the edges (RegQuad) by new list position, for
-  // the forms that keep it in registers
-  int32_t p_q[RegQuadHeld(M) ? kRegQuadWords : 1][M];
+  static constexpr int kRecords = RegRecords(M);
+  static constexpr int kEvents = 2 * M;  // accumulator entries a flush gathers at a time
+  // Interval records, side 0 the left edge, side 1 the right one: x before
+  // the step; x after it (left: after the quad-piece update too); dy.  The
+  // emission overwrites them by its set-ups (ul/ur, ll/lr, lDY/rDY).
+  int32_t xa[2][kRecords], xb[2][kRecords], dy[2][kRecords];
+  uint32_t meta[kRecords];
+  int32_t start[32];   // first span of each set-up of the records being emitted
+  int32_t q[8][M];     // quad-piece state by quad slot (RegQuad)
+  uint8_t free_slot[M];  // quad slots no edge holds
   union {
     struct {
-      // the step's intervals (blit_trapezoid_row set-ups) and their first span
-      TrapRowSoA<kIntervals> iv;
-      int32_t iv_start[kIntervals + 4];
-    } b;
-    // accumulator flush scratch (used between steps, never during a blit)
-    int32_t ev[2 * kFlushEvents];
+      // edge state by new list position (reorder and insertion)
+      int32_t x[M], dx[M], dy[M], low[M], wc[M];
+      // the sort's keys: x and list position
+      int32_t kx[M], kp[M];
+    } p;
+    // accumulator flush (never during a step): the nonzero entries of the
+    // row's difference array, then the runs they start
+    struct {
+      int32_t pos[kEvents], val[kEvents];
+      int32_t run[kEvents + 2], sat[kEvents + 2];
+    } f;
   } u;
-  uint8_t surv[M];  // 1: survives the step
 };
 // Host and device must agree on these sizes (the host sizes the launch).
 static_assert(sizeof(RegSharedT<32>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<64>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<128>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
-
-SKC_HD int32_t MakeWc(int winding, int count) { return (winding & 0xFF) | ((count & 0xFF) << 8); }
-SKC_HD int WcWinding(int32_t wc) { return (int8_t)(wc & 0xFF); }
-SKC_HD int WcCount(int32_t wc) { return (int8_t)((wc >> 8) & 0xFF); }
 
 SKC_HD long long LaneMax64(const Lanes& L, long long v) {
 #ifdef SKC_WARP_LANES
@@ -141,222 +103,551 @@ SKC_HD long long LaneMax64(const Lanes& L, long long v) {
 #endif
   return v;
 }
+// v of the lane below (lane 0: `first`).
+SKC_HD int32_t LanePrev(const Lanes& L, int32_t v, int32_t first) {
+#ifdef SKC_WARP_LANES
+  const int32_t t = __shfl_up_sync(0xffffffffu, v, 1);
+  return L.lane == 0 ? first : t;
+#else
+  return first;
+#endif
+}
+SKC_HD uint32_t LaneOr(const Lanes& L, uint32_t v) {
+#ifdef SKC_WARP_LANES
+  return __reduce_or_sync(0xffffffffu, v);
+#else
+  return v;
+#endif
+}
+SKC_HD unsigned LeMask(const Lanes& L) { return (2u << L.lane) - 1u; }
+
+// Quad-piece state of an edge at its quad slot: forward-difference position,
+// steps and second differences, the last point (the shift is in the edge's
+// packed word).
+template <int M>
+SKC_HD void RegQuadPut(RegSharedT<M>& sh, int slot, const Edge& e) {
+  sh.q[0][slot] = e.qx;
+  sh.q[1][slot] = e.qy;
+  sh.q[2][slot] = e.qdx;
+  sh.q[3][slot] = e.qdy;
+  sh.q[4][slot] = e.qddx;
+  sh.q[5][slot] = e.qddy;
+  sh.q[6][slot] = e.q_last_x;
+  sh.q[7][slot] = e.q_last_y;
+}
+template <int M>
+SKC_HD void RegQuadGet(const RegSharedT<M>& sh, int slot, Edge* e) {
+  e->qx = sh.q[0][slot];
+  e->qy = sh.q[1][slot];
+  e->qdx = sh.q[2][slot];
+  e->qdy = sh.q[3][slot];
+  e->qddx = sh.q[4][slot];
+  e->qddy = sh.q[5][slot];
+  e->q_last_x = sh.q[6][slot];
+  e->q_last_y = sh.q[7][slot];
+}
+
+// v at the next list position (the last one's is undefined).
+template <int S>
+SKC_HD void LaneNext(const Lanes& L, const int32_t (&v)[S], int s, int32_t* out) {
+#ifdef SKC_WARP_LANES
+  int32_t t = __shfl_down_sync(0xffffffffu, v[s], 1);
+  if (S > 1) {
+    const int32_t u = __shfl_sync(0xffffffffu, v[s + 1 < S ? s + 1 : s], 0);
+    if (L.lane == 31) t = u;
+  }
+  *out = t;
+#else
+  *out = v[s + 1 < S ? s + 1 : s];
+#endif
+}
+// v at the list position before (position 0: undefined).
+template <int S>
+SKC_HD void LanePrevOf(const Lanes& L, const int32_t (&v)[S], int s, int32_t* out) {
+#ifdef SKC_WARP_LANES
+  int32_t t = __shfl_up_sync(0xffffffffu, v[s], 1);
+  if (S > 1) {
+    const int32_t u = __shfl_sync(0xffffffffu, v[s > 0 ? s - 1 : 0], 31);
+    if (L.lane == 0) t = u;
+  }
+  *out = t;
+#else
+  *out = v[s > 0 ? s - 1 : 0];
+#endif
+}
 
 // Row accumulator of the sweep (the difference array and its touched range).
 struct AccState {
   int32_t* diff;
   int left, width;
-  int y;       // row being accumulated (kNaN32: none yet)
+  int y;       // row being accumulated (kNaN32: none)
   int lo, hi;  // touched entries [lo, hi] (this lane's adds; reduced at the flush)
-  int32_t* ev; // flush scratch: (position, value) of nonzero entries
-  int ev_cap;
+  // a flush under way: next entry to read, the sum and its saturated value
+  // before it, the run open there
+  bool flushing;
+  int at;
+  int32_t sum, sat;
+  int open;    // entry the open run starts at (-1: none), its value is `sat`
 };
 
-template <typename Sink>
-SKC_HD void AccFlush(const Lanes& L, AccState& a, Sink* sink) {
-  if (a.y == kNaN32) return;
+SKC_HD void AccFlushBegin(const Lanes& L, AccState& a) {
   a.lo = LaneMin(L, a.lo);
   a.hi = LaneMax(L, a.hi);
-  if (a.lo <= a.hi) {
-    const bool read = sink->acc_row(L, a.y, a.diff, a.left, a.lo, a.hi, a.ev, a.ev_cap);
-    L.sync();
-    if (SKC_LIKELY(read)) {
-      if (L.leader()) a.diff[a.hi] = 0;
-    } else {
-      for (int i = a.lo + L.lane; i <= a.hi; i += Lanes::n) a.diff[i] = 0;
-    }
-    L.sync();
-  }
-  a.lo = 0x7fffffff;
-  a.hi = -1;
+  a.at = a.lo;
+  a.sum = a.sat = 0;
+  a.open = -1;
+  a.flushing = true;
 }
 
-template <typename Sink>
-SKC_HD void AccFlushIfNeed(const Lanes& L, AccState& a, Sink* sink, int row) {
-  if (a.y == row) return;
-  if (a.y != kNaN32) AccFlush(L, a, sink);
-  a.y = row;
-}
-
-// Trapezoid rows of a row's steps waiting for their spans: the set-ups of
-// intervals [0, n) in the shared interval block, `total` spans, canvas row y.
-struct BlitPending {
-  int n, total, y;
-};
-
-// The spans of the pending intervals, numbered in interval order, spread
-// over the lanes (span g on lane g mod 32), so a long partial row does not
-// hold one lane while the others wait.  Direct spans are written in that
-// order, the others go to the row accumulator.
-template <int M, typename Sink>
-SKC_HD void RegBlitFlush(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as,
-                         BlitPending& pend) {
+// The next runs of an accumulated row (SpanBuilder::Flush, sw_raster.cc:
+// 103-136): the row's alphas are the saturated prefix sums of the difference
+// array, and a run starts at every entry whose alpha differs from its left
+// neighbour's.  Gathers the next nonzero entries (each is reset to zero) and
+// leaves the runs they complete in sh.u.f.run / sat, each ending where the
+// next one starts; returns their number.  A run still open waits in `a` for
+// the next call; the flush ends with the touched range.
+template <int M>
+SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
   constexpr int NL = Lanes::n;
-  if (pend.n == 0) return;
-  sink->row_begin(L, pend.y);
-  if (L.leader()) sh.u.b.iv_start[pend.n] = pend.total;
+  int ne = 0;
+#pragma unroll 1
+  while (a.at < a.hi && ne + NL <= RegSharedT<M>::kEvents) {
+    const int i = a.at + L.lane;
+    const int32_t d = i < a.hi ? a.diff[i] : 0;
+    const unsigned mask = L.ballot(d != 0);
+    if (mask) {
+      if (d != 0) {
+        const int e = ne + Lanes::popc(mask & L.lt_mask());
+        sh.u.f.pos[e] = i;
+        sh.u.f.val[e] = d;
+        a.diff[i] = 0;
+      }
+      ne += Lanes::popc(mask);
+    }
+    a.at += NL;
+  }
+  int ns = 0;
+  if (a.open >= 0) {
+    if (L.leader()) {
+      sh.u.f.run[0] = a.open;
+      sh.u.f.sat[0] = a.sat;
+    }
+    ns = 1;
+  }
   L.sync();
-  const int T = pend.total;
-  const int y = pend.y;
-  uint32_t run = 0;
-  unsigned long long frags = 0;
-  int lo = 0x7fffffff, hi = -1;
-  int iv = 0;
-  for (int gb = 0; gb < T; gb += NL) {
-    const int g = gb + L.lane;
+#pragma unroll 1
+  for (int eb = 0; eb < ne; eb += NL) {
+    const int e = eb + L.lane;
+    const bool valid = e < ne;
+    const int32_t incl = LaneScanIncl(L, valid ? sh.u.f.val[e] : 0) + a.sum;
+    const int32_t sat = min_(incl, 255);
+    const int32_t before = LanePrev(L, sat, a.sat);
+    const bool start = valid && sat != before;
+    const unsigned starts = L.ballot(start);
+    if (start) {
+      const int r = ns + Lanes::popc(starts & L.lt_mask());
+      sh.u.f.run[r] = sh.u.f.pos[e];
+      sh.u.f.sat[r] = sat;
+    }
+    ns += Lanes::popc(starts);
+    a.sum = LaneBcast(L, incl, NL - 1);
+    a.sat = LaneBcast(L, sat, NL - 1);
+  }
+  L.sync();
+  if (a.at >= a.hi) {  // the row's end closes the last run
+    if (L.leader()) {
+      sh.u.f.run[ns] = a.hi;
+      if (a.lo <= a.hi) a.diff[a.hi] = 0;
+    }
+    a.flushing = false;
+    a.lo = 0x7fffffff;
+    a.hi = -1;
+    a.y = kNaN32;
+  } else if (ns > 0) {
+    --ns;
+    a.open = sh.u.f.run[ns];
+  }
+  L.sync();
+  return ns;
+}
+
+// Spans of the logged intervals [0, nrec), rows in order; `last`: and of the
+// row still accumulated.  Chunks of one record per lane are set up at once;
+// their spans are made in runs of rows that end with the first row that
+// accumulates (an accumulated row's spans follow its direct ones in the pool,
+// so the accumulator is flushed before a later row's spans are written).  One
+// loop makes the spans of both kinds, a span per lane, so that the code that
+// stores them is there once (the sweep's instruction fetch is its scarcest
+// resource).
+template <int M, typename Sink>
+SKC_HD void RegEmit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as, int nrec,
+                    Fixed left_clip, Fixed right_clip, bool last) {
+  constexpr int NL = Lanes::n;
+  int32_t last_ur = 0, last_lr = 0;  // the previous chunk's last right edge
+  // the chunk [lo, lo + nv): this lane's record's row, spans before it and
+  // through it; the chunk's row starts and accumulating records
+  int lo = 0, nv = 0, row = 0, excl = 0, incl = 0;
+  bool spans = false;
+  unsigned heads = 0, accs = 0;
+  int a = 0;         // next record of the chunk
+  int w = 0, g1 = 0;  // spans of the run under way
+  int fi = 0, fn = 0, fy = 0;  // accumulated runs to store, their row
+#pragma unroll 1
+  for (;;) {
     bool kept = false;
     uint2 v = make_uint2(0, 0);
-    if (g < T) {
-      while (sh.u.b.iv_start[iv + 1] <= g) ++iv;
-      const TrapRow t = sh.u.b.iv.get(iv);
-      int x = 0, len = 0;
-      uint8_t a = 0;
-      TrapSpan(t, g - sh.u.b.iv_start[iv], x, len, a);
-      if (t.real) {
-        if (sink->keep(x, y, len, a)) {
-          kept = true;
-          v = sink->pack(x, len, a);
-          frags += (unsigned)len;
-        }
-      } else {
-        int o0 = x - as.left, o1 = o0 + len;
-        o0 = max_(o0, 0);
-        o1 = min_(o1, as.width);
-        if (o0 < o1) {
-          lo = min_(lo, o0);
-          hi = max_(hi, o1);
-          if (a != 0) {
-            AtomicAddI32(&as.diff[o0], (int32_t)a);
-            AtomicAddI32(&as.diff[o1], -(int32_t)a);
+    int y = 0, x = 0, len = 0;
+    uint8_t al = 0;
+    if (fi < fn) {
+      const int i = fi + L.lane;
+      y = fy;
+      if (i < fn) {
+        const int x0 = sh.u.f.run[i];
+        x = as.left + x0;
+        len = sh.u.f.run[i + 1] - x0;
+        al = (uint8_t)sh.u.f.sat[i];
+        kept = al != 0;
+      }
+      fi += NL;
+    } else if (as.flushing) {
+      fy = as.y;
+      L.sync();
+      fn = AccRuns(L, as, sh);
+      fi = 0;
+      continue;
+    } else if (w < g1) {
+      // the set-up of span w + lane: set-ups are packed in span order, so
+      // it is the number of set-ups that start at or before the span
+      const uint32_t rel = (uint32_t)(excl - w);
+      const uint32_t bits = LaneOr(L, (spans && rel < (uint32_t)NL) ? 1u << rel : 0u);
+      const int before = Lanes::popc(L.ballot(spans && excl < w));
+      const int g = w + L.lane;
+      if (g < g1) {
+        const int j = before + Lanes::popc(bits & LeMask(L)) - 1;
+        const uint32_t mt = sh.meta[lo + j];
+        TrapRow q;
+        q.ul = sh.xa[0][lo + j];
+        q.ur = sh.xa[1][lo + j];
+        q.ll = sh.xb[0][lo + j];
+        q.lr = sh.xb[1][lo + j];
+        q.lDY = sh.dy[0][lo + j];
+        q.rDY = sh.dy[1][lo + j];
+        q.full = (uint8_t)(mt & 0xFF);
+        q.real = (mt & kRecReal) != 0;
+        y = (int)mt >> 16;
+        TrapSpan(q, g - sh.start[j], x, len, al);
+        kept = q.real;
+        if (!kept) {
+          int o0 = x - as.left, o1 = o0 + len;
+          o0 = max_(o0, 0);
+          o1 = min_(o1, as.width);
+          if (o0 < o1) {
+            as.lo = min_(as.lo, o0);
+            as.hi = max_(as.hi, o1);
+            if (al != 0) {
+              AtomicAddI32(&as.diff[o0], (int32_t)al);
+              AtomicAddI32(&as.diff[o1], -(int32_t)al);
+            }
           }
         }
       }
-    }
-    const unsigned km = L.ballot(kept);
-    const uint32_t cnt = (uint32_t)Lanes::popc(km);
-    if (cnt) {
-      const uint64_t at = sink->reserve(L, run, cnt);
-      uint2* dst = sink->span_ptr(at + run + (uint32_t)Lanes::popc(km & L.lt_mask()));
-      if (kept && dst) *dst = v;
-      run += cnt;
-    }
-  }
-  // the fragment count and the accumulator's touched range stay per lane
-  // (summed at the pass's end, reduced at the row's flush)
-  as.lo = min_(as.lo, lo);
-  as.hi = max_(as.hi, hi);
-  sink->commit(L, run, frags);
-  pend.n = 0;
-  pend.total = 0;
-  L.sync();
-}
-
-// The intervals [0, K) of a step, then (trailing_a >= 0) the interval left
-// open by the last left edge: blit_trapezoid_row for each.  One lane per
-// interval does the row's set-up and counts its spans; the set-ups wait in
-// the interval block, with those of the row's earlier steps, until the row
-// ends or the block is full (a row's partial steps all go to the
-// accumulator, whose sums do not depend on order; a full step is the only
-// step of its row), and their spans are then made in one pass.
-template <int M, typename Sink>
-SKC_HD void RegBlit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as,
-                    BlitPending& pend, const Edge* W, int n, int y, Fixed next_y, int K, int m,
-                    int k, uint8_t full, Fixed left_clip, Fixed right_clip, int trailing_a,
-                    bool trailing_nr) {
-  constexpr int NL = Lanes::n;
-  const int total = K + (trailing_a >= 0 ? 1 : 0);
-  if (pend.n > 0 && (pend.y != y || pend.n + total > RegSharedT<M>::kIntervals))
-    RegBlitFlush(L, sh, sink, as, pend);
-  AccFlushIfNeed(L, as, sink, y);
-  int carry = 0;
-  for (int kb = 0; kb < total; kb += NL) {
-    const int ki = kb + L.lane;
-    int cnt = 0;
-    if (ki < total) {
-      Fixed ul, ur, ll, lr, lDY, rDY;
-      bool nr;
-      if (ki < K) {
-        const int a = sh.ia[ki], b = sh.ib[ki];
-        ul = max_(sh.xo[a], left_clip);
-        lDY = sh.dyo[a];
-        ur = min_(right_clip, sh.xo[b]);
-        ll = max_(left_clip, sh.xf[a]);
-        lr = min_(right_clip, sh.xg[b]);
-        rDY = sh.dyo[b];
-        int prev_right;
-        if (ki == 0) {
-          prev_right = FixedFloorToInt(left_clip);
-        } else {
-          const int pb = sh.ib[ki - 1];
-          prev_right = FixedCeilToInt(max_(min_(right_clip, sh.xo[pb]), sh.xg[pb]));
-        }
-        bool tc = prev_right > FixedFloorToInt(ul) || prev_right > FixedFloorToInt(sh.xf[a]);
-        if (!tc) {
-          // edges_too_close(right edge, its successor before the step)
-          int32_t nxo, ndx;
-          Fixed nup;
-          if (b + 1 < m) {
-            nxo = sh.xo[b + 1];
-            ndx = sh.dxo[b + 1];
-            nup = kMinS32;  // active: upper_y <= y < next_y
-          } else if (k < n) {
-            nxo = W[k].x;
-            ndx = W[k].dx;
-            nup = W[k].upper_y;
-          } else {
-            nxo = kMaxS32;
-            ndx = 0;
-            nup = kMaxS32;
-          }
-          tc = nup < next_y && wadd(sh.xg[b], kFixed1) >= wsub(nxo, iabs_(ndx));
-        }
-        nr = tc;
-      } else {
-        const int a = trailing_a;
-        ul = max_(sh.xo[a], left_clip);
-        lDY = sh.dyo[a];
-        ur = right_clip;
-        ll = max_(left_clip, sh.xf[a]);
-        lr = right_clip;
-        rDY = 0;
-        nr = trailing_nr;
+      w += NL;
+    } else if (a < nv) {
+      // the run [a, b) of records: to the end of the first row that
+      // accumulates
+      const int row_a = LaneBcast(L, row, a);
+      if (as.y != kNaN32 && as.y != row_a) {
+        AccFlushBegin(L, as);
+        continue;
       }
+      int at = a;  // the record whose row ends the run
+      if (as.y == kNaN32) {
+        const unsigned m = accs & ~((1u << a) - 1u);
+        at = m ? Lanes::ffs(m) - 1 : NL;
+      }
+      int b = nv;
+      if (at < nv) {
+        const unsigned h = heads & ~((2u << at) - 1u);
+        if (h) b = Lanes::ffs(h) - 1;
+        as.y = LaneBcast(L, row, at);
+      }
+      w = LaneBcast(L, excl, a);
+      g1 = LaneBcast(L, incl, b - 1);
+      a = b;
+      continue;
+    } else if (lo + nv < nrec) {
+      // the next chunk's set-ups
+      lo += nv;
+      a = w = g1 = 0;
+      const int i = lo + L.lane;
+      const bool valid = i < nrec;
+      nv = min_(NL, nrec - lo);
       TrapRow t;
-      if (TrapPrepare(t, ul, ur, ll, lr, lDY, rDY, full, nr)) {
-        cnt = TrapCount(t);
-        sh.u.b.iv.put(pend.n + ki, t);
+      int32_t ul = 0, ur = 0, ll = 0, lr = 0;
+      uint32_t meta = 0;
+      t.lDY = t.rDY = 0;
+      L.sync();
+      if (valid) {
+        ul = sh.xa[0][i];
+        ll = sh.xb[0][i];
+        t.lDY = sh.dy[0][i];
+        ur = sh.xa[1][i];
+        lr = sh.xb[1][i];
+        t.rDY = sh.dy[1][i];
+        meta = sh.meta[i];
       }
+      const int32_t pur = LanePrev(L, ur, last_ur), plr = LanePrev(L, lr, last_lr);
+      last_ur = LaneBcast(L, ur, NL - 1);
+      last_lr = LaneBcast(L, lr, NL - 1);
+      row = (int)meta >> 16;
+      const uint8_t full = (uint8_t)(meta & 0xFF);
+      const int prev_right = (meta & kRecFirst)
+                                 ? FixedFloorToInt(left_clip)
+                                 : FixedCeilToInt(max_(min_(right_clip, pur), plr));
+      const Fixed cul = max_(ul, left_clip);
+      bool nr = (meta & kRecClose) != 0;
+      if (!(meta & kRecTrailing))
+        nr = nr || prev_right > FixedFloorToInt(cul) || prev_right > FixedFloorToInt(ll);
+      int cnt = 0;
+      bool real = false;
+      if (valid && TrapPrepare(t, cul, min_(right_clip, ur), max_(left_clip, ll),
+                               min_(right_clip, lr), t.lDY, t.rDY, full, nr)) {
+        cnt = TrapCount(t);
+        real = t.real;
+      }
+      incl = LaneScanIncl(L, cnt);
+      excl = incl - cnt;
+      spans = cnt > 0;
+      const unsigned some = L.ballot(spans);
+      L.sync();
+      if (spans) {  // the set-ups that make spans, packed from `lo`
+        const int j = Lanes::popc(some & L.lt_mask());
+        sh.xa[0][lo + j] = t.ul;
+        sh.xa[1][lo + j] = t.ur;
+        sh.xb[0][lo + j] = t.ll;
+        sh.xb[1][lo + j] = t.lr;
+        sh.dy[0][lo + j] = t.lDY;
+        sh.dy[1][lo + j] = t.rDY;
+        sh.meta[lo + j] = (meta & 0xFFFF00FFu) | (real ? kRecReal : 0u);
+        sh.start[j] = excl;
+      }
+      L.sync();
+      const int prow = LanePrev(L, row, kNaN32);
+      heads = L.ballot(valid && row != prow);
+      accs = L.ballot(spans && !real);
+      continue;
+    } else if (last && as.y != kNaN32) {
+      AccFlushBegin(L, as);
+      continue;
+    } else {
+      break;
     }
-    const int32_t incl = LaneScanIncl(L, cnt);
-    if (ki < total) sh.u.b.iv_start[pend.n + ki] = pend.total + carry + incl - cnt;
-    carry += LaneBcast(L, incl, NL - 1);
+    if (kept) {
+      kept = sink->keep(x, y, len, al);
+      v = sink->pack(x, len, al);
+    }
+    sink->put_rows(L, kept, v, y, (unsigned)len);
   }
-  pend.y = y;
-  pend.n += total;
-  pend.total += carry;
   L.sync();
 }
 
-// WalkEdges over the pass's sorted edges W[0, n) (modified in place: quad
-// pieces).  Returns 0 if the active list would exceed M edges.
+// Slot s (warp-uniform) of a per-slot register.
+template <int S, typename T>
+SKC_HD T SlotGet(const T (&v)[S], int s) {
+  if (Lanes::n == 1) return v[s];
+  T r = v[0];
+#pragma unroll
+  for (int i = 1; i < S; ++i)
+    if (s == i) r = v[i];
+  return r;
+}
+template <int S, typename T>
+SKC_HD void SlotSet(T (&v)[S], int s, T x) {
+  if (Lanes::n == 1) {
+    v[s] = x;
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < S; ++i)
+    if (s == i) v[i] = x;
+}
+
+// Stores an active list by list position for a reorder, then loads it back.
+template <int M>
+SKC_HD void RegStage(RegSharedT<M>& sh, int r, int32_t x, int32_t dx, int32_t dy, int32_t low,
+                     int32_t wc) {
+  sh.u.p.x[r] = x;
+  sh.u.p.dx[r] = dx;
+  sh.u.p.dy[r] = dy;
+  sh.u.p.low[r] = low;
+  sh.u.p.wc[r] = wc;
+}
+
+template <int M, int S>
+SKC_HD void RegLoad(const Lanes& L, const RegSharedT<M>& sh, int m, int32_t (&x)[S],
+                    int32_t (&dx)[S], int32_t (&dy)[S], int32_t (&low)[S], int32_t (&wc)[S]) {
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int p = s * Lanes::n + L.lane;
+    if (p < m) {
+      x[s] = sh.u.p.x[p];
+      dx[s] = sh.u.p.dx[p];
+      dy[s] = sh.u.p.dy[p];
+      low[s] = sh.u.p.low[p];
+      wc[s] = sh.u.p.wc[p];
+    }
+  }
+}
+
+// The interval left open by the last left edge of a step (its right edge was
+// culled), logged behind the step's other intervals, with its too-close test
+// against the left edge's predecessor after the reorder (its new predecessor
+// if it survives, else the last processed survivor before it).
+template <int M, int S>
+SKC_HD void RegTrailing(const Lanes& L, RegSharedT<M>& sh, const int32_t (&x)[S],
+                        const int32_t (&dx)[S], const int32_t (&low)[S], const int (&off)[S],
+                        Fixed next_y, int m, int nr, int nrec, uint32_t meta, Fixed left_clip) {
+  constexpr int NL = Lanes::n;
+  // the left edge: position, x, dx, whether it goes on
+  int32_t mine = -1, xa = 0, dxa = 0, la = 0;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    if (off[s] == nr && s * NL + L.lane < m) {
+      mine = s * NL + L.lane;
+      xa = x[s];
+      dxa = dx[s];
+      la = low[s];
+    }
+  }
+  const int a = LaneMax(L, mine);
+  xa = LaneBcast(L, xa, NL == 32 ? a & 31 : 0);
+  dxa = LaneBcast(L, dxa, NL == 32 ? a & 31 : 0);
+  const bool a_surv = LaneBcast(L, la, NL == 32 ? a & 31 : 0) > next_y;
+  long long key = 0;
+  bool found = false;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int p = s * NL + L.lane;
+    if (p < m && low[s] > next_y) {
+      const int32_t xi = x[s];
+      const bool cand = a_surv ? (p != a && (xi < xa || (xi == xa && p < a))) : p < a;
+      if (cand) {
+        const long long kk = ((long long)xi << 32) | (unsigned)p;
+        if (!found || kk > key) key = kk;
+        found = true;
+      }
+    }
+  }
+  const bool any = L.ballot(found) != 0;
+  if (!found) key = (long long)kMinS32 << 32;
+  key = LaneMax64(L, key);
+  const int32_t pred_x = any ? (int32_t)(key >> 32) : left_clip;
+  const bool tc = wadd(pred_x, kFixed1) >= wsub(xa, iabs_(dxa));
+  if (L.leader()) {
+    const int at = nrec + nr;
+    sh.xa[1][at] = sh.xb[1][at] = kMaxS32;  // the right clip
+    sh.dy[1][at] = 0;
+    sh.meta[at] = meta | kRecTrailing | (nr == 0 ? kRecFirst : 0u) |
+                  (((meta & 0xFF) == 0xFF && tc) ? kRecClose : 0u);
+  }
+}
+
+// An edge moved left of an earlier one.  The reference ripples each such
+// edge backwards (backward_insert_edge_based_on_x), which leaves the list
+// stably sorted by new x; its crossing check then compares an edge with its
+// predecessor at that moment: the latest (in sorted order) earlier-listed
+// edge whose x is not greater.  Sorts the (x, list position) keys by odd-even
+// transposition (the list is nearly sorted, so few phases run), finds each
+// edge's predecessor by a short backward scan, reorders the list and returns
+// whether this lane saw a crossing.
+template <int M, int S>
+SKC_HD bool RegSort(const Lanes& L, RegSharedT<M>& sh, int m, int32_t (&x)[S], int32_t (&dx)[S],
+                    int32_t (&dy)[S], int32_t (&low)[S], int32_t (&wc)[S]) {
+  constexpr int NL = Lanes::n;
+  int32_t* kx = sh.u.p.kx;
+  int32_t* kp = sh.u.p.kp;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int p = s * NL + L.lane;
+    if (p < m) {
+      kx[p] = x[s];
+      kp[p] = p;
+      sh.u.p.dx[p] = dx[s];
+    }
+  }
+  L.sync();
+  bool dirty_prev = true;
+#pragma unroll 1
+  for (int phase = 0; phase < m + 2; ++phase) {
+    bool swapped = false;
+#pragma unroll 1
+    for (int i = 2 * L.lane + (phase & 1); i + 1 < m; i += 2 * NL) {
+      const int32_t xa = kx[i], xb = kx[i + 1];
+      const int32_t pa = kp[i], pb = kp[i + 1];
+      if (xb < xa || (xb == xa && pb < pa)) {
+        kx[i] = xb;
+        kx[i + 1] = xa;
+        kp[i] = pb;
+        kp[i + 1] = pa;
+        swapped = true;
+      }
+    }
+    L.sync();
+    const bool dirty = L.ballot(swapped) != 0;
+    if (!dirty && !dirty_prev) break;
+    dirty_prev = dirty;
+  }
+  bool cross = false;
+#pragma unroll 1
+  for (int r = L.lane; r < m; r += NL) {
+    const int pr = kp[r];
+    int q = r - 1;
+#pragma unroll 1
+    while (q >= 0 && kp[q] > pr) --q;
+    if (q >= 0 && wadd(kx[q], sh.u.p.dx[kp[q]]) > wadd(kx[r], sh.u.p.dx[pr])) cross = true;
+  }
+  L.sync();
+  // rank of each list position, by way of the wc row
+#pragma unroll 1
+  for (int r = L.lane; r < m; r += NL) sh.u.p.wc[kp[r]] = r;
+  L.sync();
+  int rank[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int p = s * NL + L.lane;
+    rank[s] = p < m ? sh.u.p.wc[p] : 0;
+  }
+  L.sync();
+#pragma unroll
+  for (int s = 0; s < S; ++s)
+    if (s * NL + L.lane < m) RegStage<M>(sh, rank[s], x[s], dx[s], dy[s], low[s], wc[s]);
+  L.sync();
+  RegLoad<M, S>(L, sh, m, x, dx, dy, low, wc);
+  L.sync();
+  return cross;
+}
+
+// WalkEdges over the pass's sorted edges W[0, n).  Returns 0 if the active
+// list would exceed M edges.
 template <int M, typename Sink>
-SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, Edge* W, int n, Sink* sink, AccState& as,
-                   float scan_top, bool even_odd, int start_y, int stop_y, Fixed left_clip,
-                   Fixed right_clip) {
+SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink* sink,
+                   AccState& as, float scan_top, bool even_odd, int start_y, int stop_y,
+                   Fixed left_clip, Fixed right_clip) {
   constexpr int NL = Lanes::n;
   constexpr int S = M / NL;
+  constexpr int R = RegSharedT<M>::kRecords;
   constexpr unsigned kFull = NL == 32 ? 0xffffffffu : 1u;
   const int winding_mask = even_odd ? 1 : -1;
-  int32_t r_idx[S], r_x[S], r_dx[S], r_dy[S], r_low[S], r_wc[S];
-  constexpr bool kQ = RegQuadHeld(M);
-  RegQuad r_q[kQ ? S : 1];
+  // rows whose coverage is kept (scan_top is a whole number)
+  const int row_lo = max_((int)scan_top, sink->row0), row_hi = sink->row1;
+  const Fixed y_stop = IntToFixed(stop_y);
+  int32_t x[S], dx[S], dy[S], low[S], wc[S];
+  int off[S];  // where the edge logs: side * R + its interval of the step; < 0: it does not
 
-  BlitPending pend;
-  pend.n = pend.total = 0;
-  pend.y = kNaN32;
   Fixed y = max_(W[0].upper_y, IntToFixed(start_y));
   // initial activation: the edges with upper_y <= y, in their sorted order
   int k = 0;
+#pragma unroll 1
   for (int base = 0; base < n; base += NL) {
     const int i = base + L.lane;
     const unsigned mask = L.ballot(i < n && W[i].upper_y <= y);
@@ -365,387 +656,316 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, Edge* W, int n, Sink* sink
   }
   if (k > M) return 0;
   int m = k;
-  Fixed nny = kMaxS32;
-  {
-    int32_t lmin = kMaxS32;
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
-      const int p = s * NL + L.lane;
-      r_idx[s] = r_x[s] = r_dx[s] = r_dy[s] = r_low[s] = r_wc[s] = 0;
-      if (p < m) {
-        Edge e = W[p];
-        GoY(&e, y);
-        if (kQ) r_q[s].load(e);
-        r_idx[s] = p;
-        r_x[s] = e.x;
-        r_dx[s] = e.dx;
-        r_dy[s] = e.dy;
-        r_low[s] = e.lower_y;
-        r_wc[s] = MakeWc(e.winding, e.curve_count);
-        if (e.lower_y > y) lmin = min_(lmin, e.lower_y);
-      }
+  for (int s = 0; s < S; ++s) {
+    const int p = s * NL + L.lane;
+    x[s] = dx[s] = dy[s] = low[s] = wc[s] = 0;
+    off[s] = -1;
+    if (p < m) {
+      Edge e = W[p];
+      GoY(&e, y);
+      x[s] = e.x;
+      dx[s] = e.dx;
+      dy[s] = e.dy;
+      low[s] = e.lower_y;
+      wc[s] = MakeWc(e.winding, e.curve_count, e.curve_shift, p);
+      if (e.curve_count > 0) RegQuadPut(sh, p, e);
     }
-    lmin = LaneMin(L, lmin);
-    nny = min_(nny, lmin);
-    if (k < n && W[k].upper_y > y) nny = min_(nny, W[k].upper_y);
+    sh.free_slot[p] = (uint8_t)(M - 1 - p);  // taken from the end: slots m, m + 1, ...
   }
+  int n_free = M - m;
+  Fixed pend_y = k < n ? W[k].upper_y : kMaxS32;
+  // of the list: intervals a step logs (and how many of them a right edge
+  // closes), whether one stays open, the lowest end of a piece, the lowest
+  // one past y
+  int nr = 0, K = 0;
+  bool final_in = false;
+  Fixed lmin = kMaxS32, lnext = kMaxS32;
+  bool cross = false, changed = true;
+  int nrec = 0;
+  L.sync();
 
+#pragma unroll 1
   for (;;) {
-    Fixed next_y = min_(nny, FixedCeilToFixed(y + 1));
-    int y_shift = 0;
-    if ((next_y - y) & (kFixed1 >> 2)) {
-      y_shift = 2;
-      next_y = y + (kFixed1 >> 2);
-    } else if ((next_y - y) & (kFixed1 >> 1)) {
-      y_shift = 1;
-    }
-    const uint8_t full = partial_alpha_h(0xFF, next_y - y);
-    nny = kMaxS32;
-    const int ns = (m + NL - 1) / NL;
-
-    // ---- A: advance every active edge
-    int32_t wcarry = 0;
-    int nl = 0, nr = 0;
-    unsigned smask[S];
-    int32_t lmin = kMaxS32;
+    bool done = false;
+#pragma unroll 1
+    for (;;) {
+      if (changed) {
+        // ---- what the list determines
+        int32_t carry = 0;
+        int nl = 0;
+        nr = 0;
+        int32_t l0 = kMaxS32, l1 = kMaxS32;
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
-      smask[s] = 0;
-      if (s < ns) {
-        const int p = s * NL + L.lane;
-        const bool valid = p < m;
-        const int32_t wv = valid ? (int32_t)WcWinding(r_wc[s]) : 0;
-        const int32_t incl = LaneScanIncl(L, wv) + wcarry;
-        const int32_t excl = incl - wv;
-        const bool in = (incl & winding_mask) != 0;
-        const bool pin = (excl & winding_mask) != 0;
-        const bool is_left = valid && in && !pin;
-        const bool is_right = valid && !in && pin;
-        const unsigned lm = L.ballot(is_left), rm = L.ballot(is_right);
-        bool surv = false;
-        if (valid) {
-          const int32_t xo = r_x[s], dxo = r_dx[s], dyo = r_dy[s];
-          int32_t x = wadd(xo, dxo >> y_shift);  // GoYShift
-          const int32_t xg = x;
-          if (SKC_COLD(r_low[s] <= next_y && WcCount(r_wc[s]) > 0)) {
-            Edge e;
-            if (kQ) {
-              r_q[s].put(e);
-            } else {
-              e = W[r_idx[s]];
+        for (int s = 0; s < S; ++s) {
+          if (s == 0 || s * NL < m) {
+            const bool valid = s * NL + L.lane < m;
+            const bool neg = (wc[s] & 2) != 0;
+            const unsigned bp = L.ballot(valid && !neg), bn = L.ballot(valid && neg);
+            const unsigned le = LeMask(L);
+            const int32_t incl = carry + Lanes::popc(bp & le) - Lanes::popc(bn & le);
+            const int32_t excl = incl - (neg ? -1 : 1);
+            const bool in = (incl & winding_mask) != 0;
+            const bool pin = (excl & winding_mask) != 0;
+            const unsigned lm = L.ballot(valid && in && !pin), rm = L.ballot(valid && !in && pin);
+            off[s] = -1;
+            if (valid && in != pin)
+              off[s] = in ? nl + Lanes::popc(lm & L.lt_mask())
+                          : R + nr + Lanes::popc(rm & L.lt_mask());
+            nl += Lanes::popc(lm);
+            nr += Lanes::popc(rm);
+            carry += Lanes::popc(bp) - Lanes::popc(bn);
+            if (valid) {
+              l0 = min_(l0, low[s]);
+              if (low[s] > y) l1 = min_(l1, low[s]);
             }
-            e.x = x;
-            e.y = next_y;
-            e.dx = dxo;
-            e.dy = dyo;
-            e.lower_y = r_low[s];
-            e.winding = (int8_t)WcWinding(r_wc[s]);
-            e.curve_count = (int8_t)WcCount(r_wc[s]);
-            while (e.lower_y <= next_y && e.curve_count > 0) {
-              e.snapped_x = e.x;  // KeepContinuous (sw_edge.cc:294-297)
-              e.snapped_y = e.y;
-              if (!UpdateQuad(&e)) break;
-            }
-            if (kQ) {
-              r_q[s].load(e);
-            } else {
-              W[r_idx[s]] = e;
-            }
-            x = e.x;
-            r_dx[s] = e.dx;
-            r_dy[s] = e.dy;
-            r_low[s] = e.lower_y;
-            r_wc[s] = MakeWc(e.winding, e.curve_count);
           }
-          r_x[s] = x;
-          surv = r_low[s] > next_y;
-          if (surv) lmin = min_(lmin, r_low[s]);
-          sh.xo[p] = xo;
-          sh.xg[p] = xg;
-          sh.xf[p] = x;
-          sh.dxo[p] = dxo;
-          sh.dyo[p] = dyo;
-          sh.dxf[p] = r_dx[s];
-          sh.surv[p] = surv ? 1 : 0;
-          if (is_left) sh.ia[nl + Lanes::popc(lm & L.lt_mask())] = p;
-          if (is_right) sh.ib[nr + Lanes::popc(rm & L.lt_mask())] = p;
         }
-        smask[s] = L.ballot(surv);
-        nl += Lanes::popc(lm);
-        nr += Lanes::popc(rm);
-        wcarry = LaneBcast(L, incl, min_(NL, m - s * NL) - 1);
+        final_in = (carry & winding_mask) != 0;
+        K = nr + (final_in ? 1 : 0);
+        lmin = LaneMin(L, l0);
+        lnext = LaneMin(L, l1);
+        changed = false;
       }
-    }
-    const bool final_in = (wcarry & winding_mask) != 0;
-    L.sync();
+      if (nrec + K > R) break;  // the buffer is full: emit, then take the step
+      Fixed nny = min_(lnext, pend_y);
+      if (cross) nny = min_(nny, y + (kFixed1 >> kAccuracy));
+      cross = false;
+      if (m == 0) {  // nothing active: on to the next edge
+        y = pend_y;
+        if (y >= y_stop) {
+          done = true;
+          break;
+        }
+      } else {
+        Fixed next_y = min_(nny, FixedCeilToFixed(y + 1));
+        int y_shift = 0;
+        if ((next_y - y) & (kFixed1 >> 2)) {
+          y_shift = 2;
+          next_y = y + (kFixed1 >> 2);
+        } else if ((next_y - y) & (kFixed1 >> 1)) {
+          y_shift = 1;
+        }
+        const uint8_t full = partial_alpha_h(0xFF, next_y - y);
+        const int row = y >> 16;
+        const bool log = K > 0 && row >= row_lo && row < row_hi;
+        const uint32_t meta = ((uint32_t)row << 16) | full;
 
-    // ---- C: survivors in stable order of their new x; intersections
-    int m2 = 0;
-    int r_rank[S];
-    bool cross = false, inv = false;
-    {
-      int last = -1, before = 0;
+        // ---- A: advance every active edge, log the intervals
+        int32_t xo[S];
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-        r_rank[s] = 0;
-        if (s < ns) {
-          const unsigned below = smask[s] & L.lt_mask();
-          const bool surv = (smask[s] >> (NL == 32 ? L.lane : 0)) & 1u;
-          const int q = below ? s * NL + (31 - clz_(below)) : last;
-          r_rank[s] = before + Lanes::popc(below);
-          if (surv && q >= 0) {
-            const int32_t xq = sh.xf[q];
-            if (xq > r_x[s]) inv = true;
-            if (wadd(xq, sh.dxf[q]) > wadd(r_x[s], r_dx[s])) cross = true;
+        for (int s = 0; s < S; ++s) {
+          xo[s] = x[s];
+          x[s] = wadd(x[s], dx[s] >> y_shift);  // GoYShift
+        }
+        if (log) {
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            if (s == 0 || s * NL < m) {
+              uint32_t close = 0;
+              if (full == 0xFF) {
+                // edges_too_close(right edge, its successor before the step);
+                // an edge still pending starts at next_y or later
+                const int p = s * NL + L.lane;
+                int32_t nxo = 0, ndx = 0;
+                LaneNext<S>(L, xo, s, &nxo);
+                LaneNext<S>(L, dx, s, &ndx);
+                if (p + 1 < m && wadd(x[s], kFixed1) >= wsub(nxo, iabs_(ndx))) close = kRecClose;
+              }
+              if (off[s] >= 0) {
+                const int at = off[s] + nrec;
+                (&sh.xa[0][0])[at] = xo[s];
+                (&sh.xb[0][0])[at] = x[s];
+                (&sh.dy[0][0])[at] = dy[s];
+                if (off[s] >= R) sh.meta[at - R] = meta | close | (off[s] == R ? kRecFirst : 0u);
+              }
+            }
           }
-          before += Lanes::popc(smask[s]);
-          if (smask[s]) last = s * NL + (31 - clz_(smask[s]));
         }
-      }
-      m2 = before;
-    }
-    const bool any_inv = L.ballot(inv) != 0;
-    if (SKC_COLD(any_inv)) {
-      // Some survivor moved left of an earlier one.  The reference ripples
-      // each such edge backwards (backward_insert_edge_based_on_x), which
-      // leaves the survivors stably sorted by new x; its crossing check then
-      // compares an edge with its predecessor at that moment: the latest
-      // (in sorted order) earlier-listed survivor whose x is not greater.
-      // Sort the survivors' (x, list position) keys in place by odd-even
-      // transposition (the list is nearly sorted, so few phases run), then
-      // find each one's predecessor by a short backward scan.
-      int32_t* kx = sh.p_x;
-      int32_t* kp = sh.p_idx;
+
+        // ---- pieces that end in the step: the next quad piece, or the edge's end
+        if (next_y >= lmin) {
+          changed = true;
+#pragma unroll 1
+          for (int s = 0; s * NL < m; ++s) {  // one copy of the update for all slots
+            const int32_t ls = SlotGet<S>(low, s), ws = SlotGet<S>(wc, s);
+            if (s * NL + L.lane < m && ls <= next_y && WcCount(ws) > 0) {
+              const int slot = WcSlot(ws);
+              Edge e;
+              RegQuadGet(sh, slot, &e);
+              e.x = SlotGet<S>(x, s);
+              e.y = next_y;
+              e.dx = SlotGet<S>(dx, s);
+              e.dy = SlotGet<S>(dy, s);
+              e.lower_y = ls;
+              e.winding = (int8_t)WcWinding(ws);
+              e.curve_count = (int8_t)WcCount(ws);
+              e.curve_shift = (uint8_t)WcShift(ws);
+#pragma unroll 1
+              while (e.lower_y <= next_y && e.curve_count > 0) {
+                e.snapped_x = e.x;  // KeepContinuous (sw_edge.cc:294-297)
+                e.snapped_y = e.y;
+                if (!UpdateQuad(&e)) break;
+              }
+              RegQuadPut(sh, slot, e);
+              SlotSet<S>(x, s, e.x);
+              SlotSet<S>(dx, s, e.dx);
+              SlotSet<S>(dy, s, e.dy);
+              SlotSet<S>(low, s, e.lower_y);
+              SlotSet<S>(wc, s, MakeWc(e.winding, e.curve_count, e.curve_shift, slot));
+              const int o = SlotGet<S>(off, s);
+              if (log && o >= 0 && o < R) (&sh.xb[0][0])[o + nrec] = e.x;
+            }
+          }
+        }
+        if (SKC_COLD(final_in && log))
+          RegTrailing<M, S>(L, sh, x, dx, low, off, next_y, m, nr, nrec, meta, left_clip);
+        if (next_y >= lmin) {
+          // ---- the edges that go on, in list order
+          unsigned smask[S];
+          int m2 = 0;
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (s < ns && p < m && sh.surv[p]) {
-          kx[r_rank[s]] = r_x[s];
-          kp[r_rank[s]] = p;
+          for (int s = 0; s < S; ++s) {
+            smask[s] = L.ballot(s * NL + L.lane < m && low[s] > next_y);
+            m2 += Lanes::popc(smask[s]);
+          }
+          if (m2 != m) {
+            int r0 = 0, d0 = n_free;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+              if (s == 0 || s * NL < m) {
+                const int p = s * NL + L.lane;
+                const unsigned gone = L.ballot(p < m) & ~smask[s];
+                if ((smask[s] >> (NL == 32 ? L.lane : 0)) & 1u)
+                  RegStage<M>(sh, r0 + Lanes::popc(smask[s] & L.lt_mask()), x[s], dx[s], dy[s],
+                              low[s], wc[s]);
+                else if (p < m)
+                  sh.free_slot[d0 + Lanes::popc(gone & L.lt_mask())] = (uint8_t)WcSlot(wc[s]);
+                r0 += Lanes::popc(smask[s]);
+                d0 += Lanes::popc(gone);
+              }
+            }
+            n_free = d0;
+            m = m2;
+            L.sync();
+            RegLoad<M, S>(L, sh, m, x, dx, dy, low, wc);
+            L.sync();
+          }
+        }
+        if (log) nrec += K;
+
+        // ---- C: the list in stable order of the new x; intersections
+        bool inv = false, crs = false;
+        {
+          int32_t sum[S];
+#pragma unroll
+          for (int s = 0; s < S; ++s) sum[s] = wadd(x[s], dx[s]);
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            if (s == 0 || s * NL < m) {
+              const int p = s * NL + L.lane;
+              int32_t px = 0, ps = 0;
+              LanePrevOf<S>(L, x, s, &px);
+              LanePrevOf<S>(L, sum, s, &ps);
+              if (p > 0 && p < m) {
+                inv = inv || px > x[s];
+                crs = crs || ps > sum[s];
+              }
+            }
+          }
+        }
+        if (L.ballot(inv || crs)) {
+          if (L.ballot(inv)) {
+            crs = RegSort<M, S>(L, sh, m, x, dx, dy, low, wc);
+            changed = true;
+          }
+          cross = L.ballot(crs) != 0;
+        }
+        y = next_y;
+        if (y >= y_stop) {
+          done = true;
+          break;
         }
       }
-      L.sync();
-      bool dirty_prev = true;
-      for (int phase = 0; phase < m2 + 2; ++phase) {
-        bool swapped = false;
-        for (int i = 2 * L.lane + (phase & 1); i + 1 < m2; i += 2 * NL) {
-          const int32_t xa = kx[i], xb = kx[i + 1];
-          const int32_t pa = kp[i], pb = kp[i + 1];
-          if (xb < xa || (xb == xa && pb < pa)) {
-            kx[i] = xb;
-            kx[i + 1] = xa;
-            kp[i] = pb;
-            kp[i + 1] = pa;
-            swapped = true;
+
+      // ---- D: insert_new_edges (sw_raster.cc:207-247) as a merge
+      if (pend_y <= y) {
+        int c = 0;
+#pragma unroll 1
+        for (int base = k; base < n; base += NL) {
+          const int i = base + L.lane;
+          const unsigned mask = L.ballot(i < n && W[i].upper_y <= y);
+          c += Lanes::popc(mask);
+          if (mask != kFull) break;
+        }
+        if (SKC_COLD(m + c > M)) return 0;
+        // the first new edge goes after every active edge with x <= its x,
+        // each later one after the one before it and the active edges with
+        // smaller x
+        const int32_t x0 = W[k].x;
+        int before[S];  // new edges before each active one
+#pragma unroll
+        for (int s = 0; s < S; ++s) before[s] = x[s] > x0 ? 1 : 0;
+#pragma unroll 1
+        for (int tb = 0; tb < c; tb += NL) {
+          const int t = tb + L.lane;
+          Edge e;
+          int np = 0;
+          if (t < c) e = W[k + t];
+          const int32_t xt_mine = t < c ? e.x : 0;
+          const int tn = min_(NL, c - tb);
+#pragma unroll 1
+          for (int j = 0; j < tn; ++j) {
+            const int32_t xt = LaneBcast(L, xt_mine, j);
+            const bool first = tb + j == 0;
+            int cnt = 0;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+              if (s == 0 || s * NL < m) {
+                const bool act = s * NL + L.lane < m;
+                cnt += Lanes::popc(L.ballot(act && (x[s] <= x0 || (!first && x[s] < xt))));
+                if (!first && x[s] > x0 && xt <= x[s]) before[s]++;
+              }
+            }
+            if (j == L.lane || NL == 1) np = tb + j + cnt;
+          }
+          if (t < c) {
+            const int slot = sh.free_slot[n_free - 1 - t];
+            RegStage<M>(sh, np, e.x, e.dx, e.dy, e.lower_y,
+                           MakeWc(e.winding, e.curve_count, e.curve_shift, slot) | kWcNew);
+            if (e.curve_count > 0) RegQuadPut(sh, slot, e);
+          }
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          const int p = s * NL + L.lane;
+          if (p < m) RegStage<M>(sh, p + before[s], x[s], dx[s], dy[s], low[s], wc[s]);
+        }
+        n_free -= c;
+        m += c;
+        k += c;
+        pend_y = k < n ? W[k].upper_y : kMaxS32;
+        L.sync();
+        RegLoad<M, S>(L, sh, m, x, dx, dy, low, wc);
+        bool cross2 = false;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          const int p = s * NL + L.lane;
+          if (p < m && (wc[s] & kWcNew)) {
+            wc[s] &= ~kWcNew;
+            if (p > 0 && wadd(sh.u.p.x[p - 1], sh.u.p.dx[p - 1]) > wadd(x[s], dx[s])) cross2 = true;
           }
         }
         L.sync();
-        const bool dirty = L.ballot(swapped) != 0;
-        if (!dirty && !dirty_prev) break;
-        dirty_prev = dirty;
+        if (L.ballot(cross2)) cross = true;
+        changed = true;
       }
-      cross = false;
-      for (int r = L.lane; r < m2; r += NL) {
-        const int pr = kp[r];
-        sh.ax[pr] = r;
-        int q = r - 1;
-        while (q >= 0 && kp[q] > pr) --q;
-        if (q >= 0 && wadd(kx[q], sh.dxf[kp[q]]) > wadd(kx[r], sh.dxf[pr])) cross = true;
-      }
-      L.sync();
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (s < ns && p < m && sh.surv[p]) r_rank[s] = sh.ax[p];
-      }
-      L.sync();
     }
-    lmin = LaneMin(L, lmin);
-    nny = min_(nny, lmin);
-    if (L.ballot(cross)) nny = min_(nny, next_y + (kFixed1 >> kAccuracy));
-
-    // ---- the interval left open by the last left edge (its right edge was
-    // culled): too-close test against the left edge's predecessor after the
-    // reorder (its new predecessor if it survives, else the last processed
-    // survivor before it)
-    int trailing_a = -1;
-    bool trailing_nr = false;
-    if (SKC_COLD(final_in)) {
-      const int a = sh.ia[nr];
-      const bool a_surv = sh.surv[a] != 0;
-      const int32_t xa = sh.xf[a];
-      long long key = 0;
-      bool found = false;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (s < ns && p < m && sh.surv[p]) {
-          const int32_t xi = r_x[s];
-          const bool cand = a_surv ? (p != a && (xi < xa || (xi == xa && p < a))) : p < a;
-          if (cand) {
-            const long long kk = ((long long)xi << 32) | (unsigned)p;
-            if (!found || kk > key) key = kk;
-            found = true;
-          }
-        }
-      }
-      const bool any = L.ballot(found) != 0;
-      if (!found) key = (long long)kMinS32 << 32;
-      key = LaneMax64(L, key);
-      const int32_t pred_x = any ? (int32_t)(key >> 32) : left_clip;
-      const bool tc = wadd(pred_x, kFixed1) >= wsub(xa, iabs_(sh.dxf[a]));
-      trailing_a = a;
-      trailing_nr = full == 0xFF && tc;
-    }
-
-    // ---- B: coverage of the step's intervals, in list order
-    const int row = y >> 16;
-    if (nr + (final_in ? 1 : 0) > 0 && !(row < scan_top)) {
-      RegBlit(L, sh, sink, as, pend, W, n, row, next_y, nr, m, k, full, left_clip, right_clip,
-              trailing_a, trailing_nr);
-    }
-
-    // ---- reorder the survivors into the new list (nothing moves when every
-    // edge survives in order: the rank of position p is then p)
-    if (SKC_COLD(m2 != m || any_inv)) {
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        if (s < ns && ((smask[s] >> (NL == 32 ? L.lane : 0)) & 1u)) {
-          const int r = r_rank[s];
-          sh.p_idx[r] = r_idx[s];
-          sh.p_x[r] = r_x[s];
-          sh.p_dx[r] = r_dx[s];
-          sh.p_dy[r] = r_dy[s];
-          sh.p_low[r] = r_low[s];
-          sh.p_wc[r] = r_wc[s];
-          if (kQ) {
-#pragma unroll
-            for (int j = 0; j < kRegQuadWords; ++j) sh.p_q[j][r] = r_q[s].w[j];
-          }
-        }
-      }
-      L.sync();
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (p < m2) {
-          r_idx[s] = sh.p_idx[p];
-          r_x[s] = sh.p_x[p];
-          r_dx[s] = sh.p_dx[p];
-          r_dy[s] = sh.p_dy[p];
-          r_low[s] = sh.p_low[p];
-          r_wc[s] = sh.p_wc[p];
-          if (kQ) {
-#pragma unroll
-            for (int j = 0; j < kRegQuadWords; ++j) r_q[s].w[j] = sh.p_q[j][p];
-          }
-        }
-      }
-      L.sync();
-    }
-    m = m2;
-    y = next_y;
-    if (y >= IntToFixed(stop_y)) break;
-
-    // ---- D: insert_new_edges (sw_raster.cc:207-247) as a merge
-    if (SKC_COLD(k < n && W[k].upper_y <= y)) {
-      int c = 0;
-      for (int base = k; base < n; base += NL) {
-        const int i = base + L.lane;
-        const unsigned mask = L.ballot(i < n && W[i].upper_y <= y);
-        c += Lanes::popc(mask);
-        if (mask != kFull) break;
-      }
-      if (SKC_COLD(m + c > M)) return 0;
-      const int32_t x0 = W[k].x;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (p < m) sh.ax[p] = r_x[s];
-      }
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (p < m) {
-          const int32_t xa = r_x[s];
-          int before = 0;
-          if (xa > x0) {
-            before = 1;
-            for (int t = 1; t < c; ++t) before += W[k + t].x <= xa ? 1 : 0;
-          }
-          const int np = p + before;
-          sh.p_idx[np] = r_idx[s];
-          sh.p_x[np] = r_x[s];
-          sh.p_dx[np] = r_dx[s];
-          sh.p_dy[np] = r_dy[s];
-          sh.p_low[np] = r_low[s];
-          sh.p_wc[np] = r_wc[s];
-          if (kQ) {
-#pragma unroll
-            for (int j = 0; j < kRegQuadWords; ++j) sh.p_q[j][np] = r_q[s].w[j];
-          }
-        }
-      }
-      L.sync();
-      int32_t lmin2 = kMaxS32;
-      for (int tb = 0; tb < c; tb += NL) {
-        const int t = tb + L.lane;
-        if (t < c) {
-          const Edge e = W[k + t];
-          const int32_t xt = e.x;
-          int cnt = 0;
-          for (int i = 0; i < m; ++i) {
-            const int32_t xa = sh.ax[i];
-            cnt += (xa <= x0 || (t >= 1 && xa < xt)) ? 1 : 0;
-          }
-          const int np = t + cnt;
-          sh.p_idx[np] = k + t;
-          sh.p_x[np] = e.x;
-          sh.p_dx[np] = e.dx;
-          sh.p_dy[np] = e.dy;
-          sh.p_low[np] = e.lower_y;
-          sh.p_wc[np] = MakeWc(e.winding, e.curve_count);
-          if (kQ) {
-            RegQuad q;
-            q.load(e);
-#pragma unroll
-            for (int j = 0; j < kRegQuadWords; ++j) sh.p_q[j][np] = q.w[j];
-          }
-          if (e.lower_y > y) lmin2 = min_(lmin2, e.lower_y);
-        }
-      }
-      L.sync();
-      const int mm = m + c;
-      bool cross2 = false;
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int p = s * NL + L.lane;
-        if (p < mm) {
-          r_idx[s] = sh.p_idx[p];
-          r_x[s] = sh.p_x[p];
-          r_dx[s] = sh.p_dx[p];
-          r_dy[s] = sh.p_dy[p];
-          r_low[s] = sh.p_low[p];
-          r_wc[s] = sh.p_wc[p];
-          if (kQ) {
-#pragma unroll
-            for (int j = 0; j < kRegQuadWords; ++j) r_q[s].w[j] = sh.p_q[j][p];
-          }
-          if (r_idx[s] >= k && p > 0 &&
-              wadd(sh.p_x[p - 1], sh.p_dx[p - 1]) > wadd(r_x[s], r_dx[s]))
-            cross2 = true;
-        }
-      }
-      L.sync();
-      lmin2 = LaneMin(L, lmin2);
-      nny = min_(nny, lmin2);
-      if (L.ballot(cross2)) nny = min_(nny, y + (kFixed1 >> kAccuracy));
-      m = mm;
-      k += c;
-    }
-    if (k < n && W[k].upper_y > y) nny = min_(nny, W[k].upper_y);
+    L.sync();
+    RegEmit(L, sh, sink, as, nrec, left_clip, right_clip, done);
+    nrec = 0;
+    if (done) break;
   }
-  RegBlitFlush(L, sh, sink, as, pend);
   return 1;
 }
 

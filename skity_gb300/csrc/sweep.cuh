@@ -46,13 +46,13 @@ SKC_HD int32_t LaneBcast(const Lanes& L, int32_t v, int src) {
 }
 SKC_HD int32_t LaneMin(const Lanes& L, int32_t v) {
 #ifdef SKC_WARP_LANES
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+  v = __reduce_min_sync(0xffffffffu, v);
 #endif
   return v;
 }
 SKC_HD int32_t LaneMax(const Lanes& L, int32_t v) {
 #ifdef SKC_WARP_LANES
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  v = __reduce_max_sync(0xffffffffu, v);
 #endif
   return v;
 }
@@ -318,22 +318,15 @@ SKC_HD int TrapCount(const TrapRow& t) {
   return c;
 }
 
-// Pixel i of blit_aaa_trapezoid_row (AaaRow above).
-SKC_HD void AaaSpan(Fixed ul, Fixed ur, Fixed ll, Fixed lr, Fixed lDY, Fixed rDY, uint8_t full,
-                    bool real, int i, int& x, int& len, uint8_t& a) {
-  const int L0 = FixedFloorToInt(ul), R = FixedCeilToInt(lr);
-  len = 1;
-  if (R - L0 == 1) {
-    const uint8_t t = trapezoid_to_alpha(ur - ul, lr - ll);
-    x = L0;
-    a = real ? t : partial_alpha_a(t, full);
-    return;
-  }
+// Alpha of pixel i of blit_aaa_trapezoid_row (AaaRow above), which starts at
+// the pixel of ul and is more than one pixel long.
+SKC_HD uint8_t AaaAlpha(Fixed ul, Fixed ur, Fixed ll, Fixed lr, Fixed lDY, Fixed rDY, uint8_t full,
+                        int i) {
   const int uL = FixedFloorToInt(ul), lL = FixedCeilToInt(ll);
   const int uR = FixedFloorToInt(ur), lR = FixedCeilToInt(lr);
   const bool two_left = uL + 2 == lL, two_right = uR + 2 == lR;
-  const int px = L0 + i;
-  const int n = R - L0;
+  const int px = uL + i;
+  const int n = lR - uL;
   uint8_t v = full;
   if (two_left) {
     if (i <= 1) {
@@ -357,70 +350,65 @@ SKC_HD void AaaSpan(Fixed ul, Fixed ur, Fixed ll, Fixed lr, Fixed lDY, Fixed rDY
     const uint8_t t = triangle_entry(false, ur - IntToFixed(uR), lr - IntToFixed(uR), rDY, full, px - uR);
     v = v > t ? (uint8_t)(v - t) : 0;
   }
-  x = px;
-  a = v;
+  return v;
 }
 
+// The k-th span is one of four things: the full run in the middle; a pixel of
+// a two-pixel end (a triangle, or what a triangle leaves); the only pixel of
+// a one-pixel row or end (a trapezoid); a pixel of a longer one.  Which, and
+// its parameters, are chosen first, so that the lanes of a warp meet in one
+// copy of each.
 SKC_HD void TrapSpan(const TrapRow& t, int k, int& x, int& len, uint8_t& a) {
   const Fixed joinLeft = FixedCeilToFixed(t.ll);
   const Fixed joinRite = FixedFloorToFixed(t.ur);
-  if (joinLeft > joinRite) {
-    AaaSpan(t.ul, t.ur, t.ll, t.lr, t.lDY, t.rDY, t.full, t.real, k, x, len, a);
-    return;
-  }
-  if (t.ul < joinLeft) {
-    const int n = FixedCeilToInt(joinLeft - t.ul);
-    if (n == 1) {
-      if (k == 0) {
-        const uint8_t v = trapezoid_to_alpha(joinLeft - t.ul, joinLeft - t.ll);
-        x = t.ul >> 16;
-        len = 1;
-        a = t.real ? v : partial_alpha_a(v, t.full);
-        return;
+  Fixed ul = t.ul, ur = t.ur, ll = t.ll, lr = t.lr, lDY = t.lDY, rDY = t.rDY;
+  Fixed tri = 0, triDY = 0;
+  bool two = false, rest = false;  // a two-pixel end; what the triangle leaves
+  len = 1;
+  if (joinLeft <= joinRite) {
+    const int nl = t.ul < joinLeft ? FixedCeilToInt(joinLeft - t.ul) : 0;
+    const int cl = nl <= 2 ? nl : AaaCount(t.ul, joinLeft);
+    if (k < cl) {
+      ur = lr = joinLeft;
+      rDY = kMaxS32;
+      if (nl == 2) {
+        const Fixed first = joinLeft - kFixed1 - ul;
+        two = true;
+        rest = k != 0;
+        tri = k == 0 ? first : ll - ul - first;
+        triDY = lDY;
       }
-      k -= 1;
-    } else if (n == 2) {
-      if (k < 2) {
-        const Fixed first = joinLeft - kFixed1 - t.ul;
-        x = (t.ul >> 16) + k;
-        len = 1;
-        a = k == 0 ? partial_triangle_to_alpha(first, t.lDY)
-                   : (uint8_t)(t.full - partial_triangle_to_alpha(t.ll - t.ul - first, t.lDY));
-        return;
-      }
-      k -= 2;
     } else {
-      const int c = AaaCount(t.ul, joinLeft);
-      if (k < c) {
-        AaaSpan(t.ul, joinLeft, t.ll, joinLeft, t.lDY, kMaxS32, t.full, t.real, k, x, len, a);
-        return;
+      k -= cl;
+      if (joinLeft < joinRite) {
+        if (k == 0) {
+          x = FixedFloorToInt(joinLeft);
+          len = FixedFloorToInt(joinRite - joinLeft);
+          a = t.full;
+          return;
+        }
+        k -= 1;
       }
-      k -= c;
+      ul = ll = joinRite;
+      lDY = kMaxS32;
+      if (FixedCeilToInt(lr - joinRite) == 2) {
+        const Fixed first = joinRite + kFixed1 - ur;
+        two = true;
+        rest = k == 0;
+        tri = k == 0 ? first : lr - ur - first;
+        triDY = rDY;
+      }
     }
   }
-  if (joinLeft < joinRite) {
-    if (k == 0) {
-      x = FixedFloorToInt(joinLeft);
-      len = FixedFloorToInt(joinRite - joinLeft);
-      a = t.full;
-      return;
-    }
-    k -= 1;
-  }
-  const int n = FixedCeilToInt(t.lr - joinRite);
-  if (n == 1) {
-    const uint8_t v = trapezoid_to_alpha(t.ur - joinRite, t.lr - joinRite);
-    x = joinRite >> 16;
-    len = 1;
+  x = FixedFloorToInt(ul) + k;
+  if (two) {
+    const uint8_t v = partial_triangle_to_alpha(tri, triDY);
+    a = rest ? (uint8_t)(t.full - v) : v;
+  } else if (FixedCeilToInt(lr) - FixedFloorToInt(ul) == 1) {
+    const uint8_t v = trapezoid_to_alpha(ur - ul, lr - ll);
     a = t.real ? v : partial_alpha_a(v, t.full);
-  } else if (n == 2) {
-    const Fixed first = joinRite + kFixed1 - t.ur;
-    x = (joinRite >> 16) + k;
-    len = 1;
-    a = k == 0 ? (uint8_t)(t.full - partial_triangle_to_alpha(first, t.rDY))
-               : partial_triangle_to_alpha(t.lr - t.ur - first, t.rDY);
   } else {
-    AaaSpan(joinRite, t.ur, joinRite, t.lr, kMaxS32, t.rDY, t.full, t.real, k, x, len, a);
+    a = AaaAlpha(ul, ur, ll, lr, lDY, rDY, t.full, k);
   }
 }
 
