@@ -78,7 +78,7 @@ struct DeviceBatch {
   std::vector<BandSeg> h_segs;
   bool slices_dirty = true;   // pass capacities changed: slice offsets and passes re-uploaded
   uint64_t cap_sweep = 0, cap_rows = 0, cap_bins = 0;
-  uint64_t cap_scratch = 0;
+  uint64_t slices_end = 0;    // end of the geometry slices in `scratch`
   // the launch parameters the replay graphs were recorded with
   DevBatch graph_b{};
   DevPlan graph_q{};

@@ -68,8 +68,7 @@ int LaunchGeometry(const DevBatch& b, cudaStream_t stream) {
 
 // Sweeps: one warp per pass, passes taken in the batch's sweep order
 // (longest expected sweeps first, so the long ones do not form the tail).
-// Four forms, each launched over every pass and taking the ones SweepForm
-// gives it: register forms for up to 32, 64 and 128 active edges (2 warps
+// Four forms, each taking the passes SweepForm gives it: register forms for up to 32, 64 and 128 active edges (2 warps
 // per block, each with its RegSharedT block and accumulator in shared
 // memory), then the generic sweep (4 warps per block, state in global
 // memory) for longer lists.
@@ -82,8 +81,18 @@ __device__ __forceinline__ uint32_t DynamicSmemBytes() {
   return v;
 }
 
-__device__ __forceinline__ uint32_t SweepPassAt(const DevBatch& b, uint32_t i) {
-  return b.sweep_order ? b.sweep_order[i] : i;
+// The i-th pass of a sweep form (n_passes: there is none).  A device plan
+// lists each form's passes together, and a plan that fell short sweeps
+// nothing (the host renders again with its buffers grown); without a plan the
+// form's launch goes through all passes.
+__device__ __forceinline__ uint32_t SweepPassAt(const DevBatch& b, int form, uint32_t i) {
+  if (b.plan) {
+    const uint32_t at = b.plan->form_end[form + 1] + i;
+    return (b.plan->flags || at >= b.plan->form_end[form]) ? b.n_passes : b.sweep_order[at];
+  }
+  if (i >= b.n_passes) return b.n_passes;
+  const uint32_t p = b.sweep_order ? b.sweep_order[i] : i;
+  return SweepForm(b.geom[p], b.pass_class[p]) == form ? p : b.n_passes;
 }
 
 // Lets the next overlapped launch start once every CTA of this one runs.
@@ -118,26 +127,23 @@ __global__ void __launch_bounds__(32 * kRegWarpsMax) k_sweep_reg(DevBatch b) {
   AllowNextLaunch();
   const int w = threadIdx.x >> 5;
   const uint32_t nw = blockDim.x >> 5;
-  const uint32_t i = blockIdx.x * nw + w;
-  if (i < b.n_passes) {
-    const uint32_t p = SweepPassAt(b, i);
-    if (SweepForm(b.geom[p], b.pass_class[p]) == kForm) {
-      if (DynamicSmemBytes() < nw * RegSmemBytes<M>(b.reg_diff_cap)) {  // self-check
-        FlagError(b.err, 16);
-      } else {
-        Lanes L;
-        L.lane = threadIdx.x & 31;
-        uint8_t* mine = reg_smem + (size_t)w * RegSmemBytes<M>(b.reg_diff_cap);
-        if (!SweepPassReg<M>(b, p, L, (RegSharedT<M>*)mine,
-                             (int32_t*)(mine + sizeof(RegSharedT<M>)), b.reg_diff_cap) &&
-            L.leader()) {
-          // each pass is taken by one form, so the list holds at most n_passes
-          const uint32_t at = b.sweep_retry ? atomicAdd(b.sweep_retry, 1u) : b.n_passes;
-          if (at < b.n_passes) {
-            b.sweep_retry[1 + at] = p;
-          } else {
-            FlagError(b.err, 32);  // no list: the pass stays unswept, the render fails
-          }
+  const uint32_t p = SweepPassAt(b, kForm, blockIdx.x * nw + w);
+  if (p < b.n_passes) {
+    if (DynamicSmemBytes() < nw * RegSmemBytes<M>(b.reg_diff_cap)) {  // self-check
+      FlagError(b.err, 16);
+    } else {
+      Lanes L;
+      L.lane = threadIdx.x & 31;
+      uint8_t* mine = reg_smem + (size_t)w * RegSmemBytes<M>(b.reg_diff_cap);
+      if (!SweepPassReg<M>(b, p, L, (RegSharedT<M>*)mine,
+                           (int32_t*)(mine + sizeof(RegSharedT<M>)), b.reg_diff_cap) &&
+          L.leader()) {
+        // each pass is taken by one form, so the list holds at most n_passes
+        const uint32_t at = b.sweep_retry ? atomicAdd(b.sweep_retry, 1u) : b.n_passes;
+        if (at < b.n_passes) {
+          b.sweep_retry[1 + at] = p;
+        } else {
+          FlagError(b.err, 32);  // no list: the pass stays unswept, the render fails
         }
       }
     }
@@ -160,12 +166,12 @@ __global__ void __launch_bounds__(32 * kSweepWarps) k_sweep_retry(DevBatch b) {
 template <bool kRaw>
 __global__ void __launch_bounds__(32 * kSweepWarps) k_sweep(DevBatch b) {
   AllowNextLaunch();
-  const uint32_t i = blockIdx.x * kSweepWarps + (threadIdx.x >> 5);
-  if (i < b.n_passes) {
-    const uint32_t p = SweepPassAt(b, i);
+  const uint32_t p =
+      SweepPassAt(b, kSweepGeneric, blockIdx.x * kSweepWarps + (threadIdx.x >> 5));
+  if (p < b.n_passes) {
     Lanes L;
     L.lane = threadIdx.x & 31;
-    if (SweepForm(b.geom[p], b.pass_class[p]) == kSweepGeneric) SweepPass<kRaw>(b, p, L);
+    SweepPass<kRaw>(b, p, L);
   }
   FinishOverlapped(b.sweep_done ? b.sweep_done + kSweepGeneric : nullptr);
 }

@@ -125,6 +125,29 @@ struct PassGeom {
   int32_t raw_spans;    // the pass keeps raw spans (kPassRawSpans): swept by the generic form
 };
 
+// Which sweep form takes pass p: the register form for up to 32, 64 or 128
+// active edges, or the generic form, by the geometry's bound of the active
+// list (PassGeom::max_active); pass_class != 0 forces the generic form.
+// The forms' kernels take disjoint passes and depend on nothing the others
+// write, so their launches may overlap.
+constexpr int kRegMaxM = 128;  // the largest active list held in registers
+enum : int { kSweepReg64 = 0, kSweepReg128 = 2, kSweepGeneric = 1, kSweepReg32 = 3 };
+constexpr int kSweepForms = 4;
+// pass_class of a pass no sweep form takes (nothing to sweep, or no room)
+constexpr uint8_t kSweepSkip = 4;
+// The 32-edge form runs last (lightest form) and takes only short passes,
+// so that no long sweep starts at the end of the sweep launches.
+constexpr int kReg32MaxRows = 1100;
+SKC_HD int SweepForm(const PassGeom& g, uint8_t pass_class) {
+  if (pass_class != 0) return pass_class;
+  if (g.raw_spans) return kSweepGeneric;  // the path-clip stages' passes (rare)
+  const int ma = g.max_active;
+  return (ma <= 32 && g.row1 - g.row0 <= kReg32MaxRows) ? kSweepReg32
+         : ma <= 64                                     ? kSweepReg64
+         : ma <= kRegMaxM                               ? kSweepReg128
+                                                        : kSweepGeneric;
+}
+
 struct PassSweep {      // per-pass sweep buffers, set after geometry
   uint64_t work_off;    // byte offset of the pass's sweep memory
   uint64_t bytes;       // its size
@@ -226,8 +249,6 @@ enum : uint32_t {
   kPlanRows = 4,          // row-span table short
   kPlanBins = 8,          // pass bins short
 };
-// pass_class of a pass no sweep form takes (nothing to sweep, or no room)
-constexpr uint8_t kSweepSkip = 4;
 
 struct PlanStatus {  // zeroed before each render, read back after it
   uint32_t flags;
@@ -239,6 +260,10 @@ struct PlanStatus {  // zeroed before each render, read back after it
   unsigned long long spans, edges;
   unsigned long long frags_by_brush[4];
   unsigned long long sort_total[2];  // items of the sweep and tile sorts
+  // the passes of sweep form f are [form_end[f + 1], form_end[f]) of the sweep
+  // order (the forms' keys sort in descending order)
+  uint32_t form_end[kSweepForms + 1];
+  uint32_t pad;
 };
 
 struct BandSeg {   // a pass-bin segment: the passes [p0, p1) of the band's canvas

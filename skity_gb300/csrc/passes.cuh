@@ -596,25 +596,6 @@ SKC_HD int RunRegSweep(const DevBatch& b, uint32_t p, const PassGeom& g, Sink* s
                  g.start_y, g.stop_y, g.left_bound, g.right_bound);
 }
 
-// Which sweep form takes pass p: the register form for up to 32, 64 or 128
-// active edges, or the generic form, by the geometry's bound of the active
-// list (PassGeom::max_active); pass_class != 0 forces the generic form.
-// The forms' kernels take disjoint passes and depend on nothing the others
-// write, so their launches may overlap.
-enum : int { kSweepReg64 = 0, kSweepReg128 = 2, kSweepGeneric = 1, kSweepReg32 = 3 };
-// The 32-edge form runs last (lightest form) and takes only short passes,
-// so that no long sweep starts at the end of the sweep launches.
-constexpr int kReg32MaxRows = 1100;
-SKC_HD int SweepForm(const PassGeom& g, uint8_t pass_class) {
-  if (pass_class != 0) return pass_class;
-  if (g.raw_spans) return kSweepGeneric;  // the path-clip stages' passes (rare)
-  const int ma = g.max_active;
-  return (ma <= 32 && g.row1 - g.row0 <= kReg32MaxRows) ? kSweepReg32
-         : ma <= 64                                     ? kSweepReg64
-         : ma <= kRegMaxM                               ? kSweepReg128
-                                                        : kSweepGeneric;
-}
-
 // Sweep of pass p through the register form of size M.  Returns false when
 // its active list outgrows M after all: the caller then sweeps the pass with
 // the generic form (SweepPass, which clears the rows the attempt wrote).

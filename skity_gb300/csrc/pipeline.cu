@@ -288,9 +288,13 @@ static int32_t PrepareDevice(skity_cuda_context_s* ctx, DeviceBatch& db, DevBatc
       total += L.bytes;
     }
     if (ctx->budget && total > ctx->budget) return SKITY_CUDA_ERROR_OUT_OF_DEVICE_MEMORY;
-    SKC_TRY(db.scratch.ensure(std::max<uint64_t>(total, 16)));
+    // with room behind the slices for those that outgrow their estimate
+    uint64_t want = total + total / 32 + (1u << 20);
+    if (ctx->budget) want = std::max(total, std::min(want, ctx->budget));
+    SKC_TRY(db.scratch.ensure(want));
     SKC_TRY(Upload(db.passes, hb.passes, s));
     db.slices_dirty = false;
+    db.slices_end = total;
   }
   SKC_TRY(db.geom.ensure(npm * sizeof(PassGeom)));
   SKC_TRY(db.sweep.ensure(npm * sizeof(PassSweep)));
@@ -494,11 +498,19 @@ static int32_t DeviceRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool tim
   st.passes = np;
   const uint64_t kMaxPool = 0xFFFFFFFFull;  // span indices are 32-bit
   double discarded_ms = 0;
+  bool all = true;             // the geometry of every pass is to run, else of
+  std::vector<uint32_t> todo;  // these (the others' stands from the attempt before)
   for (int attempt = 0; attempt < 8; ++attempt) {
     DevBatch b;
     DevPlan q;
     int32_t rc = PrepareDevice(ctx, db, b, q);
     if (rc) return rc;
+    DevBatch eb = b;
+    if (!all) {
+      SKC_TRY(Upload(db.pass_list, todo, s));
+      eb.pass_list = db.pass_list.as<uint32_t>();
+      eb.n_list = (uint32_t)todo.size();
+    }
     const bool replay = db.graph_ok && std::memcmp(&b, &db.graph_b, sizeof b) == 0 &&
                         std::memcmp(&q, &db.graph_q, sizeof q) == 0;
     int launches = 0;
@@ -508,7 +520,7 @@ static int32_t DeviceRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool tim
     } else {
       for (int part = 0; part < 6; ++part) {
         SKC_TRY(cudaEventRecord(ctx->stage[2 * part], s));
-        launches += EnqueueDevice(db, b, q, ctx->num_sms, s, part);
+        launches += EnqueueDevice(db, eb, q, ctx->num_sms, s, part);
         SKC_TRY(cudaEventRecord(ctx->stage[2 * part + 1], s));
       }
     }
@@ -555,13 +567,30 @@ static int32_t DeviceRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool tim
     DropReplay(db);
     discarded_ms += ElapsedMs(ctx->ev0, ctx->ev1);
     st.retries++;
+    todo.clear();
+    all = false;
     if (ps.flags & kPlanGeomOverflow) {
+      // the passes that outgrew their slices get new ones behind the others,
+      // and only they run again; without room there, all slices move
       db.h_geom.resize(np);
       SKC_TRY(cudaMemcpy(db.h_geom.data(), db.geom.p, (size_t)np * sizeof(PassGeom),
                          cudaMemcpyDeviceToHost));
-      for (uint32_t p = 0; p < np; ++p)
-        if (db.h_geom[p].status) GrowCaps(hb.passes[p], db.h_geom[p]);
-      db.slices_dirty = true;
+      uint64_t end = db.slices_end;
+      for (uint32_t p = 0; p < np; ++p) {
+        if (!db.h_geom[p].status) continue;
+        GrowCaps(hb.passes[p], db.h_geom[p]);
+        SliceLayout L;
+        L.compute(hb.passes[p].cap, sizeof(Edge));
+        hb.passes[p].slice_off = end;
+        end += L.bytes;
+        todo.push_back(p);
+      }
+      if (end <= db.scratch.cap) {
+        db.slices_end = end;
+        SKC_TRY(Upload(db.passes, hb.passes, s));
+      } else {
+        all = db.slices_dirty = true;
+      }
     }
     if (ps.sweep_need > db.cap_sweep) db.cap_sweep = ps.sweep_need + ps.sweep_need / 8;
     if (ps.rows_need > db.cap_rows) db.cap_rows = ps.rows_need + ps.rows_need / 8;

@@ -5,8 +5,9 @@
 //   k_scan2         1 block         : exclusive prefix sums (u64) of both
 //   k_plan_place    1 thread / pass : PassSweep, PassComp, sweep form, band
 //                                     range
-//   k_sort_*        sweep order     : passes by expected sweep length, longest
-//                                     first (stable bucket sort)
+//   k_sort_*        sweep order     : passes by sweep form, then by expected
+//                                     sweep length, longest first (stable
+//                                     bucket sort)
 //   k_bin_count     1 warp / segment: passes meeting a band (warp ballots)
 //   k_scan2         1 block         : segment offsets
 //   k_bin_fill      1 warp / segment: the bins, draw order kept by ballot ranks
@@ -50,16 +51,23 @@ __device__ __forceinline__ void PassNeeds(const PassGeom& g, unsigned long long*
   *rows = has ? (unsigned long long)nr : 0ull;
 }
 
-// Sort key of a work estimate: 0 for no work, else 8 buckets per octave
-// (1 + 8 floor(log2 c) + the next three bits of c), at most kSortBuckets - 1:
-// the orders below are by work to within about 9%, ties in index order.
-constexpr uint32_t kSortBuckets = 512;
-__device__ __forceinline__ uint32_t WorkBucket(unsigned long long c) {
+// Sort key of a work estimate: 0 for no work, else 2^kBits buckets per octave
+// (1 + 2^kBits floor(log2 c) + the next kBits bits of c), at most `buckets` -
+// 1: the tile order below is by work to within about 9% (3 bits), the sweep
+// order to within 19% (2 bits), ties in index order.
+constexpr uint32_t kSortBuckets = 512;    // of a work estimate, tiles
+constexpr uint32_t kSweepBuckets = 128;   // of a work estimate, sweeps
+// the sweep order's keys: kSweepBuckets per form, the forms in the order of
+// kFormRank (the passes no form takes last)
+constexpr uint32_t kSweepKeys = (kSweepForms + 1) * kSweepBuckets;
+template <uint32_t kBits>
+__device__ __forceinline__ uint32_t WorkBucket(unsigned long long c, uint32_t buckets) {
   if (!c) return 0u;
   const uint32_t e = 63u - (uint32_t)__clzll(c);
-  const uint32_t sub = e >= 3 ? (uint32_t)(c >> (e - 3)) & 7u : (uint32_t)(c << (3 - e)) & 7u;
-  const uint32_t k = 1u + 8u * e + sub;
-  return k < kSortBuckets ? k : kSortBuckets - 1u;
+  const uint32_t mask = (1u << kBits) - 1u;
+  const uint32_t sub = (e >= kBits ? (uint32_t)(c >> (e - kBits)) : (uint32_t)(c << (kBits - e))) & mask;
+  const uint32_t k = 1u + (e << kBits) + sub;
+  return k < buckets ? k : buckets - 1u;
 }
 
 __global__ void __launch_bounds__(kPlanThreads) k_plan_sizes(DevBatch b, DevPlan q) {
@@ -239,31 +247,37 @@ __global__ void __launch_bounds__(32 * kBinWarps) k_bin_fill(DevPlan q) {
 // histograms, one prefix sum over (key descending, block), then each block
 // places its items, warp by warp, ranking equal keys inside a warp with
 // __match_any_sync.
+constexpr uint32_t kMaxSortKeys = 2 * kSortBuckets;
+static_assert(kSweepKeys <= kMaxSortKeys, "shared histograms");
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 2048;
 
-// Key of item i: kind 0 the sweep of pass i (rows x (1 + active-list bound)),
-// kind 1 compositor tile i (passes in its band's bin + 1) x its width; the
+// Key of item i: kind 0 the sweep of pass i (its form, then rows x (1 +
+// active-list bound): each form's launch takes its own passes, longest first,
+// so no warp of a CTA waits out a pass of another form), kind 1 compositor tile i (passes in its band's bin + 1) x its width; the
 // temp canvases' tiles (i >= n_main) sort after every main tile.
 __device__ __forceinline__ uint32_t SortKey(const DevBatch& b, const DevPlan& q, int kind,
                                             uint32_t i) {
   if (kind == 0) {
     const PassGeom g = b.geom[i];
     const unsigned long long rows = b.sweep[i].bytes ? (unsigned long long)(g.row1 - g.row0) : 0ull;
-    return WorkBucket(rows * (unsigned long long)(1 + (g.max_active > 0 ? g.max_active : 0)));
+    const int form = SweepForm(g, b.pass_class[i]);
+    const uint32_t k = WorkBucket<2>(
+        rows * (unsigned long long)(1 + (g.max_active > 0 ? g.max_active : 0)), kSweepBuckets);
+    return (form < kSweepForms ? (uint32_t)(1 + form) * kSweepBuckets : 0u) + k;
   }
   const RowTask t = q.tasks_in[i];
   const CanvasDesc& cd = b.canvases[t.canvas];
   const uint32_t band = cd.band0 + (t.y >> b.band_shift);
   const unsigned long long n = q.band_off[band + 1] - q.band_off[band];
-  const uint32_t k = WorkBucket((n + 1ull) * (unsigned long long)(t.x1 - t.x0));
+  const uint32_t k = WorkBucket<3>((n + 1ull) * (unsigned long long)(t.x1 - t.x0), kSortBuckets);
   return i < q.n_main ? kSortBuckets + k : k;
 }
 
 // hist[(nb - 1 - key) * nblocks + block] = items of the block with that key
 __global__ void __launch_bounds__(kSortThreads)
     k_sort_hist(DevBatch b, DevPlan q, int kind, uint32_t n, uint32_t nb) {
-  __shared__ uint32_t h[2 * kSortBuckets];
+  __shared__ uint32_t h[kMaxSortKeys];
   for (uint32_t k = threadIdx.x; k < nb; k += kSortThreads) h[k] = 0;
   __syncthreads();
   const uint32_t i0 = blockIdx.x * kSortItems;
@@ -281,9 +295,17 @@ __global__ void __launch_bounds__(kSortThreads)
 
 __global__ void __launch_bounds__(kSortThreads)
     k_sort_place(DevPlan q, int kind, uint32_t n, uint32_t nb) {
-  __shared__ uint32_t cur[2 * kSortBuckets];
+  __shared__ uint32_t cur[kMaxSortKeys];
   for (uint32_t k = threadIdx.x; k < nb; k += kSortThreads)
     cur[k] = (uint32_t)q.sort_hist[(unsigned long long)(nb - 1 - k) * gridDim.x + blockIdx.x];
+  // Where the sweep forms' passes are in the sweep order.  Form f's keys are
+  // [1 + f, 2 + f) x kSweepBuckets, so its passes end where the largest key
+  // below them starts: a prefix sum of the sort.
+  if (kind == 0 && blockIdx.x == 0 && threadIdx.x <= (unsigned)kSweepForms) {
+    const uint32_t key = threadIdx.x * kSweepBuckets + kSweepBuckets - 1;
+    q.st->form_end[threadIdx.x] =
+        (uint32_t)q.sort_hist[(unsigned long long)(nb - 1 - key) * gridDim.x];
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
@@ -364,7 +386,7 @@ int LaunchPlan(const DevBatch& b, const DevPlan& q, cudaStream_t s) {
     k_plan_sizes<<<Blocks(np, kPlanThreads), kPlanThreads, 0, s>>>(b, q);
     k_scan2<<<1, kScanThreads, 0, s>>>(q.a, q.r, np, &q.st->sweep_need, &q.st->rows_need);
     k_plan_place<<<Blocks(np, kPlanThreads), kPlanThreads, 0, s>>>(b, q);
-    n += 3 + LaunchSort(b, q, 0, np, kSortBuckets, s);
+    n += 3 + LaunchSort(b, q, 0, np, kSweepKeys, s);
   }
   if (q.n_segs) {
     k_bin_count<<<Blocks(q.n_segs, kBinWarps), 32 * kBinWarps, 0, s>>>(q);

@@ -29,11 +29,11 @@
 // A path whose active list would exceed M edges (the form's size) is not swept here
 // (RegWalk returns 0) and goes to LaneSweep.
 #pragma once
+#include "kernels.cuh"
 #include "sweep.cuh"
 
 namespace skc {
 
-constexpr int kRegMaxM = 128;  // the largest active list held in registers
 // Interval records the walk logs before they are emitted: a step with at
 // most M active edges logs at most M / 2 + 1.
 SKC_HD constexpr int RegRecords(int M) { return M == 32 ? 64 : M; }
