@@ -307,21 +307,36 @@ SKC_HD uint32_t GradientColor(const Brush& b, float current, const float4* color
   if (stop_count > 0 && current <= o[0]) {
     out = c[0];
   } else {
-    float step = 1.f / (color_count - 1);
-    int i = 0, si = 0, ei = 1;
+    // the first interval whose ends are on either side of `current` (with
+    // offsets: searched without an early exit, so the lanes of a warp take the
+    // same loop)
+    int i = color_count - 1, si = 0, ei = 1;
     float start = 0.f, end = 0.f;
-    for (i = 0; i < color_count - 1; i++) {
-      if (stop_count > 0) {
-        start = o[i];
-        end = o[i + 1];
-      } else {
-        start = step * i;
-        end = step * (i + 1);
+    if (stop_count > 0) {
+      float lo = o[0];
+#pragma unroll 2
+      for (int k = 0; k < color_count - 1; k++) {
+        const float hi = o[k + 1];
+        i = min_(i, current >= lo && current <= hi ? k : color_count - 1);
+        lo = hi;
       }
-      if (current >= start && current <= end) {
+      if (i < color_count - 1) {
         si = i;
         ei = i + 1;
-        break;
+        start = o[si];
+        end = o[ei];
+      }
+    } else {
+      const float step = 1.f / (color_count - 1);
+#pragma unroll 1
+      for (i = 0; i < color_count - 1; i++) {
+        start = step * i;
+        end = step * (i + 1);
+        if (current >= start && current <= end) {
+          si = i;
+          ei = i + 1;
+          break;
+        }
       }
     }
     if (i == color_count - 1 && color_count > 0) {
@@ -339,6 +354,104 @@ SKC_HD uint32_t GradientColor(const Brush& b, float current, const float4* color
     }
   }
   return ColorToPMColor(Color4fToColor(out.x, out.y, out.z, out.w));
+}
+
+// A gradient's stops as a compositor warp keeps them in shared memory: the
+// offsets and colours, the correctly rounded reciprocal of each interval's
+// length, and for 32 cells of [0, 1] the first interval a parameter in the
+// cell can lie in.
+struct StagedStops {
+  float4* colors;   // [kStagedStops]
+  float* offsets;   // [kStagedStops]
+  float* recip;     // [kStagedStops]
+  uint8_t* first;   // [32]
+};
+
+// Whether GradientColorStaged takes a gradient, stop by stop: finite colours,
+// offsets within [-4, 4] that do not descend (a NaN is neither), intervals
+// that are empty or long enough for its division.
+SKC_HD bool StagedStop(float4 c, float o, float next) {
+  const float big = 1e30f;
+  return fabs_(c.x) <= big && fabs_(c.y) <= big && fabs_(c.z) <= big && fabs_(c.w) <= big &&
+         fabs_(o) <= 4.0f && o <= next && (o == next || next - o >= 1.0f / (1 << 20));
+}
+SKC_HD uint32_t FirstInterval(const float* offsets, int n, int cell) {
+  int i = 0;
+  const float at = cell * (1.0f / 32);
+  if (cell > 0)
+    while (i < n - 2 && offsets[i + 1] < at) ++i;
+  return (uint32_t)i;
+}
+
+// value / total, correctly rounded, from r = 1 / total correctly rounded:
+// after one Newton step the quotient is faithful, and a second one with the
+// then exact residual rounds it correctly (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990).  For
+// total in [2^-20, 8] and value in [1e-15, total] no step leaves the normal
+// range.
+SKC_HD float DivByRecip(float value, float total, float r) {
+#ifdef __CUDA_ARCH__
+  float q = value * r;
+  q = __fmaf_rn(__fmaf_rn(-q, total, value), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, total, value), r, q);
+#else
+  float q = value * r;
+  q = fmaf(fmaf(-q, total, value), r, q);
+  return fmaf(fmaf(-q, total, value), r, q);
+#endif
+}
+
+SKC_HD float Saturate(float v) {
+#ifdef __CUDA_ARCH__
+  return __saturatef(v);
+#else
+  return v > 0.f ? (v < 1.f ? v : 1.f) : 0.f;
+#endif
+}
+
+// GradientColor over staged stops (`n` of them, with offsets): the same
+// colour.  The interval is searched from its cell's first one; the channels
+// are clamped before they are scaled by 255 instead of after (the same byte:
+// 255 v is exact in order, and past the ends both give 0 or 255), and red and
+// blue are premultiplied in one word.
+SKC_HD uint32_t GradientColorStaged(uint32_t tile, int n, float current, const StagedStops& st) {
+  const float kNZ = 1.0f / (1 << 12);
+  if (fabs_(current) <= kNZ) {
+    current = 0.0f;
+  } else if (fabs_(current - 1.0f) <= kNZ) {
+    current = 1.0f;
+  }
+  if (tile == 3 && (current < 0.0f || current >= 1.0f)) return 0;
+  current = RemapFloatTile(current, tile);
+  int i = 0;
+  float mix = 0.0f;
+  if (!(current <= st.offsets[0])) {
+    const int cell = (int)min_(max_(current * 32.0f, 0.0f), 31.0f);
+    i = st.first[cell];
+    while (i < n - 1 && !(current <= st.offsets[i + 1])) ++i;
+    if (i < n - 1) {
+      const float start = st.offsets[i], total = st.offsets[i + 1] - start;
+      const float value = current - start;
+      mix = 0.5f;
+      if (total > 0) mix = value >= 1e-15f ? DivByRecip(value, total, st.recip[i]) : value / total;
+    }
+  }
+  float4 c = st.colors[i];
+  if (mix != 0.0f) {
+    const float4 e = st.colors[i + 1];
+    const float om = 1 - mix;
+    c.x = c.x * om + e.x * mix;
+    c.y = c.y * om + e.y * mix;
+    c.z = c.z * om + e.z * mix;
+    c.w = c.w * om + e.w * mix;
+  }
+  const uint32_t a = (uint32_t)(Saturate(c.w) * 255), r = (uint32_t)(Saturate(c.x) * 255);
+  const uint32_t g = (uint32_t)(Saturate(c.y) * 255), b = (uint32_t)(Saturate(c.z) * 255);
+  // MulDiv255Round by a: 255 leaves a channel as it is
+  uint32_t rb = ((r << 16) | b) * a + 0x800080u;
+  rb = ((rb + ((rb >> 8) & 0xFF00FFu)) >> 8) & 0xFF00FFu;
+  const uint32_t gg = MulDiv255Round(g, a);
+  return (a << 24) | rb | (gg << 8);
 }
 
 // SweepGradientColorBrush::CalculateColor's parameter (sw_span_brush.cc:
@@ -500,8 +613,8 @@ SKC_HD uint32_t BrushColorCommon(const Brush& b, int x, int y, const float4* col
   float sx = x + 0.5f, sy = y + 0.5f;
   float mx = sx * b.m[0] + sy * b.m[1] + b.m[2];
   float my = sx * b.m[3] + sy * b.m[4] + b.m[5];
-  if (b.kind == 1) return GradientColor(b, mx, colors, offsets);
-  if (b.kind == 2) return GradientColor(b, sqrt_(mx * mx + my * my), colors, offsets);
+  if (b.kind == 1 || b.kind == 2)
+    return GradientColor(b, b.kind == 1 ? mx : sqrt_(mx * mx + my * my), colors, offsets);
   if (mx < 0.0f || mx >= 1.0f || my < 0.0f || my >= 1.0f) return 0;
   uint32_t ix = (uint32_t)(mx * (float)b.img_w), iy = (uint32_t)(my * (float)b.img_h);
   ix = min_(ix, b.img_w - 1);
@@ -517,8 +630,8 @@ SKC_HD uint32_t BrushColor(const Brush& b, int x, int y, const float4* colors, c
   float sx = x + 0.5f, sy = y + 0.5f;
   float mx = sx * b.m[0] + sy * b.m[1] + b.m[2];
   float my = sx * b.m[3] + sy * b.m[4] + b.m[5];
-  if (b.kind == 1) return GradientColor(b, mx, colors, offsets);
-  if (b.kind == 2) return GradientColor(b, sqrt_(mx * mx + my * my), colors, offsets);
+  if (b.kind == 1 || b.kind == 2)
+    return GradientColor(b, b.kind == 1 ? mx : sqrt_(mx * mx + my * my), colors, offsets);
   if (b.kind == 6) return ImageShaderColor(mx, my, b.tile, b.img_w, b.img_h, images + b.img_off);
   if (b.kind >= 4)
     return OtherGradientColor(b.kind, b.tile, b.stop_count, b.has_offsets, b.stop0, b.bias, b.scale,

@@ -230,32 +230,39 @@ int LaunchSweep(const DevBatch& b, cudaStream_t stream) {
 // shared memory.  The passes come from the row band's bin (draw order); each
 // pass row's spans are loaded 32 at a time, the ones meeting the tile are
 // applied in emission order, in batches of disjoint spans (every pixel's
-// blends stay in the reference's order).
+// blends stay in the reference's order).  A batch's pixels are numbered
+// through its spans and taken 32 at a time, whatever their spans' lengths, so
+// the lanes stay full: a lane finds its pixel's span from a bit mask of the
+// span starts among the 32.  (With short spans on a lane each and long ones
+// by the whole warp in turn, 3.45 warp instructions a solid fragment.)
 // ---------------------------------------------------------------------------
 constexpr int kCompWarps = 4;
 // CTAs per SM the compositor's register budget leaves room for (its stalls
 // are mostly dependent integer chains: more resident warps hide them)
 constexpr int kCompMinBlocks = 6;
-// spans up to this many tile pixels are shaded by one lane
-constexpr int kShortSpan = 4;
 
 // gradient stops a warp stages in shared memory (longer gradients are read
 // from global memory)
 constexpr int kStagedStops = 16;
 // shared memory of one compositor warp: its tile row, padded to 16 bytes (a
 // tile may be any number of pixels wide, the stop colours are read as
-// float4), then the staged stops
+// float4), then the staged stops (colours, offsets, reciprocals, cells), then
+// a batch's spans (two words each)
 __host__ __device__ constexpr size_t CompRowBytes(uint32_t chunk) {
   return ((size_t)chunk * 4 + 15) & ~(size_t)15;
 }
 __host__ __device__ constexpr size_t CompWarpSmem(uint32_t chunk) {
-  return CompRowBytes(chunk) + kStagedStops * (16 + 4);
+  return CompRowBytes(chunk) + kStagedStops * (16 + 4 + 4) + 32 + 32 * 8;
 }
+struct CompShared {  // the parts of a warp's shared memory
+  uint32_t* row;
+  StagedStops stops;
+  uint2* spans;
+};
 
 template <bool kAll>
-__device__ __forceinline__ void CompositeTile(const DevBatch& b, const RowTask& rt, uint32_t* row,
-                                              float4* stage_colors, float* stage_offsets,
-                                              int lane);
+__device__ __forceinline__ void CompositeTile(const DevBatch& b, const RowTask& rt,
+                                              const CompShared& sh, int lane);
 
 // counter == null: warp w of block k takes tile 4k + w; otherwise every warp
 // takes tiles from the counter until none is left (persistent grid).
@@ -273,12 +280,16 @@ __global__ void __launch_bounds__(32 * kCompWarps, kCompMinBlocks)
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   uint8_t* mine = reg_smem + (size_t)wib * CompWarpSmem(chunk);
-  uint32_t* row = (uint32_t*)mine;
-  float4* stage_colors = (float4*)(mine + CompRowBytes(chunk));
-  float* stage_offsets = (float*)(stage_colors + kStagedStops);
+  CompShared sh;
+  sh.row = (uint32_t*)mine;
+  sh.stops.colors = (float4*)(mine + CompRowBytes(chunk));
+  sh.stops.offsets = (float*)(sh.stops.colors + kStagedStops);
+  sh.stops.recip = sh.stops.offsets + kStagedStops;
+  sh.stops.first = (uint8_t*)(sh.stops.recip + kStagedStops);
+  sh.spans = (uint2*)(sh.stops.first + 32);
   if (!counter) {
     const uint32_t task = blockIdx.x * kCompWarps + wib;
-    if (task < n_tasks) CompositeTile<kAll>(b, tasks[task], row, stage_colors, stage_offsets, lane);
+    if (task < n_tasks) CompositeTile<kAll>(b, tasks[task], sh, lane);
     return;
   }
   for (;;) {
@@ -286,103 +297,186 @@ __global__ void __launch_bounds__(32 * kCompWarps, kCompMinBlocks)
     if (lane == 0) task = atomicAdd(counter, 1u);
     task = __shfl_sync(0xffffffffu, task, 0);
     if (task >= n_tasks) return;
-    CompositeTile<kAll>(b, tasks[task], row, stage_colors, stage_offsets, lane);
+    CompositeTile<kAll>(b, tasks[task], sh, lane);
     __syncwarp();
   }
 }
 
-// The spans [s0, s1) of one pass row applied to the row tile.  kAll: every
-// brush kind, colour filter and blend mode; otherwise the common ones only
-// (solid, linear, radial and image brushes; clear, src, dst, src-over).
-template <bool kAll>
-__device__ __forceinline__ void CompositeSpans(const DevBatch& b, const Brush& br,
-                                               const float4* stop_colors,
-                                               const float* stop_offsets, uint32_t s0,
-                                               uint32_t s1, int x0, int x1, int y, uint32_t* row,
+// The head of a brush: what solid fills need.
+struct BrushHead {
+  uint32_t kind, blend, solid, global_alpha;
+};
+
+// How a pass's pixels are made.
+//   solid:    a src-over fill without a colour filter: the span's colour is
+//             made once a span, and a pixel is one PMSrcOver.  FastBlend's
+//             shortcuts need no test: premultiplied colours of alpha 0 are 0,
+//             and 256 - alpha is 1 for alpha 255, which leaves nothing of the
+//             destination.
+//   gradient: a linear or radial one, src-over, no colour filter, whose stops
+//             GradientColorStaged takes; blended the same way.
+//   other:    everything else, pixel by pixel as the reference does it.
+enum CompKind { kCompSolid, kCompGradient, kCompOther };
+
+// The spans [s0, s1) of one pass row applied to the row tile; `mine`: this
+// lane's span of the first 32, already loaded.
+template <bool kAll, int kKind>
+__device__ __forceinline__ void CompositeSpans(const DevBatch& b, const BrushHead& bh,
+                                               const Brush& br, const CompShared& sh, uint2 mine,
+                                               uint32_t s0, uint32_t s1, int x0, int x1, int y,
                                                int lane) {
-  const uint2* sp = b.spans;
+  uint32_t* row = sh.row;
+  const uint32_t le = (2u << lane) - 1u;
+  const float4* stop_colors = b.stop_colors;
+  const float* stop_offsets = b.stop_offsets;
+  // one pixel; v: the span's colour (solid) or alpha
+  auto pixel = [&](int px, uint32_t v) {
+    uint32_t& d = row[px];
+    if (kKind == kCompSolid) {
+      d = PMSrcOver(v, d);
+    } else if (kKind == kCompGradient) {
+      const float sx = (px + x0) + 0.5f, sy = y + 0.5f;
+      const float mx = sx * br.m[0] + sy * br.m[1] + br.m[2];
+      float t = mx;
+      if (br.kind == 2) {
+        const float my = sx * br.m[3] + sy * br.m[4] + br.m[5];
+        t = sqrt_(mx * mx + my * my);
+      }
+      uint32_t c = GradientColorStaged(br.tile, (int)br.stop_count, t, sh.stops);
+      if (v != 255) c = AlphaMulQ(c, v);
+      d = PMSrcOver(c, d);
+    } else {
+      uint32_t c = kAll ? BrushColor(br, px + x0, y, stop_colors, stop_offsets, b.pixels,
+                                     b.roundtrip, b.conicals)
+                        : BrushColorCommon(br, px + x0, y, stop_colors, stop_offsets, b.pixels,
+                                           b.roundtrip);
+      if (v != 255) c = AlphaMulQ(c, v);
+      if (kAll && br.cf_type) c = FilterColor(br, c, b.srgb_tables, b.cf_matrices);
+      d = kAll ? BlendPixel(d, c, br.blend) : BlendPixelCommon(d, c, br.blend);
+    }
+  };
+#pragma unroll 1
   for (uint32_t sb = s0; sb < s1; sb += 32) {
     int xs = 0, xe = 0;
-    uint32_t alpha = 0;
-    bool pending = false;
+    uint32_t v = 0;
     if (sb + lane < s1) {
-      const uint2 mine = sp[sb + lane];
-      const int sx = (int)(mine.x & 0xFFFF), slen = (int)(mine.x >> 16);
-      xs = max(sx, x0);
-      xe = min(sx + slen, x1);
-      alpha = mine.y & br.global_alpha;
-      pending = xs < xe;
+      xs = max((int)(mine.x & 0xFFFF), x0);
+      xe = min((int)(mine.x & 0xFFFF) + (int)(mine.x >> 16), x1);
+      v = mine.y & bh.global_alpha;
+      if (kKind == kCompSolid) v = v != 255 ? AlphaMulQ(bh.solid, v) : bh.solid;
     }
-    // Spans are applied in batches: the longest run of pending spans
-    // (in emission order) in which each starts at or after the end of
-    // the one before.  Those are disjoint, so inside a batch the order
-    // does not matter: short spans are shaded by their own lane, long
-    // ones by the whole warp (pixel column mod 32 per lane).
-    uint32_t pmask = __ballot_sync(0xffffffffu, pending);
+    if (sb + 32 + lane < s1) mine = b.spans[sb + 32 + lane];
+    // Spans are applied in batches: the longest run of pending spans (in
+    // emission order) in which each starts at or after the end of the one
+    // before.  Those are disjoint, so inside a batch the order does not
+    // matter.
+    uint32_t pmask = __ballot_sync(0xffffffffu, xs < xe);
+#pragma unroll 1
     while (pmask) {
-      const uint32_t below = pmask & ((1u << lane) - 1u);
-      const int prev = below ? 31 - __clz(below) : lane;
-      const int prev_xe = __shfl_sync(0xffffffffu, xe, prev);
-      const bool clash = pending && below && prev_xe > xs;
-      const uint32_t cmask = __ballot_sync(0xffffffffu, clash);
+      const bool pending = (pmask >> lane) & 1u;
+      const uint32_t below = pmask & (le >> 1);
+      const int prev_xe = __shfl_sync(0xffffffffu, xe, below ? 31 - __clz(below) : lane);
+      const uint32_t cmask = __ballot_sync(0xffffffffu, pending && below && prev_xe > xs);
       const uint32_t batch = cmask ? pmask & ((1u << (__ffs(cmask) - 1)) - 1u) : pmask;
-      const bool mine_now = (batch >> lane) & 1u;
-      const bool is_short = xe - xs <= kShortSpan;
-      if (mine_now && is_short) {
-        for (int x = xs; x < xe; ++x) {
-          uint32_t c = kAll ? BrushColor(br, x, y, stop_colors, stop_offsets, b.pixels,
-                                         b.roundtrip, b.conicals)
-                            : BrushColorCommon(br, x, y, stop_colors, stop_offsets, b.pixels,
-                                               b.roundtrip);
-          if (alpha != 255) c = AlphaMulQ(c, alpha);
-          if (kAll && br.cf_type) c = FilterColor(br, c, b.srgb_tables, b.cf_matrices);
-          uint32_t& d = row[x - x0];
-          d = kAll ? BlendPixel(d, c, br.blend) : BlendPixelCommon(d, c, br.blend);
+      const bool now = (batch >> lane) & 1u;
+      int len = now ? xe - xs : 0;
+      int at = xs - x0;
+      // whole blocks of 32 pixels of the long spans, a lane a pixel
+      if (kKind != kCompOther) {
+        uint32_t lmask = __ballot_sync(0xffffffffu, len >= 32);
+#pragma unroll 1
+        while (lmask) {
+          const int j = __ffs(lmask) - 1;
+          lmask &= lmask - 1;
+          const int q = __shfl_sync(0xffffffffu, at, j) + lane;
+          const int n = __shfl_sync(0xffffffffu, len, j) & ~31;
+          const uint32_t qv = __shfl_sync(0xffffffffu, v, j);
+#pragma unroll 1
+          for (int i = 0; i < n; i += 32) pixel(q + i, qv);
         }
+        at += len & ~31;
+        len &= 31;
+        __syncwarp();
       }
-      uint32_t lmask = __ballot_sync(0xffffffffu, mine_now && !is_short);
-      while (lmask) {
-        const int j = __ffs(lmask) - 1;
-        lmask &= lmask - 1;
-        const int qs = __shfl_sync(0xffffffffu, xs, j);
-        const int qe = __shfl_sync(0xffffffffu, xe, j);
-        const uint32_t qa = __shfl_sync(0xffffffffu, alpha, j);
-        for (int x = qs + ((lane - qs) & 31); x < qe; x += 32) {
-          uint32_t c = kAll ? BrushColor(br, x, y, stop_colors, stop_offsets, b.pixels,
-                                         b.roundtrip, b.conicals)
-                            : BrushColorCommon(br, x, y, stop_colors, stop_offsets, b.pixels,
-                                               b.roundtrip);
-          if (qa != 255) c = AlphaMulQ(c, qa);
-          if (kAll && br.cf_type) c = FilterColor(br, c, b.srgb_tables, b.cf_matrices);
-          uint32_t& d = row[x - x0];
-          d = kAll ? BlendPixel(d, c, br.blend) : BlendPixelCommon(d, c, br.blend);
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      const int excl = incl - len;
+      // the pixels left over, numbered through the batch's spans (packed:
+      // pixel - number, colour or alpha) and taken 32 at a time
+      const uint32_t some = kKind != kCompOther ? __ballot_sync(0xffffffffu, len > 0) : batch;
+      if ((some >> lane) & 1u)
+        sh.spans[__popc(some & (le >> 1))] = make_uint2((uint32_t)(at - excl), v);
+      __syncwarp();
+      int before = -1;  // spans that start before the 32 pixels, less one
+#pragma unroll 1
+      for (int w = 0; w < total; w += 32) {
+        const uint32_t rel = (uint32_t)(excl - w);
+        const uint32_t starts =
+            __reduce_or_sync(0xffffffffu, (len > 0 && rel < 32u) ? 1u << rel : 0u);
+        const int g = w + lane;
+        if (g < total) {
+          const uint2 sp = sh.spans[before + __popc(starts & le)];
+          pixel((int)sp.x + g, sp.y);
         }
+        before += __popc(starts);
       }
       __syncwarp();
-      if (mine_now) pending = false;
       pmask &= ~batch;
     }
   }
 }
 
+// Stages a gradient's stops for a warp; whether GradientColorStaged takes it.
+__device__ __forceinline__ bool StageStops(const DevBatch& b, const Brush& br,
+                                           const StagedStops& st, int lane) {
+  const int n = (int)br.stop_count;
+  if (n < 2 || n > kStagedStops || !br.has_offsets) return false;
+  float4 c = make_float4(0, 0, 0, 0);
+  float o = 0;
+  if (lane < n) {
+    c = b.stop_colors[br.stop0 + lane];
+    o = b.stop_offsets[br.stop0 + lane];
+  }
+  const float next = __shfl_down_sync(0xffffffffu, o, 1);
+  const bool fits = lane >= n || StagedStop(c, o, lane < n - 1 ? next : o);
+  if (!__all_sync(0xffffffffu, fits)) return false;
+  __syncwarp();
+  if (lane < n) {
+    st.colors[lane] = c;
+    st.offsets[lane] = o;
+    st.recip[lane] = 1.0f / (next - o);
+  }
+  __syncwarp();
+  st.first[lane] = (uint8_t)FirstInterval(st.offsets, n, lane);
+  __syncwarp();
+  return true;
+}
+
 template <bool kAll>
-__device__ __forceinline__ void CompositeTile(const DevBatch& b, const RowTask& rt, uint32_t* row,
-                                              float4* stage_colors, float* stage_offsets,
-                                              int lane) {
+__device__ __forceinline__ void CompositeTile(const DevBatch& b, const RowTask& rt,
+                                              const CompShared& sh, int lane) {
   const CanvasDesc cd = b.canvases[rt.canvas];
   const int y = (int)rt.y;
   const int x0 = (int)rt.x0, x1 = (int)rt.x1;
   const int n = x1 - x0;
+  uint32_t* row = sh.row;
   uint32_t* gpx = (uint32_t*)(b.pixels + cd.px_off) + (size_t)y * cd.w + x0;
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     row[i] = cd.has_clear ? cd.clear_pm : RGBAtoARGB(gpx[i]);
   }
   __syncwarp();
   const uint32_t band = cd.band0 + ((uint32_t)y >> b.band_shift);
   const uint32_t e0 = b.band_off[band], e1 = b.band_off[band + 1];
-  // 32 bin entries at a time: each lane looks up its pass's row entry, so
-  // the row-table loads of 32 passes are in flight together and passes
-  // with no spans on this row cost no serial step
+  // 32 bin entries at a time: each lane looks up its pass's row entry and
+  // brush, so the loads of 32 passes are in flight together and passes with
+  // no spans on this row cost no serial step
+#pragma unroll 1
   for (uint32_t eb = e0; eb < e1; eb += 32) {
     const uint32_t e = eb + lane;
     uint2 rs = make_uint2(0, 0);
@@ -394,32 +488,54 @@ __device__ __forceinline__ void CompositeTile(const DevBatch& b, const RowTask& 
         brush = pc.brush;
       }
     }
+    BrushHead bh = {0, 0, 0, 0};
+    if (rs.y != 0) {
+      const Brush& q = b.brushes[brush];
+      bh.kind = q.kind;
+      bh.blend = q.blend;
+      bh.solid = q.solid;
+      bh.global_alpha = q.global_alpha;
+    }
     uint32_t mask = __ballot_sync(0xffffffffu, rs.y != 0);
+    // the first 32 spans of a pass are loaded while the pass before is blended
+    auto first_spans = [&](uint32_t m) {
+      const int bit = m ? __ffs(m) - 1 : 0;
+      const uint32_t f0 = __shfl_sync(0xffffffffu, rs.x, bit);
+      const uint32_t fn = __shfl_sync(0xffffffffu, rs.y, bit);
+      uint2 v = make_uint2(0, 0);
+      if (m && lane < (int)min(fn, 32u)) v = b.spans[f0 + lane];
+      return v;
+    };
+    uint2 next = first_spans(mask);
+#pragma unroll 1
     while (mask) {
       const int bit = __ffs(mask) - 1;
       mask &= mask - 1;
+      const uint2 mine = next;
+      next = first_spans(mask);
       const uint32_t s0 = __shfl_sync(0xffffffffu, rs.x, bit);
       const uint32_t s1 = s0 + __shfl_sync(0xffffffffu, rs.y, bit);
       const uint32_t qbrush = __shfl_sync(0xffffffffu, brush, bit);
-      Brush br = b.brushes[qbrush];
-      const float4* stop_colors = b.stop_colors;
-      const float* stop_offsets = b.stop_offsets;
-      if ((br.kind == 1 || br.kind == 2) && br.stop_count <= (uint32_t)kStagedStops) {
-        // the gradient's stops, read for every pixel, staged in shared memory
-        __syncwarp();
-        if (lane < (int)br.stop_count) {
-          stage_colors[lane] = b.stop_colors[br.stop0 + lane];
-          stage_offsets[lane] = b.stop_offsets[br.stop0 + lane];
-        }
-        __syncwarp();
-        stop_colors = stage_colors;
-        stop_offsets = stage_offsets;
-        br.stop0 = 0;
+      BrushHead qh;
+      qh.kind = __shfl_sync(0xffffffffu, bh.kind, bit);
+      qh.blend = __shfl_sync(0xffffffffu, bh.blend, bit);
+      qh.solid = __shfl_sync(0xffffffffu, bh.solid, bit);
+      qh.global_alpha = __shfl_sync(0xffffffffu, bh.global_alpha, bit);
+      Brush br;
+      if (qh.kind == 0 && qh.blend == 3 && (!kAll || b.brushes[qbrush].cf_type == 0)) {
+        CompositeSpans<kAll, kCompSolid>(b, qh, br, sh, mine, s0, s1, x0, x1, y, lane);
+        continue;
       }
-      CompositeSpans<kAll>(b, br, stop_colors, stop_offsets, s0, s1, x0, x1, y, row, lane);
+      br = b.brushes[qbrush];
+      if ((qh.kind == 1 || qh.kind == 2) && qh.blend == 3 && (!kAll || br.cf_type == 0) &&
+          StageStops(b, br, sh.stops, lane))
+        CompositeSpans<kAll, kCompGradient>(b, qh, br, sh, mine, s0, s1, x0, x1, y, lane);
+      else
+        CompositeSpans<kAll, kCompOther>(b, qh, br, sh, mine, s0, s1, x0, x1, y, lane);
     }
   }
   __syncwarp();
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) gpx[i] = ARGBtoRGBA(row[i]);
 }
 
