@@ -280,9 +280,13 @@ SKC_HD float RemapFloatTile(float t, uint32_t tile) {  // sw_span_brush.cc:21-32
   } else if (tile == 1) {
     t = t - floor_(t);
   } else if (tile == 2) {
-    // float - 2 * std::floor(float * 0.5) - 1 evaluates in double
+    // float - 2 * std::floor(float * 0.5) - 1 evaluates in double; below 2^20
+    // the whole number it takes off is a float, and one float subtraction
+    // rounds the same difference
     float t1 = t - 1;
-    float t2 = (float)((double)t1 - 2.0 * floor((double)t1 * 0.5) - 1.0);
+    float t2 = fabs_(t1) < 1048576.0f
+                   ? t1 - (2.0f * floor_(t1 * 0.5f) + 1.0f)
+                   : (float)((double)t1 - 2.0 * floor((double)t1 * 0.5) - 1.0);
     t = fabs_(t2);
   }
   return t;

@@ -66,6 +66,7 @@ struct DeviceBatch {
   std::vector<uint32_t> h_band_off, h_bins;
   uint32_t chunk = 1024;
   uint32_t n_bands = 0;
+  uint32_t any_stroke = 0;  // a pass is stroked
   RasterConfig cfg;
   DevBuf task_next;  // persistent compositor's counters
   DevBuf retry;      // DevBatch::sweep_retry

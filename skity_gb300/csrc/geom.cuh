@@ -9,6 +9,7 @@
 // on the CPU against std::sort and the oracle.
 #pragma once
 #include <stdint.h>
+#include <cmath>
 #include <vector_types.h>  // float4 / uint2 on host builds too
 
 // branch hints: SKC_COLD(c) for conditions that are rarely true on the hot
@@ -20,7 +21,6 @@
 #define SKC_HD __host__ __device__ __forceinline__
 #define SKC_HDN inline __host__ __device__ __noinline__
 #else
-#include <cmath>
 #define SKC_HD inline
 #define SKC_HDN inline
 #endif
@@ -30,6 +30,20 @@ namespace skc {
 // ---------------------------------------------------------------------------
 // math shims (same IEEE operations on host and device)
 // ---------------------------------------------------------------------------
+SKC_HD float fma_(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  return __fmaf_rn(a, b, c);
+#else
+  return std::fma(a, b, c);
+#endif
+}
+SKC_HD float rsqrt_(float x) {  // within a few units in the last place
+#ifdef __CUDA_ARCH__
+  return rsqrtf(x);
+#else
+  return 1.0f / std::sqrt(x);
+#endif
+}
 #ifdef __CUDACC__
 SKC_HD float fabs_(float x) { return fabsf(x); }
 SKC_HD float sqrt_(float x) { return sqrtf(x); }
@@ -408,15 +422,32 @@ SKC_HD double CubicQuadCountD(const P c[4]) {
   P p2x2 = mkP(c[2].x * 3.f - c[3].x, c[2].y * 3.f - c[3].y);
   P d = mkP(p2x2.x - p1x2.x, p2x2.y - p1x2.y);
   float err = d.x * d.x + d.y * d.y;
+  // The ceiling is known from a float power unless that is close to a whole
+  // number (double arithmetic runs at 1/64 of the float rate): exp2f and
+  // log2f are within 4e-7 of it for these exponents.
+  if (err > 1e-20f && err < 1e20f) {
+    const float v = exp2f(log2f(err * (float)(1.0 / max_hypot2)) * (1.0f / 6.0f));
+    const float c = ceil_(v), slack = 1e-4f * c;
+    if (c - v > slack && v - (c - 1.0f) > slack) return max_(1., (double)c);
+  }
   return max_(1., ceild_(pow_(err / max_hypot2, 1. / 6.0)));
 }
 
 // Cubic::ToQuads, quad i of quad_count (cubic.cc:42-61)
 SKC_HD void CubicQuadAt(const P c[4], const CubicCoeff& cc, const QuadCoeff& qc,
                         double quad_count, int i, P out[3]) {
-  double t0d = i / quad_count;
-  double t1d = (i + 1) / quad_count;
-  float t1 = (float)t0d, t2 = (float)t1d;
+  // (float)(i / quad_count) in double: i / n of whole numbers below 2^20 is too
+  // far from any float's rounding boundary for the double rounding to show, so
+  // the float division gives it
+  float t1, t2;
+  if (quad_count < 1048576.0) {
+    const float n = (float)quad_count;
+    t1 = (float)i / n;
+    t2 = (float)(i + 1) / n;
+  } else {
+    t1 = (float)(i / quad_count);
+    t2 = (float)((i + 1) / quad_count);
+  }
   P s0 = cc.eval(t1);
   P s3 = cc.eval(t2);
   float scale = (t2 - t1) * (1.f / 3.f);

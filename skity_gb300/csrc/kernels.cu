@@ -1,8 +1,8 @@
 // GB300 kernels of the raster pipeline.
 //
-//   k_geometry   1 thread / pass : Path -> QuadPath (-> stroke -> QuadPath)
-//                                  (1 to 32 passes a warp by the batch's size)
-//                                  -> fixed-point edges -> introsort
+//   k_stroke     1 warp / pass   : stroked passes: Path -> QuadPath -> outline
+//   k_edges      1 warp / pass   : Path (or outline) -> QuadPath -> fixed-point
+//                                  edges -> introsort
 //   k_sweep_*    1 warp / pass   : analytic-AA sweep (register form, generic
 //                                  form for very long active lists) writing
 //                                  each row's spans contiguously into the
@@ -12,9 +12,9 @@
 //                                  tile, then writes the tile back
 //   k_blur_h/_v  1 thread / row / column of each blur temp canvas: StackBlur
 //
-// Geometry and sweeps are inherently sequential per path (the reference's
-// scanline sweep carries state across rows), so the parallelism there is
-// across paths; compositing is parallel across rows and, inside a row,
+// The stroker and the sweeps are inherently sequential per path (the
+// reference's scanline sweep carries state across rows), so the parallelism
+// there is across paths; compositing is parallel across rows and, inside a row,
 // across pixels with a fixed lane per pixel column (no cross-lane hazards).
 #include <cuda_runtime.h>
 
@@ -26,44 +26,40 @@
 
 namespace skc {
 
-// Geometry: lanes [0, lanes) of each warp take a pass each, the others idle.
-// A pass's chain is long and branchy (curve subdivision, the stroker, edge
-// set-up, the sort), so the lanes of a warp diverge on almost every verb:
-// packing 32 passes a warp costs the least issue when there are passes
-// enough to fill the GPU many times over, while a batch of few passes
-// finishes sooner with fewer per warp (its time is its longest chains').
-// Measured on the GB300: 32 a warp for the 256-canvas batch (135,670
-// passes: 6.1 ms against 26.0 at 1), 8 for the 20,000-path scene (36.0 ms
-// against 42.8 at 32), 1 for the 305-path tiger picture (7.8 ms against 10.2).
-__global__ void __launch_bounds__(128) k_geometry(DevBatch b, uint32_t lanes) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t lane = t & 31;
-  if (lane >= lanes) return;
-  const uint32_t i = (t >> 5) * lanes + lane;
+// Geometry, a warp a pass (edges.cuh): the stroker of the stroked passes, then
+// quads, edges and sort.  With the whole chain on one thread, packed 1 to 32
+// passes a warp, it was the batch's longest passes' serial chains, and half of
+// a stroke's was double arithmetic (1/64 of the float rate).  Before / after:
+// the 20,000-path scene 36.4 / 6.8 ms, 64 canvases of fills 3.3 / 0.84, a
+// picture of 305 long outlines 32.7 / 5.6, 512x512 of 1,000 fills 0.70 / 0.09.
+constexpr int kGeomWarps = 4;
+__global__ void __launch_bounds__(32 * kGeomWarps) k_stroke(DevBatch b) {
+  const uint32_t i = blockIdx.x * kGeomWarps + (threadIdx.x >> 5);
   if (i >= b.n_list) return;
-  GeometryPass(b, b.pass_list ? b.pass_list[i] : i);
+  Lanes L;
+  L.lane = threadIdx.x & 31;
+  StrokePass(b, b.pass_list ? b.pass_list[i] : i, L);
 }
 
-// Passes per warp: n / (16 warps per SM over the SMs), a power of two in [1, 32].
-static uint32_t GeometryLanes(uint32_t n) {
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-    cudaGetLastError();
-    sms = 152;
-  }
-  const uint32_t per = n / (16u * (uint32_t)sms);
-  uint32_t lanes = 1;
-  while (lanes < 32 && lanes * 2 <= per) lanes *= 2;
-  return lanes;
+__global__ void __launch_bounds__(32 * kGeomWarps) k_edges(DevBatch b) {
+  __shared__ SortShared sh[kGeomWarps];
+  const uint32_t i = blockIdx.x * kGeomWarps + (threadIdx.x >> 5);
+  if (i >= b.n_list) return;
+  Lanes L;
+  L.lane = threadIdx.x & 31;
+  EdgesPass(b, b.pass_list ? b.pass_list[i] : i, L, &sh[threadIdx.x >> 5]);
 }
 
 int LaunchGeometry(const DevBatch& b, cudaStream_t stream) {
   if (b.n_list == 0) return 0;
-  const uint32_t lanes = GeometryLanes(b.n_list);
-  const uint32_t warps = (b.n_list + lanes - 1) / lanes;
-  k_geometry<<<(warps + 3) / 4, 128, 0, stream>>>(b, lanes);
-  return 1;
+  const uint32_t grid = (b.n_list + kGeomWarps - 1) / kGeomWarps;
+  int n = 1;
+  if (b.any_stroke) {
+    k_stroke<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
+    n++;
+  }
+  k_edges<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
+  return n;
 }
 
 // Sweeps: one warp per pass, passes taken in the batch's sweep order

@@ -194,8 +194,9 @@ struct DevBatch {
   const float* stop_offsets;
   uint8_t* pixels;
   const uint8_t* roundtrip;
-  const uint32_t* pass_list;  // passes to (re)run in the geometry kernel
+  const uint32_t* pass_list;  // passes to (re)run in the geometry kernels
   uint32_t n_list;
+  uint32_t any_stroke;  // a pass is stroked: the stroker's kernel runs
   uint8_t* pass_class;  // sweep form per pass: 0 register sweep, 1 generic
   int32_t reg_diff_cap; // accumulator entries per warp in shared memory
   const uint32_t* band_off;  // per band: first entry in bins (one past the end follows)

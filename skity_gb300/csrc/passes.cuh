@@ -3,182 +3,21 @@
 // __global__ wrappers in kernels.cu).
 #pragma once
 #include "kernels.cuh"
+#include "edges.cuh"
 #include "stroke.cuh"
 #include "regsweep.cuh"
 
 namespace skc {
 
-// ---------------------------------------------------------------------------
-// geometry: Path -> QuadPath (-> stroke -> QuadPath) -> edges -> introsort
-// ---------------------------------------------------------------------------
+// The whole geometry of a pass on one thread (the CPU execution of the
+// pipeline; the GPU runs its two parts on a warp each, kernels.cu).
 SKC_HDN void GeometryPass(const DevBatch& b, uint32_t p) {
-  const PassDesc pd = b.passes[p];
-  const DrawDesc dd = b.draws[pd.draw];
-  PassGeom g;
-  g.status = 0;
-  g.n_edges = 0;
-  g.start_y = g.stop_y = 0;
-  g.left_bound = g.right_bound = 0;
-  g.acc_left = g.acc_width = 0;
-  g.scan_top = 0;
-  g.row0 = g.row1 = 0;
-  g.raw_spans = (pd.flags & kPassRawSpans) != 0 ? 1 : 0;
-  for (int k = 0; k < 13; ++k) g.need[k] = 0;
-  g.max_active = 0;
-
-  SliceLayout L;
-  L.compute(pd.cap, sizeof(Edge));
-  uint8_t* base = b.scratch + pd.slice_off;
-  PathView src;
-  src.verbs = b.verbs + dd.v0;
-  src.pts = b.pts + dd.p0;
-  src.w = b.weights + dd.w0;
-  src.nv = (int)dd.nv;
-  src.np = (int)dd.np;
-  src.nw = (int)dd.nw;
-
-  DPath q1;
-  q1.init(base + L.off[0], pd.cap[0], (P*)(base + L.off[1]), pd.cap[1], (float*)(base + L.off[2]),
-          pd.cap[2]);
-  QuadPath(src, &q1);
-  g.need[0] = q1.nv;
-  g.need[1] = q1.np;
-  g.need[2] = q1.nw;
-  if (q1.overflow()) {
-    g.status = 1;
-    b.geom[p] = g;
-    return;
-  }
-  PathView quad = q1.view();
-  DPath q2;
-  if (pd.flags & kPassStroke) {
-    DPath outer, inner;
-    outer.init(base + L.off[3], pd.cap[3], (P*)(base + L.off[4]), pd.cap[4],
-               (float*)(base + L.off[5]), pd.cap[5]);
-    inner.init(base + L.off[6], pd.cap[6], (P*)(base + L.off[7]), pd.cap[7],
-               (float*)(base + L.off[8]), pd.cap[8]);
-    int imax[3];
-    StrokePath(q1.view(), pd.stroke_width, pd.miter, (int)(pd.cap_join & 0xFF),
-               (int)(pd.cap_join >> 8), &outer, &inner, imax);
-    g.need[3] = outer.nv;
-    g.need[4] = outer.np;
-    g.need[5] = outer.nw;
-    g.need[6] = imax[0];
-    g.need[7] = imax[1];
-    g.need[8] = imax[2];
-    if (outer.overflow() || imax[0] > pd.cap[6] || imax[1] > pd.cap[7] || imax[2] > pd.cap[8]) {
-      g.status = 1;
-      b.geom[p] = g;
-      return;
-    }
-    q2.init(base + L.off[9], pd.cap[9], (P*)(base + L.off[10]), pd.cap[10],
-            (float*)(base + L.off[11]), pd.cap[11]);
-    QuadPath(outer.view(), &q2);
-    g.need[9] = q2.nv;
-    g.need[10] = q2.np;
-    g.need[11] = q2.nw;
-    if (q2.overflow()) {
-      g.status = 1;
-      b.geom[p] = g;
-      return;
-    }
-    quad = q2.view();
-  }
-  const Xform xf = PassXform(pd);
-  RasterBounds rb = pd.clipped
-                        ? ComputeBounds(quad, xf, pd.clip[0], pd.clip[1], pd.clip[2], pd.clip[3])
-                        : ComputeBounds(quad, xf);
-  if (rb.empty) {
-    b.geom[p] = g;
-    return;
-  }
-  Edge* edges = (Edge*)(base + L.off[12]);
-  int n = BuildEdges(quad, xf, rb.st, rb.sb, edges, pd.cap[12]);
-  g.need[12] = n;
-  if (n > pd.cap[12]) {
-    g.status = 1;
-    b.geom[p] = g;
-    return;
-  }
-  if (n == 0) {
-    b.geom[p] = g;
-    return;
-  }
-  int32_t* idx = (int32_t*)(base + L.off[14]);
-  for (int i = 0; i < n; ++i) idx[i] = i;
-  EdgeLess less;
-  less.e = edges;
-  introsort(idx, n, less);
-  Edge* S = (Edge*)(base + L.off[13]);
-  for (int i = 0; i < n; ++i) {
-    S[i] = edges[idx[i]];
-    S[i].prev = i == 0 ? n : i - 1;
-    S[i].next = i + 1 == n ? n + 1 : i + 1;
-  }
-  // ProcessEdges sentinels (sw_raster.cc:706-729)
-  Edge h;
-  h.prev = -1;
-  h.next = 0;
-  h.upper_y = h.lower_y = kMinS32;
-  h.x = kMinS32;
-  h.dx = 0;
-  h.dy = kMaxS32;
-  h.upper_x = kMinS32;
-  h.y = 0;
-  h.curve_count = 0;
-  h.curve_shift = 0;
-  h.winding = 0;
-  Edge tl = h;
-  tl.prev = n - 1;
-  tl.next = -1;
-  tl.upper_y = tl.lower_y = kMaxS32;
-  tl.x = kMaxS32;
-  tl.upper_x = kMaxS32;
-  S[n] = h;
-  S[n + 1] = tl;
-  // Bound of the sweep's active list: an edge joins it at upper_y and
-  // leaves after its last piece, so the list never holds more edges than
-  // the largest overlap of the [upper_y, last y) ranges.
-  {
-    int32_t* low = idx;  // free after the copy above
-    for (int i = 0; i < n; ++i)
-      low[i] = S[i].curve_count != 0 ? max_(S[i].lower_y, S[i].q_last_y) : S[i].lower_y;
-    IntLess il;
-    introsort(low, n, il);
-    int cur = 0, best = 0;
-    for (int i = 0, j = 0; i < n;) {
-      if (j < n && low[j] <= S[i].upper_y) {
-        --cur;
-        ++j;
-      } else {
-        best = max_(best, ++cur);
-        ++i;
-      }
-    }
-    g.max_active = best;
-  }
-
-  const CanvasDesc cd = b.canvases[pd.canvas];
-  g.n_edges = n;
-  g.start_y = (int)rb.t;
-  g.stop_y = (int)rb.sb;
-  // static_cast<uint32_t>(float) << 16 with x86-64 conversion semantics
-  g.left_bound = (Fixed)((uint32_t)(int64_t)rb.sl << 16);
-  g.right_bound = (Fixed)((uint32_t)(int64_t)rb.sr << 16);
-  g.acc_left = (int)rb.l;
-  g.acc_width = (int)(rb.r - rb.l);
-  g.scan_top = rb.st;
-  // canvas rows; a ClipPath pass keeps all of its rows (the clip's span list
-  // is empty or not over all rows, SWCanvas::State::HasClip)
-  const bool all_rows = (pd.flags & kPassClipPath) != 0;
-  int r0 = all_rows ? g.start_y : max_(g.start_y, 0), r1 = all_rows ? g.stop_y : min_(g.stop_y, (int)cd.h);
-  if (r0 < r1) {
-    g.row0 = r0;
-    g.row1 = r1;
-  }
-  b.geom[p] = g;
+  Lanes lanes;
+  lanes.lane = 0;
+  SortShared sh;
+  StrokePass(b, p, lanes);
+  EdgesPass(b, p, lanes, &sh);
 }
-
 
 // ---------------------------------------------------------------------------
 // sweep: the span sink and the sweep passes

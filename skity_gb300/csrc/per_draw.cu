@@ -4,7 +4,7 @@
 // src/render/sw/sw_canvas.cc:357-411).  Per draw, on one stream and with no
 // host round trip:
 //
-//   k_geometry        the draw's passes (fill and / or stroke)
+//   k_stroke, k_edges the draw's passes (fill and / or stroke)
 //   k_draw_plan       1 thread: the passes' sweep memory, row tables and
 //                     sweep form, the span pool reset
 //   k_sweep_*         the sweep forms (each takes the passes of its form)
@@ -252,6 +252,8 @@ int32_t RenderPerDraw(skity_cuda_context_s* ctx, DeviceBatch& db) {
         v.passes = db.passes.as<PassDesc>() + p0;
         v.n_passes = k;
         v.n_list = k;
+        v.any_stroke = 0;
+        for (uint32_t i = p0; i < p1; ++i) v.any_stroke |= hb.passes[i].flags & kPassStroke;
         v.geom = db.geom.as<PassGeom>() + p0;
         v.sweep = db.sweep.as<PassSweep>() + p0;
         v.comp = db.comp.as<PassComp>() + p0;

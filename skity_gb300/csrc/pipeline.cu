@@ -77,6 +77,8 @@ int32_t UploadBatch(skity_cuda_context_s* ctx, DeviceBatch& db) {
   SKC_TRY(Upload(db.pts, hb.pts, s));
   SKC_TRY(Upload(db.weights, hb.weights, s));
   SKC_TRY(Upload(db.draws, hb.draws, s));
+  db.any_stroke = 0;
+  for (const PassDesc& pd : hb.passes) db.any_stroke |= pd.flags & kPassStroke;
   db.cfg = ctx->cfg;
   db.n_bands = AssignBands(hb, db.cfg.band_shift);
   SKC_TRY(Upload(db.canvases, hb.canvases, s));
@@ -147,6 +149,7 @@ static int EnqueuePlanned(skity_cuda_context_s* ctx, DeviceBatch& db, cudaStream
   const uint32_t np = b.n_passes;
   b.pass_list = nullptr;
   b.n_list = np;
+  b.any_stroke = db.any_stroke;
   switch (part) {
     case 0:
       if (!db.keep_pixels) {
@@ -342,6 +345,7 @@ static int32_t PrepareDevice(skity_cuda_context_s* ctx, DeviceBatch& db, DevBatc
   b.passes = db.passes.as<PassDesc>();
   b.n_passes = np;
   b.n_list = np;
+  b.any_stroke = db.any_stroke;
   b.canvases = db.canvases.as<CanvasDesc>();
   b.scratch = db.scratch.as<uint8_t>();
   b.geom = db.geom.as<PassGeom>();
@@ -698,6 +702,7 @@ static int32_t PlanAndRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool ti
     b.geom = db.geom.as<PassGeom>();
     b.pass_list = db.pass_list.as<uint32_t>();
     b.n_list = (uint32_t)todo.size();
+    b.any_stroke = db.any_stroke;
     SKC_TRY(cudaEventRecord(ctx->stage[0], s));
     st.kernel_launches += LaunchGeometry(b, s);
     SKC_TRY(cudaEventRecord(ctx->stage[1], s));

@@ -7,9 +7,8 @@
 
 namespace skc {
 
-// SWEdge / SWQuadEdge (sw_edge.hpp:18-81), list links as indices
+// SWEdge / SWQuadEdge (sw_edge.hpp:18-81) without the list links
 struct Edge {
-  int32_t prev, next;
   Fixed x, y, dx, dy, upper_x, upper_y, lower_y;
   int8_t curve_count;
   uint8_t curve_shift;
@@ -69,11 +68,20 @@ SKC_HD bool SetLine(Edge* e, P p0, P p1) {  // sw_edge.cc:18-43
   e->curve_shift = 0;
   return UpdateLine(e, x0, y0, x1, y1, slope);
 }
-SKC_HD bool CanBeIgnored(float top, float bottom, Fixed y0, Fixed y1) {  // :72-88
+// CanBeIgnored (:72-88): the edge [y0, y1] lies outside the scan bounds
+// [top, bottom], each as ScanFixed gives it.
+SKC_HD Fixed ScanFixed(float y) {
   const int mul = 1 << kAccuracy;
-  Fixed start_y = SnapY(FDot6ToFixed(ScalarToFDot6(top * mul)) >> kAccuracy);
-  Fixed stop_y = SnapY(FDot6ToFixed(ScalarToFDot6(bottom * mul)) >> kAccuracy);
-  return y0 >= stop_y || y1 <= start_y;
+  return SnapY(FDot6ToFixed(ScalarToFDot6(y * mul)) >> kAccuracy);
+}
+SKC_HD bool CanBeIgnored(Fixed top, Fixed bottom, Fixed y0, Fixed y1) {
+  return y0 >= bottom || y1 <= top;
+}
+// Whether SetLine makes an edge of a line that is not ignored, from its ends
+// alone.
+SKC_HD bool LineKept(P p0, P p1, Fixed top, Fixed bottom) {
+  const Fixed y0 = ScanFixed(p0.y), y1 = ScanFixed(p1.y);
+  return FixedToFDot6(wsub(y1, y0)) != 0 && !CanBeIgnored(top, bottom, min_(y0, y1), max_(y0, y1));
 }
 SKC_HD int diff_to_shift(FDot6 dx, FDot6 dy, int shiftAA) {  // :97-119
   dx = iabs_(dx);
@@ -174,6 +182,17 @@ SKC_HD bool SetQuad(Edge* e, const P pts[3]) {  // sw_edge.cc:121-231
   return true;
 }
 
+// Whether SetQuad makes an edge of a monotone quad that is not ignored, from
+// its ends alone.
+SKC_HD bool QuadKept(const P pts[3], Fixed top, Fixed bottom) {
+  const float scale = (float)(1 << (kAccuracy + 6));
+  FDot6 y0 = (int)(pts[0].y * scale), y2 = (int)(pts[2].y * scale);
+  if (y0 > y2) swap_(y0, y2);
+  if (FDot6Round(y0) == FDot6Round(y2)) return false;
+  return !CanBeIgnored(top, bottom, SnapY(FDot6ToFixed(y0) >> kAccuracy),
+                       SnapY(FDot6ToFixed(y2) >> kAccuracy));
+}
+
 // ChopQuadAtYExtrema (src/geometry/geometry.cc:311-349)
 SKC_HD int ChopQuadAtYExtrema(const P src[3], P dst[5]) {
   float a = src[0].y, b = src[1].y, c = src[2].y;
@@ -223,27 +242,16 @@ struct Xform {
   }
 };
 
-// The clip bounds (cl, ct, cr, cb) are the canvas's global clip bounds:
+// Scan bounds of a path with bounds (l, t, r, b) (any: it has points).  The
+// clip bounds (cl, ct, cr, cb) are the canvas's global clip bounds:
 // kMaxCullRect (+-1e9, include/skity/render/canvas.hpp:26) unless a
 // ClipRect narrowed them.
-SKC_HD RasterBounds ComputeBounds(const PathView& q, const Xform& xf, float cl = -1e9f,
-                                  float ct = -1e9f, float cr = 1e9f, float cb = 1e9f) {
+SKC_HD RasterBounds ScanBounds(bool any, float l, float t, float r, float b, float cl, float ct,
+                               float cr, float cb) {
   RasterBounds rb;
   rb.empty = true;
   rb.l = rb.t = rb.r = rb.b = rb.sl = rb.st = rb.sr = rb.sb = 0;
-  int n = q.np;
-  if (q.nv > 1 && q.verbs[q.nv - 1] == kMove) n--;
-  if (n <= 0) return rb;
-  const P p0 = xf.map(q.pts[0]);
-  float l = p0.x, t = p0.y, r = l, b = t;
-  for (int i = 1; i < n; ++i) {
-    const P pi = xf.map(q.pts[i]);
-    const float x = pi.x, y = pi.y;
-    l = min_(l, x);
-    r = max_(r, x);
-    t = min_(t, y);
-    b = max_(b, y);
-  }
+  if (!any) return rb;
   rb.l = floor_(l);
   rb.t = floor_(t);
   rb.r = ceil_(r);
@@ -264,91 +272,17 @@ SKC_HD RasterBounds ComputeBounds(const PathView& q, const Xform& xf, float cl =
   return rb;
 }
 
-// SWEdgeBuilder::BuildEdges over PathEdgeIter (sw_edge.cc:299-336,
-// src/graphic/path_priv.hpp:75-170).  Points are mapped by the canvas
-// matrix first (Xform).  Returns the number of edges (may exceed cap: only
-// cap are stored).
-SKC_HDN int BuildEdges(const PathView& q, const Xform& xf, float top, float bottom,
-                       Edge* out, int cap) {
-  int n = 0;
-  int vi = 0, pi = 0, move_to = 0;
-  bool needs_close = false;
-  auto T = [&](int i) { return xf.map(q.pts[i]); };
-  auto add_line = [&](P a, P b) {
-    Edge e;
-    if (SetLine(&e, a, b) && !CanBeIgnored(top, bottom, e.upper_y, e.lower_y)) {
-      if (n < cap) out[n] = e;
-      n++;
-    }
-  };
-  auto add_quad = [&](const P* qq) {
-    Edge e;
-    if (SetQuad(&e, qq) && !CanBeIgnored(top, bottom, e.q_first_y, e.q_last_y)) {
-      if (n < cap) out[n] = e;
-      n++;
-    }
-  };
-  for (;;) {
-    if (vi == q.nv) {
-      if (needs_close) add_line(T(pi - 1), T(move_to));
-      return n;
-    }
-    uint8_t v = q.verbs[vi++];
-    if (v == kMove) {
-      if (needs_close) {
-        add_line(T(pi - 1), T(move_to));
-        needs_close = false;
-      }
-      move_to = pi++;
-    } else if (v == kClose) {
-      if (needs_close) {
-        add_line(T(pi - 1), T(move_to));
-        needs_close = false;
-      }
-    } else {
-      int k = (v + 2) / 2;
-      needs_close = true;
-      pi += k;
-      int s = pi - (k + 1);
-      if (v == kLine) {
-        add_line(T(s), T(s + 1));
-      } else if (v == kQuad) {
-        P seg[3] = {T(s), T(s + 1), T(s + 2)};
-        P mono[5];
-        int c = ChopQuadAtYExtrema(seg, mono);
-        for (int i = 0; i <= c; i++) add_quad(&mono[i * 2]);
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Edge sort: the reference sorts with std::sort (sw_raster.cc:679-704), whose
 // order among fully tied edges is that of introsort as the C++ runtime
 // implements it (Musser's introsort: median-of-three Hoare partitioning down
 // to blocks of 16, heapsort past a depth of 2*floor(log2 n), then insertion
 // sort).  Tied edges must keep that order for pixel parity, so the same
-// published algorithm is restated here over edge indices; tests compare its
-// permutation with std::sort.
+// published algorithm is restated here (and over a warp's lanes in edges.cuh);
+// tests compare its permutation with std::sort.
 // ---------------------------------------------------------------------------
-struct EdgeLess {
-  const Edge* e;
-  SKC_HD bool operator()(int32_t ia, int32_t ib) const {
-    int va = e[ia].upper_y, vb = e[ib].upper_y;
-    if (va == vb) {
-      va = e[ia].x;
-      vb = e[ib].x;
-    }
-    if (va == vb) {
-      va = e[ia].dx;
-      vb = e[ib].dx;
-    }
-    return va < vb;
-  }
-};
-
-template <typename Less>
-SKC_HD void heap_sift(int32_t* a, int hole, int len, int32_t value, Less less) {
+template <typename T, typename Less>
+SKC_HD void heap_sift(T* a, int hole, int len, T value, Less less) {
   // move the hole down to a leaf along larger children, then sift value up
   const int top = hole;
   int child = hole;
@@ -371,15 +305,15 @@ SKC_HD void heap_sift(int32_t* a, int hole, int len, int32_t value, Less less) {
   }
   a[hole] = value;
 }
-template <typename Less>
-SKC_HD void heap_sort_range(int32_t* a, int len, Less less) {
+template <typename T, typename Less>
+SKC_HD void heap_sort_range(T* a, int len, Less less) {
   if (len < 2) return;
   for (int parent = (len - 2) / 2;; --parent) {
     heap_sift(a, parent, len, a[parent], less);
     if (parent == 0) break;
   }
   for (int last = len - 1; last > 0; --last) {
-    int32_t v = a[last];
+    const T v = a[last];
     a[last] = a[0];
     heap_sift(a, 0, last, v, less);
   }

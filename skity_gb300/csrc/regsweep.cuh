@@ -103,15 +103,6 @@ SKC_HD long long LaneMax64(const Lanes& L, long long v) {
 #endif
   return v;
 }
-// v of the lane below (lane 0: `first`).
-SKC_HD int32_t LanePrev(const Lanes& L, int32_t v, int32_t first) {
-#ifdef SKC_WARP_LANES
-  const int32_t t = __shfl_up_sync(0xffffffffu, v, 1);
-  return L.lane == 0 ? first : t;
-#else
-  return first;
-#endif
-}
 SKC_HD uint32_t LaneOr(const Lanes& L, uint32_t v) {
 #ifdef SKC_WARP_LANES
   return __reduce_or_sync(0xffffffffu, v);

@@ -10,7 +10,7 @@
 // rejected with SKITY_CUDA_ERROR_SCRATCH_LIMIT.
 //
 // The work is the batch pipeline's, on the draw's one or two passes:
-// k_geometry (path -> quads -> stroke -> edges -> introsort), the sweep
+// k_stroke and k_edges (path -> quads -> stroke -> edges -> introsort), the sweep
 // kernels, then k_static_composite below, which blends each pass's spans
 // straight into the caller's canvas rows, in paint order.  Layout of the static scratch:
 //
@@ -160,6 +160,7 @@ int32_t StaticDraw(uint8_t* base, uint64_t path_off, uint64_t slice_off0, PassDe
   b.sweep_retry = dev->sweep_retry;
   b.pixels = pixels;
   b.n_list = npass;
+  for (uint32_t i = 0; i < npass; ++i) b.any_stroke |= pd[i].flags & kPassStroke;
   {
     uint64_t o = path_off + Align256(dd.nv);
     b.pts = (const P*)(base + o);

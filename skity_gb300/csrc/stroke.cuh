@@ -12,7 +12,30 @@ constexpr float kRoot2Over2 = 0.707106781f;
 constexpr float kSqrt2 = 1.41421356f;
 SKC_HD bool NearlyZero(float x, float tol = kNearlyZero) { return fabs_(x) <= tol; }
 
-SKC_HD bool PointSetLength(P* pt, float x, float y, float length) {
+// An unevaluated sum of two floats (hi the rounded sum), good for about 2^-46.
+struct Float2 {
+  float hi, lo;
+};
+SKC_HD Float2 TwoSum(float a, float b) {
+  const float s = a + b, bb = s - a;
+  return {s, (a - (s - bb)) + (b - bb)};
+}
+SKC_HD Float2 TwoProd(float a, float b) {
+  const float p = a * b;
+  return {p, fma_(a, b, -p)};
+}
+// The float nearest to a value known to be within 2^-42 of hi + lo, if every
+// value that close rounds to the same float.
+SKC_HD bool RoundSafe(Float2 v, float* out) {
+  const float d = fabs_(v.hi) * (1.0f / (1ull << 42));
+  const float a = v.hi + (v.lo - d), b = v.hi + (v.lo + d);
+  *out = a;
+  return a == b;
+}
+
+// x and y scaled to `length` (point_priv.hpp:81-108), in double as the
+// reference computes it.
+SKC_HDN bool PointSetLengthDouble(P* pt, float x, float y, float length) {
   double xx = x, yy = y;
   double dmag = sqrtd_(xx * xx + yy * yy);
   double dscale = length / dmag;
@@ -26,6 +49,36 @@ SKC_HD bool PointSetLength(P* pt, float x, float y, float length) {
   pt->x = x;
   pt->y = y;
   return true;
+}
+// The same floats without double arithmetic, which runs at 1/64 of the float
+// rate (it was most of the stroker's time): the scaled coordinate in pairs of
+// floats, within 2^-44 (the double result is within 2^-51), rounded where no
+// value that close to it rounds otherwise; else, and outside a range where
+// nothing under- or overflows, in double.
+SKC_HD bool PointSetLength(P* pt, float x, float y, float length) {
+  const float ax = fabs_(x), ay = fabs_(y);
+  const float big = 1.0e9f, small = 1.0e-9f;
+  if ((ax <= big && ay <= big) && (ax >= small || ax == 0) && (ay >= small || ay == 0) &&
+      max_(ax, ay) >= small && length >= small && length <= big) {
+    const Float2 x2 = TwoProd(x, x), y2 = TwoProd(y, y);
+    Float2 s = TwoSum(x2.hi, y2.hi);
+    s.lo += x2.lo + y2.lo;
+    // 1 / sqrt(s) = r + r1, from e = 1 - s r^2
+    const float r = rsqrt_(s.hi);
+    const Float2 rr = TwoProd(r, r), u = TwoProd(s.hi, rr.hi);
+    const float e = (1.0f - u.hi) - (u.lo + (s.hi * rr.lo + s.lo * rr.hi));
+    const float r1 = r * (e * (0.5f + 0.375f * e));
+    auto scaled = [&](float v, float* out) {
+      const Float2 p = TwoProd(v, length), q = TwoProd(p.hi, r);
+      return RoundSafe(TwoSum(q.hi, q.lo + (p.hi * r1 + p.lo * r)), out);
+    };
+    float ox = x, oy = y;  // zeros stay
+    if ((x == 0 || scaled(x, &ox)) && (y == 0 || scaled(y, &oy))) {
+      *pt = mkP(ox, oy);
+      return true;
+    }
+  }
+  return PointSetLengthDouble(pt, x, y, length);
 }
 SKC_HD bool CanNormalize(float dx, float dy) { return isfinite_(dx) && isfinite_(dy) && (dx || dy); }
 SKC_HD bool PointCanNormalize(float dx, float dy) {
@@ -250,14 +303,31 @@ SKC_HD float pt_to_line(P pt, P a, P b) {  // geometry.cc:257-274
   }
   return DistSqd(pt, a);
 }
+// (float)sqrt(B B - 4 A C) as double arithmetic gives it, in pairs of floats;
+// false where that does not settle it (a difference that cancels, is negative
+// or out of range, a root too close to a rounding boundary).
+SKC_HD bool DiscriminantRoot(float A, float B, float C, float* root) {
+  const Float2 b2 = TwoProd(B, B), ac = TwoProd(4.0f * A, C);
+  const float top = max_(b2.hi, fabs_(ac.hi));
+  if (!(top > 1e-20f && top < 1e30f)) return false;
+  Float2 d = TwoSum(b2.hi, -ac.hi);
+  d = TwoSum(d.hi, d.lo + (b2.lo - ac.lo));
+  if (!(d.hi > top * 0.5f)) return false;
+  const float s = sqrt_(d.hi);
+  const float rem = fma_(-s, s, d.hi) + d.lo;
+  return RoundSafe(TwoSum(s, rem / (s + s)), root);
+}
 SKC_HD int FindUnitQuadRoots(float A, float B, float C, float roots[2]) {  // :128-160
   if (A == 0) return valid_unit_divide(-C, B, roots);
   int n = 0;
-  double dr = (double)B * B - 4 * (double)A * C;
-  if (dr < 0) return 0;
-  dr = sqrtd_(dr);
-  float R = (float)dr;
-  if (isinf_(R)) return 0;
+  float R;
+  if (!DiscriminantRoot(A, B, C, &R)) {
+    double dr = (double)B * B - 4 * (double)A * C;
+    if (dr < 0) return 0;
+    dr = sqrtd_(dr);
+    R = (float)dr;
+    if (isinf_(R)) return 0;
+  }
   float Q = (B < 0) ? -(B - R) / 2 : -(B + R) / 2;
   n += valid_unit_divide(Q, A, roots + n);
   n += valid_unit_divide(C, Q, roots + n);
@@ -486,7 +556,7 @@ struct Stroker {
     inner->reset();
     segment_count = -1;
   }
-  SKC_HD bool set_normal_unitnormal(P before, P after, P* normal, P* unit) {  // :100-110
+  SKC_HD bool SetNormals(P before, P after, P* normal, P* unit) const {  // :100-110
     if (!PointSetLength(unit, (after.x - before.x) * scale, (after.y - before.y) * scale, 1.0f))
       return false;
     float tmp = unit->x;
@@ -497,7 +567,7 @@ struct Stroker {
   }
   SKC_HD bool PreJoinTo(P curr, P* normal, P* unit) {  // :795-823
     float prevX = prev_pt.x, prevY = prev_pt.y;
-    if (!set_normal_unitnormal(prev_pt, curr, normal, unit)) {
+    if (!SetNormals(prev_pt, curr, normal, unit)) {
       if (cap == kButtCap) return false;
       *normal = mkP(radius, 0);
       *unit = mkP(1, 0);
@@ -530,6 +600,32 @@ struct Stroker {
     outer->LineTo(mkP(curr.x + normal.x, curr.y + normal.y));
     inner->LineTo(mkP(curr.x - normal.x, curr.y - normal.y));
     PostJoinTo(curr, normal, unit);
+  }
+
+  // What a segment from `from` leaves behind for the next one's join, if that
+  // does not depend on the segments before it: false for segments LineTo or
+  // QuadTo may skip, replace or bend (the state they leave depends on more).
+  SKC_HD bool EndNormals(P from, bool quad, const P* pts, P* normal, P* unit) const {
+    if (quad) {
+      const P q[3] = {from, pts[0], pts[1]};
+      P reduction;
+      const int rt = CheckQuadLinear(q, &reduction);
+      if (rt == 2) {
+        if (!SetNormals(from, pts[0], normal, unit)) return false;
+        P n, u;
+        if (SetNormals(pts[0], pts[1], &n, &u)) {
+          *normal = n;
+          *unit = u;
+        }
+        return true;
+      }
+      if (rt != 1) return false;
+    }
+    const P to = pts[quad ? 1 : 0];
+    if (NearlyZero(from.x - to.x, kNearlyZero * inv_res_scale) &&
+        NearlyZero(from.y - to.y, kNearlyZero * inv_res_scale))
+      return false;
+    return SetNormals(from, to, normal, unit);
   }
 
   // ---- quads
@@ -773,7 +869,7 @@ struct Stroker {
     stroke_type = -1;
     qp.init(0, 1);
     (void)QuadStroke(quad, &qp);
-    if (!set_normal_unitnormal(quad[1], quad[2], &normalBC, &unitBC)) {
+    if (!SetNormals(quad[1], quad[2], &normalBC, &unitBC)) {
       normalBC = normalAB;
       unitBC = unitAB;
     }
@@ -781,7 +877,8 @@ struct Stroker {
   }
 };
 
-// Stroke::StrokePath (stroke.cc:866-901); src has been through QuadPath
+// Stroke::StrokePath (stroke.cc:866-901); src has been through QuadPath.  The
+// form over a warp's lanes is StrokePathLanes (edges.cuh).
 SKC_HDN void StrokePath(const PathView& src, float width, float miter, int cap, int join,
                         DPath* outer, DPath* inner, int inner_max[3]) {
   Stroker s;

@@ -62,6 +62,15 @@ SKC_HD unsigned long long LaneSum64(const Lanes& L, unsigned long long v) {
 #endif
   return v;
 }
+// v of the lane below (lane 0: `first`).
+SKC_HD int32_t LanePrev(const Lanes& L, int32_t v, int32_t first) {
+#ifdef SKC_WARP_LANES
+  const int32_t t = __shfl_up_sync(0xffffffffu, v, 1);
+  return L.lane == 0 ? first : t;
+#else
+  return first;
+#endif
+}
 SKC_HD void FlagError(uint32_t* err, uint32_t code) {
   if (!err) return;
 #ifdef __CUDA_ARCH__
