@@ -117,7 +117,7 @@ __device__ __forceinline__ void FinishOverlapped(unsigned int* done) {
 // and issue 53 %, with fewer instructions a span (105 -> 73).  64 canvases of
 // 50-2,000 paths: 38 -> 15.3 ms; 256 of them: 149 -> 68.  Register caps for
 // more warps (96, 80, 64 registers) are slower: 18.9, 22.7, 27.6 ms.
-template <int M, int kForm>
+template <int M, int kForm, bool kRaw>
 __global__ void __launch_bounds__(32 * kRegWarpsMax) k_sweep_reg(DevBatch b) {
   extern __shared__ __align__(16) uint8_t reg_smem[];
   AllowNextLaunch();
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(32 * kRegWarpsMax) k_sweep_reg(DevBatch b) {
       Lanes L;
       L.lane = threadIdx.x & 31;
       uint8_t* mine = reg_smem + (size_t)w * RegSmemBytes<M>(b.reg_diff_cap);
-      if (!SweepPassReg<M>(b, p, L, (RegSharedT<M>*)mine,
+      if (!SweepPassReg<M, kRaw>(b, p, L, (RegSharedT<M>*)mine,
                            (int32_t*)(mine + sizeof(RegSharedT<M>)), b.reg_diff_cap) &&
           L.leader()) {
         // each pass is taken by one form, so the list holds at most n_passes
@@ -192,31 +192,39 @@ static void LaunchOverlapped(void (*kernel)(Args...), dim3 grid, dim3 block, siz
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <int M, int kForm>
+template <int M, int kForm, bool kRaw>
 static void LaunchRegForm(const DevBatch& b, cudaStream_t stream, bool overlap) {
   const uint32_t nw = b.reg_warps == 1 || b.reg_warps == 4 ? b.reg_warps : 2;
   const size_t smem = nw * RegSmemBytes<M>(b.reg_diff_cap);
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_sweep_reg<M, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_sweep_reg<M, kForm, kRaw>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
-  LaunchOverlapped(k_sweep_reg<M, kForm>, dim3((b.n_passes + nw - 1) / nw), dim3(32 * nw), smem,
-                   stream, overlap, b);
+  LaunchOverlapped(k_sweep_reg<M, kForm, kRaw>, dim3((b.n_passes + nw - 1) / nw), dim3(32 * nw),
+                   smem, stream, overlap, b);
+}
+
+// The sweep forms in launch order: heaviest first, so the longest sweeps
+// start at once and each later (lighter) form fills the SMs the earlier ones'
+// tails leave idle.  kRaw: the batch has path clips, whose passes keep raw
+// spans.
+template <bool kRaw>
+static void LaunchForms(const DevBatch& b, cudaStream_t stream, bool overlap) {
+  LaunchOverlapped(k_sweep<kRaw>, dim3((b.n_passes + kSweepWarps - 1) / kSweepWarps),
+                   dim3(32 * kSweepWarps), 0, stream, false, b);
+  LaunchRegForm<kRegMaxM, kSweepReg128, kRaw>(b, stream, overlap);
+  LaunchRegForm<64, kSweepReg64, kRaw>(b, stream, overlap);
+  LaunchRegForm<32, kSweepReg32, kRaw>(b, stream, overlap);
 }
 
 // With b.sweep_done (four zeroed counters) the later forms overlap the
 // earlier ones' tails; without, they run one after the other.
 int LaunchSweep(const DevBatch& b, cudaStream_t stream) {
   if (b.n_passes == 0) return 0;
-  // heaviest form first: the longest sweeps start at once, and each later
-  // (lighter) form fills the SMs the earlier ones' tails leave idle
   const bool overlap = b.sweep_done != nullptr;
-  // path-clip passes (raw spans) come only with clip states
-  LaunchOverlapped(b.n_clip_states ? k_sweep<true> : k_sweep<false>,
-                   dim3((b.n_passes + kSweepWarps - 1) / kSweepWarps),
-                   dim3(32 * kSweepWarps), 0, stream, false, b);
-  LaunchRegForm<kRegMaxM, kSweepReg128>(b, stream, overlap);
-  LaunchRegForm<64, kSweepReg64>(b, stream, overlap);
-  LaunchRegForm<32, kSweepReg32>(b, stream, overlap);
+  if (b.n_clip_states)
+    LaunchForms<true>(b, stream, overlap);
+  else
+    LaunchForms<false>(b, stream, overlap);
   k_sweep_retry<<<64, 32 * kSweepWarps, 0, stream>>>(b);
   return 5;
 }

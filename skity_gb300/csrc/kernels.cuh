@@ -122,7 +122,7 @@ struct PassGeom {
   int32_t row0, row1;   // canvas rows that can receive spans
   int32_t need[13];     // sizes seen (exact up to the failing stage)
   int32_t max_active;   // bound of the sweep's active-list length
-  int32_t raw_spans;    // the pass keeps raw spans (kPassRawSpans): swept by the generic form
+  int32_t raw_spans;    // the pass keeps raw spans (kPassRawSpans)
 };
 
 // Which sweep form takes pass p: the register form for up to 32, 64 or 128
@@ -140,7 +140,6 @@ constexpr uint8_t kSweepSkip = 4;
 constexpr int kReg32MaxRows = 1100;
 SKC_HD int SweepForm(const PassGeom& g, uint8_t pass_class) {
   if (pass_class != 0) return pass_class;
-  if (g.raw_spans) return kSweepGeneric;  // the path-clip stages' passes (rare)
   const int ma = g.max_active;
   return (ma <= 32 && g.row1 - g.row0 <= kReg32MaxRows) ? kSweepReg32
          : ma <= 64                                     ? kSweepReg64

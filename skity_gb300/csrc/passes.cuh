@@ -38,8 +38,7 @@ SKC_HD bool ClipSpan(int& x, int y, int& len, int W, int H) {
 // alpha & global alpha is 0 under src-over (they blend to nothing).  A raw
 // sink (the passes of the path-clip stages) keeps every span of its rows as
 // the raster made it, in the raw format of pack(); only sinks built with
-// kRawCapable take that form (the generic sweep's), so the register sweeps
-// carry no test for it.
+// kRawCapable take that form (batches without path clips use the others).
 template <bool kRawCapable>
 struct SinkBase {
   int row0, row1, W, H;
@@ -305,9 +304,6 @@ struct PoolSinkT : SinkBase<kRawCapable> {
   }
 };
 
-using PoolSink = PoolSinkT<true>;       // the generic sweep's: every pass form
-using PoolSinkReg = PoolSinkT<false>;   // the register sweeps': never raw
-
 template <typename Sink>
 SKC_HD void InitPoolSink(const DevBatch& b, uint32_t p, const PassGeom& g, Sink* s) {
   const PassDesc pd = b.passes[p];
@@ -435,11 +431,13 @@ SKC_HD int RunRegSweep(const DevBatch& b, uint32_t p, const PassGeom& g, Sink* s
                  g.start_y, g.stop_y, g.left_bound, g.right_bound);
 }
 
-// Sweep of pass p through the register form of size M.  Returns false when
+// Sweep of pass p through the register form of size M (kRaw: the pass may be a
+// path clip's; batches without path clips take the form without that test).
+// Returns false when
 // its active list outgrows M after all: the caller then sweeps the pass with
 // the generic form (SweepPass, which clears the rows the attempt wrote).
 // The generic form is not inlined here, so the register kernels stay small.
-template <int M>
+template <int M, bool kRaw = true>
 SKC_HD bool SweepPassReg(const DevBatch& b, uint32_t p, const Lanes& lanes, RegSharedT<M>* sh,
                          int32_t* sdiff, int32_t sdiff_cap) {
   const PassGeom g = b.geom[p];
@@ -452,7 +450,7 @@ SKC_HD bool SweepPassReg(const DevBatch& b, uint32_t p, const Lanes& lanes, RegS
 #pragma unroll 1
   for (int r = lanes.lane; r < g.row1 - g.row0; r += Lanes::n) rows[r] = make_uint2(0, 0);
   lanes.sync();
-  PoolSinkReg sink;
+  PoolSinkT<kRaw> sink;
   InitPoolSink(b, p, g, &sink);
   if (!RunRegSweep<M>(b, p, g, &sink, lanes, sh, sdiff, sdiff_cap)) {
     lanes.sync();

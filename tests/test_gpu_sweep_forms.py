@@ -45,3 +45,22 @@ def test_forms_match_oracle(gpu_ctx, oracle_lib, teeth, width, height, slant, cu
     scenes = [comb_scene(teeth, width, height, slant, curved, e) for e in (False, True)]
     for sc, got in zip(scenes, gpu_ctx.render_streams(scenes)):
         assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
+
+
+@pytest.mark.parametrize("teeth,slant,curved", [(12, 0.2, True), (17, 1.5, False), (33, 2.0, True),
+                                                (70, 4.0, False)])
+def test_forms_under_path_clips(gpu_ctx, oracle_lib, teeth, slant, curved):
+    """Passes that keep raw spans (clip paths and the draws under them) in each
+    form: a comb drawn under a comb."""
+    width, height = 300, 30
+    comb = comb_scene(teeth, width, height, slant, curved, True)
+    scenes = []
+    for op in (S.CLIP_INTERSECT, S.CLIP_DIFFERENCE):
+        b = S.SceneBuilder(width, height)
+        b.clip_path(comb.verbs, comb.points + np.float32(0.37), op, S.EVEN_ODD)
+        p = S.default_paint()
+        p["fill_color"] = (0.7, 0.2, 0.3, 0.8)
+        b.draw_path(comb.verbs, comb.points, p)
+        scenes.append(b.build())
+    for sc, got in zip(scenes, gpu_ctx.render_streams(scenes)):
+        assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
