@@ -13,6 +13,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <mutex>
+#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -238,7 +241,39 @@ inline void SRGBTables(uint8_t out[512]) {
   }
 }
 
-inline bool ParseStream(const uint8_t* buf, size_t len, StreamView* s) {
+// Runs body(0 .. parts - 1), each once, on up to `threads` host threads (the
+// caller's among them; fewer when the system gives no more).  What a body
+// throws is thrown again here, after all of them ended.
+template <typename F>
+inline void RunParts(unsigned threads, uint32_t parts, F&& body) {
+  std::atomic<uint32_t> next{0};
+  std::exception_ptr thrown;
+  std::mutex mu;
+  auto work = [&]() {
+    try {
+      for (uint32_t r; (r = next.fetch_add(1)) < parts;) body(r);
+    } catch (...) {
+      std::lock_guard<std::mutex> lock(mu);
+      thrown = std::current_exception();
+    }
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (unsigned t = 1; t < threads; ++t) pool.emplace_back(work);
+  } catch (const std::system_error&) {
+  }
+  work();
+  for (auto& t : pool) t.join();
+  if (thrown) std::rethrow_exception(thrown);
+}
+
+// Host threads for a stream of `verbs` verbs: 16384 verbs (0.4 to 0.6 ms of
+// one thread's work) each at least, against some 30 us to start one.
+inline unsigned StreamThreads(uint64_t verbs, unsigned threads) {
+  return (unsigned)std::min<uint64_t>(threads, verbs / 16384);
+}
+
+inline bool ParseStream(const uint8_t* buf, size_t len, StreamView* s, unsigned threads = 1) {
   if (!buf || len < 72 || std::memcmp(buf, "SKSC", 4) != 0) return false;
   uint32_t hdr[7];
   std::memcpy(hdr, buf + 4, sizeof hdr);
@@ -409,27 +444,43 @@ inline bool ParseStream(const uint8_t* buf, size_t len, StreamView* s) {
   }
   if (o > len) return false;
   if (s->width == 0 || s->height == 0 || s->width > 65535 || s->height > 65535) return false;
-  for (uint32_t d = 0; d < s->nd; ++d) {
-    if (s->vo[d] > s->vo[d + 1] || s->vo[d + 1] > s->nv) return false;
-    if (s->po[d] > s->po[d + 1] || s->po[d + 1] > s->np) return false;
-    if (s->wo[d] > s->wo[d + 1] || s->wo[d + 1] > s->nw) return false;
-    if (s->paints[d].gradient >= (int32_t)s->ng) return false;
-    const PaintRec& pr = s->paints[d];
-    if (!ValidPaint(pr.style, pr.cap, pr.join, pr.stroke_width, pr.miter, pr.blur_radius))
-      return false;
-    if (!ValidTranslate(pr.translate, s->pts + 2 * (size_t)s->po[d], s->po[d + 1] - s->po[d]))
-      return false;
-    if (s->matrices) {
-      if (pr.translate[0] != 0.f || pr.translate[1] != 0.f) return false;
-      if (!ValidMatrix(s->matrices + 6 * (size_t)d, s->pts + 2 * (size_t)s->po[d],
-                       s->po[d + 1] - s->po[d]))
+  auto valid_draws = [s](uint32_t d0, uint32_t d1) {
+    for (uint32_t d = d0; d < d1; ++d) {
+      if (s->vo[d] > s->vo[d + 1] || s->vo[d + 1] > s->nv) return false;
+      if (s->po[d] > s->po[d + 1] || s->po[d + 1] > s->np) return false;
+      if (s->wo[d] > s->wo[d + 1] || s->wo[d + 1] > s->nw) return false;
+      if (s->paints[d].gradient >= (int32_t)s->ng) return false;
+      const PaintRec& pr = s->paints[d];
+      if (!ValidPaint(pr.style, pr.cap, pr.join, pr.stroke_width, pr.miter, pr.blur_radius))
+        return false;
+      if (!ValidTranslate(pr.translate, s->pts + 2 * (size_t)s->po[d], s->po[d + 1] - s->po[d]))
+        return false;
+      if (s->matrices) {
+        if (pr.translate[0] != 0.f || pr.translate[1] != 0.f) return false;
+        if (!ValidMatrix(s->matrices + 6 * (size_t)d, s->pts + 2 * (size_t)s->po[d],
+                         s->po[d + 1] - s->po[d]))
+          return false;
+      }
+      if (s->clips && !ValidClip(s->clips + 4 * (size_t)d)) return false;
+      if (s->filters && !ValidColorFilter(s->filters[d])) return false;
+      if (!ValidPath(s->verbs + s->vo[d], s->vo[d + 1] - s->vo[d], s->pts + 2 * (size_t)s->po[d],
+                     s->po[d + 1] - s->po[d], s->wts + s->wo[d], s->wo[d + 1] - s->wo[d]))
         return false;
     }
-    if (s->clips && !ValidClip(s->clips + 4 * (size_t)d)) return false;
-    if (s->filters && !ValidColorFilter(s->filters[d])) return false;
-    if (!ValidPath(s->verbs + s->vo[d], s->vo[d + 1] - s->vo[d], s->pts + 2 * (size_t)s->po[d],
-                   s->po[d + 1] - s->po[d], s->wts + s->wo[d], s->wo[d + 1] - s->wo[d]))
-      return false;
+    return true;
+  };
+  threads = std::min(StreamThreads(s->nv, threads), s->nd);
+  if (threads < 2) {
+    if (!valid_draws(0, s->nd)) return false;
+  } else {
+    const uint32_t runs = std::min(4 * threads, s->nd);
+    std::atomic<bool> ok{true};
+    RunParts(threads, runs, [&](uint32_t r) {
+      if (!valid_draws((uint32_t)((uint64_t)s->nd * r / runs),
+                       (uint32_t)((uint64_t)s->nd * (r + 1) / runs)))
+        ok = false;
+    });
+    if (!ok) return false;
   }
   for (uint32_t g = 0; g < s->ng; ++g) {
     if ((uint64_t)s->grads[g].stop_start + s->grads[g].stop_count > s->ns) return false;
@@ -569,13 +620,21 @@ inline uint32_t SolidPM(const float c[4]) {
   return ColorToPMColor(Color4fToColor(c[0], c[1], c[2], c[3]));
 }
 
+// An element that a vector's resize() leaves unset: the threads that place
+// the parts of a batch write each of them, once.
+template <typename T>
+struct Unset : T {
+  Unset() {}
+  Unset(const T& t) : T(t) {}
+};
+
 struct HostBatch {
   std::vector<uint8_t> verbs;
-  std::vector<P> pts;
+  std::vector<Unset<P>> pts;
   std::vector<float> weights;
-  std::vector<DrawDesc> draws;
-  std::vector<PassDesc> passes;
-  std::vector<Brush> brushes;
+  std::vector<Unset<DrawDesc>> draws;
+  std::vector<Unset<PassDesc>> passes;
+  std::vector<Unset<Brush>> brushes;
   std::vector<ConicalParams> conicals;
   std::vector<int16_t> cf_matrices;  // colour-filter matrices, 20 terms each
   std::vector<ClipStateDesc> clip_states;  // path-clip states of all canvases, in call order
@@ -612,7 +671,9 @@ struct HostBatch {
     d.w0 = (uint32_t)weights.size();
     d.nw = nw;
     verbs.insert(verbs.end(), v, v + nv);
-    for (uint32_t i = 0; i < np; ++i) pts.push_back(mkP(p[2 * i], p[2 * i + 1]));
+    const size_t p0 = pts.size();
+    pts.resize(p0 + np);
+    for (uint32_t i = 0; i < np; ++i) pts[p0 + i] = mkP(p[2 * i], p[2 * i + 1]);
     weights.insert(weights.end(), w, w + nw);
     draws.push_back(d);
     return (uint32_t)draws.size() - 1;
@@ -914,8 +975,23 @@ inline LayerGeom LayerGeometry(const StreamView& s, const LayerRec& L) {
   return g;
 }
 
-// One canvas of a stream into the batch; returns false on invalid input.
-inline int AddStreamCanvas(HostBatch& hb, const StreamView& s) {
+// The passes of one canvas while its draws are added: its own, and those of
+// the temp canvases (blurs and layers) it draws.
+struct CanvasPasses {
+  uint32_t canvas = 0;      // its index in the batch
+  uint32_t state_base = 0;  // path-clip states of the canvases before it
+  std::vector<PassDesc> main;
+  std::vector<std::pair<uint32_t, std::vector<PassDesc>>> temps;
+  uint32_t main_general = 0;  // CanvasDesc::general of the canvas
+};
+inline int AddDraws(HostBatch& hb, const StreamView& s, uint32_t d0, uint32_t d1,
+                    CanvasPasses& cp);
+inline int AddDrawsThreaded(HostBatch& hb, const StreamView& s, unsigned threads,
+                            CanvasPasses& cp);
+
+// One canvas of a stream into the batch, on up to `threads` host threads;
+// the status of its first draw that is not taken, or success.
+inline int AddStreamCanvas(HostBatch& hb, const StreamView& s, unsigned threads = 1) {
   uint32_t cidx = (uint32_t)hb.canvases.size();
   CanvasDesc cd;
   std::memset(&cd, 0, sizeof cd);
@@ -934,13 +1010,14 @@ inline int AddStreamCanvas(HostBatch& hb, const StreamView& s) {
     hb.image_uploads.push_back({hb.image_off[i], std::vector<uint8_t>(s.image_pixels + r.offset,
                                                                      s.image_pixels + r.offset + bytes)});
   }
-  std::vector<PassDesc> main_passes;
-  std::vector<std::pair<uint32_t, std::vector<PassDesc>>> temps;
+  CanvasPasses cp;
+  cp.canvas = cidx;
+  std::vector<PassDesc>& main_passes = cp.main;
   // Path clips: one pass rasterising each ClipPath path (RastePath with the
   // canvas matrix and global clip bounds of the call, sw_canvas.cc:317-324),
   // its spans kept raw for the clip stages; states numbered across the
   // batch.
-  const uint32_t state_base = (uint32_t)hb.clip_states.size();
+  const uint32_t state_base = cp.state_base = (uint32_t)hb.clip_states.size();
   std::vector<uint32_t> clip_pass_pos;
   {
     const uint8_t* v = s.clip_verbs;
@@ -989,6 +1066,33 @@ inline int AddStreamCanvas(HostBatch& hb, const StreamView& s) {
       w += c.nw;
     }
   }
+  threads = s.n_layers ? 1 : StreamThreads(s.vo[s.nd] - s.vo[0], threads);
+  if (threads < 2) {
+    if (int rc = AddDraws(hb, s, 0, s.nd, cp)) return rc;
+    hb.canvases[cidx].pass0 = (uint32_t)hb.passes.size();
+    hb.passes.insert(hb.passes.end(), main_passes.begin(), main_passes.end());
+    hb.canvases[cidx].pass1 = (uint32_t)hb.passes.size();
+    for (auto& tpp : cp.temps) {
+      hb.canvases[tpp.first].pass0 = (uint32_t)hb.passes.size();
+      hb.passes.insert(hb.passes.end(), tpp.second.begin(), tpp.second.end());
+      hb.canvases[tpp.first].pass1 = (uint32_t)hb.passes.size();
+    }
+  } else if (int rc = AddDrawsThreaded(hb, s, threads, cp)) {
+    return rc;
+  }
+  hb.canvases[cidx].general = cp.main_general;
+  for (uint32_t i = 0; i < (uint32_t)clip_pass_pos.size(); ++i)
+    hb.clip_states[state_base + i].pass = hb.canvases[cidx].pass0 + clip_pass_pos[i];
+  return SKITY_CUDA_SUCCESS;
+}
+
+// Draws d0 .. d1 of a stream's canvas: their arrays into the batch, their
+// passes into `cp`.  Part of the draws only in a stream without layers.
+inline int AddDraws(HostBatch& hb, const StreamView& s, uint32_t d0, uint32_t d1,
+                    CanvasPasses& cp) {
+  const uint32_t cidx = cp.canvas, state_base = cp.state_base;
+  std::vector<PassDesc>& main_passes = cp.main;
+  auto& temps = cp.temps;
   // Layers: each saved layer is a temp canvas (a zeroed bitmap over its
   // device bounds) holding the passes of its draws, and at its restore an
   // image pass draws it onto the canvas (SWCanvas::OnLayerRestore,
@@ -1114,7 +1218,7 @@ inline int AddStreamCanvas(HostBatch& hb, const StreamView& s) {
     }
     return SKITY_CUDA_SUCCESS;
   };
-  for (uint32_t d = 0; d < s.nd; ++d) {
+  for (uint32_t d = d0; d < d1; ++d) {
     const PaintRec& pr = s.paints[d];
     const uint32_t path_clip = s.draw_clip_state ? s.draw_clip_state[d] : 0u;
     if (pr.blend > 28) return SKITY_CUDA_ERROR_INVALID_ARGUMENT;  // past kLuminosity
@@ -1275,7 +1379,8 @@ inline int AddStreamCanvas(HostBatch& hb, const StreamView& s) {
     DerivedCaps(pd.cap, false);
     main_passes.push_back(pd);
   }
-  if (int rc = layer_events(s.nd)) return rc;
+  if (d1 == s.nd)
+    if (int rc = layer_events(s.nd)) return rc;
   // canvases with passes the compositor's common form does not take
   auto general = [&](const std::vector<PassDesc>& ps) {
     for (const PassDesc& pd : ps) {
@@ -1285,18 +1390,8 @@ inline int AddStreamCanvas(HostBatch& hb, const StreamView& s) {
     }
     return 0u;
   };
-  hb.canvases[cidx].general = general(main_passes);
+  cp.main_general = general(main_passes);
   for (auto& tpp : temps) hb.canvases[tpp.first].general = general(tpp.second);
-  hb.canvases[cidx].pass0 = (uint32_t)hb.passes.size();
-  for (uint32_t i = 0; i < (uint32_t)clip_pass_pos.size(); ++i)
-    hb.clip_states[state_base + i].pass = hb.canvases[cidx].pass0 + clip_pass_pos[i];
-  hb.passes.insert(hb.passes.end(), main_passes.begin(), main_passes.end());
-  hb.canvases[cidx].pass1 = (uint32_t)hb.passes.size();
-  for (auto& tpp : temps) {
-    hb.canvases[tpp.first].pass0 = (uint32_t)hb.passes.size();
-    hb.passes.insert(hb.passes.end(), tpp.second.begin(), tpp.second.end());
-    hb.canvases[tpp.first].pass1 = (uint32_t)hb.passes.size();
-  }
   return SKITY_CUDA_SUCCESS;
 }
 
@@ -1328,11 +1423,23 @@ struct BatchBase {
   }
 };
 
-// Copies batch `l` into `g` (arrays already sized for it) at base `b`,
-// moving every index and byte offset of `l` by the base: the result is the
-// batch AddStreamCanvas builds by adding l's canvases to g one after the
-// other.  b.px is 256-byte aligned, as AllocPixels places a canvas.
-inline void PlaceBatch(HostBatch& g, const HostBatch& l, const BatchBase& b) {
+// Sizes the arrays of the draws' own data for all parts up to `end`.
+inline void SizeArrays(HostBatch& g, const BatchBase& end) {
+  g.verbs.resize(end.verbs);
+  g.pts.resize(end.pts);
+  g.weights.resize(end.weights);
+  g.draws.resize(end.draws);
+  g.brushes.resize(end.brushes);
+  g.conicals.resize(end.conicals);
+  g.cf_matrices.resize(end.cf);
+  g.stop_colors.resize(end.stops);
+  g.stop_offsets.resize(end.stops);
+}
+
+// Copies the draws' own data of batch `l` into `g` (arrays already sized for
+// it) at base `b`, moving every index and byte offset by the base
+// (own_images: the image brushes' pixels are the part's too, and move).
+inline void PlaceArrays(HostBatch& g, const HostBatch& l, const BatchBase& b, bool own_images) {
   std::copy(l.verbs.begin(), l.verbs.end(), g.verbs.begin() + b.verbs);
   std::copy(l.pts.begin(), l.pts.end(), g.pts.begin() + b.pts);
   std::copy(l.weights.begin(), l.weights.end(), g.weights.begin() + b.weights);
@@ -1347,6 +1454,125 @@ inline void PlaceBatch(HostBatch& g, const HostBatch& l, const BatchBase& b) {
     d.w0 += (uint32_t)b.weights;
     g.draws[b.draws + i] = d;
   }
+  for (size_t i = 0; i < l.brushes.size(); ++i) {
+    Brush r = l.brushes[i];
+    if (r.kind == 1 || r.kind == 2 || r.kind == 4 || r.kind == 5) r.stop0 += (uint32_t)b.stops;
+    if (r.kind == 5) r.conical += (uint32_t)b.conicals;
+    if (r.kind == 3 || (own_images && r.kind == 6)) r.img_off += b.px;
+    if (r.cf_type == 2) r.cf_index += (uint32_t)b.cf;
+    g.brushes[b.brushes + i] = r;
+  }
+}
+
+// The draws of one canvas built in parts: runs of consecutive draws of about
+// equal verbs, each into a batch of its own by one host thread, copied into
+// `hb` at the places AddDraws over all of them would have used, so the batch
+// is the same.  The canvas's passes get their places here (cp.main holds its
+// clip paths' passes; they come first).  100,000 glyph outlines, 3.3 M verbs,
+// parsed and added by one thread: 111 ms; by 16: PARSE_MS.
+inline int AddDrawsThreaded(HostBatch& hb, const StreamView& s, unsigned threads,
+                            CanvasPasses& cp) {
+  // the threads take the runs from a counter, a few runs each: one run of
+  // costly draws does not hold the others up
+  const uint32_t v0 = s.vo[0], target = (s.vo[s.nd] - v0) / (4 * threads) + 1;
+  std::vector<uint32_t> cut{0};
+  for (uint32_t d = 1; d < s.nd; ++d)
+    if (s.vo[d] - s.vo[cut.back()] >= target) cut.push_back(d);
+  cut.push_back(s.nd);
+  const uint32_t runs = (uint32_t)cut.size() - 1;
+  std::vector<HostBatch> part(runs);
+  std::vector<CanvasPasses> passes(runs);
+  std::vector<int> rc(runs, SKITY_CUDA_SUCCESS);
+  RunParts(threads, runs, [&](uint32_t r) {
+    HostBatch& l = part[r];
+    l.canvases.resize(1);  // stands for the canvas itself
+    l.image_off = hb.image_off;
+    passes[r].state_base = cp.state_base;
+    const uint32_t d0 = cut[r], d1 = cut[r + 1];
+    l.verbs.reserve(s.vo[d1] - s.vo[d0]);
+    l.pts.reserve(s.po[d1] - s.po[d0]);
+    l.draws.reserve(d1 - d0);
+    l.brushes.reserve(d1 - d0);
+    passes[r].main.reserve(d1 - d0);
+    rc[r] = AddDraws(l, s, d0, d1, passes[r]);
+  });
+  for (uint32_t r = 0; r < runs; ++r)
+    if (rc[r] != SKITY_CUDA_SUCCESS) return rc[r];
+  // where each part lands
+  BatchBase end;
+  end = end.after(hb);
+  std::vector<BatchBase> base(runs);
+  std::vector<size_t> main_at(runs), temp_at(runs);
+  size_t at = hb.passes.size() + cp.main.size();
+  for (uint32_t r = 0; r < runs; ++r) {
+    if (part[r].pixel_bytes) end.px = (end.px + 255) & ~uint64_t(255);
+    base[r] = end;
+    base[r].canvases -= 1;  // a part's canvas 1 is its first temp canvas
+    end = end.after(part[r]);
+    end.canvases -= 1;
+    main_at[r] = at;
+    at += passes[r].main.size();
+  }
+  const size_t main_end = at;
+  for (uint32_t r = 0; r < runs; ++r) {
+    temp_at[r] = at;
+    for (const auto& t : passes[r].temps) at += t.second.size();
+  }
+  CanvasDesc& cd = hb.canvases[cp.canvas];
+  cd.pass0 = (uint32_t)hb.passes.size();
+  cd.pass1 = (uint32_t)main_end;
+  hb.passes.insert(hb.passes.end(), cp.main.begin(), cp.main.end());
+  hb.passes.resize(at);
+  hb.canvases.resize(end.canvases);
+  hb.temp_canvases.resize(end.temps);
+  SizeArrays(hb, end);
+  RunParts(threads, runs, [&](uint32_t r) {
+    const HostBatch& l = part[r];
+    const BatchBase& b = base[r];
+    PlaceArrays(hb, l, b, false);
+    auto place = [&](const std::vector<PassDesc>& ps, size_t to, uint32_t canvas) {
+      for (size_t i = 0; i < ps.size(); ++i) {
+        PassDesc p = ps[i];
+        p.draw += (uint32_t)b.draws;
+        p.brush += (uint32_t)b.brushes;
+        p.canvas = canvas;
+        hb.passes[to + i] = p;
+      }
+    };
+    place(passes[r].main, main_at[r], cp.canvas);
+    size_t to = temp_at[r];
+    for (size_t i = 0; i < passes[r].temps.size(); ++i) {
+      const auto& t = passes[r].temps[i];
+      const uint32_t canvas = t.first + (uint32_t)b.canvases;
+      CanvasDesc c = l.canvases[t.first];
+      c.px_off += b.px;
+      c.blur_off += b.px;
+      c.out_off += b.px;
+      c.pass0 = (uint32_t)to;
+      place(t.second, to, canvas);
+      to += t.second.size();
+      c.pass1 = (uint32_t)to;
+      hb.canvases[canvas] = c;
+      hb.temp_canvases[b.temps + i] = canvas;
+    }
+  });
+  for (uint32_t r = 0; r < runs; ++r) {
+    cp.main_general |= passes[r].main_general;
+    hb.draw_count += part[r].draw_count;
+    hb.max_temp_w = std::max(hb.max_temp_w, part[r].max_temp_w);
+    hb.max_temp_h = std::max(hb.max_temp_h, part[r].max_temp_h);
+    hb.max_temp_style = std::max(hb.max_temp_style, part[r].max_temp_style);
+  }
+  hb.pixel_bytes = end.px;
+  return SKITY_CUDA_SUCCESS;
+}
+
+// Copies batch `l` into `g` (arrays already sized for it) at base `b`,
+// moving every index and byte offset of `l` by the base: the result is the
+// batch AddStreamCanvas builds by adding l's canvases to g one after the
+// other.  b.px is 256-byte aligned, as AllocPixels places a canvas.
+inline void PlaceBatch(HostBatch& g, const HostBatch& l, const BatchBase& b) {
+  PlaceArrays(g, l, b, true);
   for (size_t i = 0; i < l.passes.size(); ++i) {
     PassDesc p = l.passes[i];
     p.draw += (uint32_t)b.draws;
@@ -1354,14 +1580,6 @@ inline void PlaceBatch(HostBatch& g, const HostBatch& l, const BatchBase& b) {
     if (!(p.flags & kPassClipPath)) p.brush += (uint32_t)b.brushes;  // a clip path's pass has none
     if (p.path_clip) p.path_clip += (uint32_t)b.clip_states;
     g.passes[b.passes + i] = p;
-  }
-  for (size_t i = 0; i < l.brushes.size(); ++i) {
-    Brush r = l.brushes[i];
-    if (r.kind == 1 || r.kind == 2 || r.kind == 4 || r.kind == 5) r.stop0 += (uint32_t)b.stops;
-    if (r.kind == 5) r.conical += (uint32_t)b.conicals;
-    if (r.kind == 3 || r.kind == 6) r.img_off += b.px;
-    if (r.cf_type == 2) r.cf_index += (uint32_t)b.cf;
-    g.brushes[b.brushes + i] = r;
   }
   for (size_t i = 0; i < l.clip_states.size(); ++i) {
     ClipStateDesc c = l.clip_states[i];
@@ -1396,17 +1614,18 @@ inline void PlaceBatch(HostBatch& g, const HostBatch& l, const BatchBase& b) {
 // success.
 inline int32_t BuildStreams(HostBatch& hb, uint32_t count, const uint8_t* const* streams,
                             const size_t* bytes, unsigned threads) {
-  auto add_range = [&](HostBatch& b, uint32_t i0, uint32_t i1) -> int32_t {
+  auto add_range = [&](HostBatch& b, uint32_t i0, uint32_t i1, unsigned t) -> int32_t {
     for (uint32_t i = i0; i < i1; ++i) {
       StreamView sv;
-      if (!ParseStream(streams[i], bytes[i], &sv)) return SKITY_CUDA_ERROR_INVALID_ARGUMENT;
-      const int32_t rc = AddStreamCanvas(b, sv);
+      if (!ParseStream(streams[i], bytes[i], &sv, t)) return SKITY_CUDA_ERROR_INVALID_ARGUMENT;
+      const int32_t rc = AddStreamCanvas(b, sv, t);
       if (rc != SKITY_CUDA_SUCCESS) return rc;
     }
     return SKITY_CUDA_SUCCESS;
   };
+  // few canvases: one after the other, the threads share each one's draws
+  if (count < 8 || threads < 2) return add_range(hb, 0, count, threads);
   if (threads > count / 4) threads = count / 4;
-  if (threads < 2) return add_range(hb, 0, count);
   uint64_t total = 0;
   for (uint32_t i = 0; i < count; ++i) total += bytes[i] + 64;
   // runs of about total / (4 * threads) bytes: the threads take them in
@@ -1426,17 +1645,7 @@ inline int32_t BuildStreams(HostBatch& hb, uint32_t count, const uint8_t* const*
   std::vector<HostBatch> part(runs);
   std::vector<int32_t> rc(runs, SKITY_CUDA_SUCCESS);
   std::vector<BatchBase> base(runs);
-  auto parallel = [&](auto&& body) {
-    std::atomic<uint32_t> next{0};
-    auto work = [&]() {
-      for (uint32_t r; (r = next.fetch_add(1)) < runs;) body(r);
-    };
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < threads; ++t) pool.emplace_back(work);
-    work();
-    for (auto& t : pool) t.join();
-  };
-  parallel([&](uint32_t r) { rc[r] = add_range(part[r], cut[r], cut[r + 1]); });
+  RunParts(threads, runs, [&](uint32_t r) { rc[r] = add_range(part[r], cut[r], cut[r + 1], 1); });
   for (uint32_t r = 0; r < runs; ++r)
     if (rc[r] != SKITY_CUDA_SUCCESS) return rc[r];
   BatchBase end;
@@ -1445,21 +1654,13 @@ inline int32_t BuildStreams(HostBatch& hb, uint32_t count, const uint8_t* const*
     base[r] = end;
     end = end.after(part[r]);
   }
-  hb.verbs.resize(end.verbs);
-  hb.pts.resize(end.pts);
-  hb.weights.resize(end.weights);
-  hb.draws.resize(end.draws);
+  SizeArrays(hb, end);
   hb.passes.resize(end.passes);
-  hb.brushes.resize(end.brushes);
-  hb.conicals.resize(end.conicals);
-  hb.cf_matrices.resize(end.cf);
   hb.clip_states.resize(end.clip_states);
   hb.canvases.resize(end.canvases);
-  hb.stop_colors.resize(end.stops);
-  hb.stop_offsets.resize(end.stops);
   hb.temp_canvases.resize(end.temps);
   hb.main_canvases.resize(end.mains);
-  parallel([&](uint32_t r) { PlaceBatch(hb, part[r], base[r]); });
+  RunParts(threads, runs, [&](uint32_t r) { PlaceBatch(hb, part[r], base[r]); });
   for (uint32_t r = 0; r < runs; ++r) {
     for (auto& u : part[r].image_uploads)
       hb.image_uploads.push_back({u.off + base[r].px, std::move(u.bytes)});

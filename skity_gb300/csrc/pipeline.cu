@@ -905,11 +905,15 @@ static int32_t PlanAndRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool ti
   return SKITY_CUDA_SUCCESS;
 }
 
-// The streams are parsed on the host's threads (BuildStreams), at most 32.
+// Host threads that parse streams and add their draws: the machine's, at most 32.
+static unsigned BuildThreads() {
+  const unsigned hw = std::thread::hardware_concurrency();
+  return std::min(hw ? hw : 1u, 32u);
+}
+
 int32_t BuildFromStreams(DeviceBatch& db, uint32_t count, const uint8_t* const* streams,
                                 const size_t* bytes) {
-  const unsigned hw = std::thread::hardware_concurrency();
-  return BuildStreams(db.hb, count, streams, bytes, std::min(hw ? hw : 1u, 32u));
+  return BuildStreams(db.hb, count, streams, bytes, BuildThreads());
 }
 
 int32_t ReadCanvas(skity_cuda_context_s* ctx, DeviceBatch& db, uint32_t index, uint8_t* out,
@@ -2141,7 +2145,7 @@ SKITY_CUDA_API int32_t skity_cuda_canvas_flush(skity_cuda_canvas canvas) {
   sv.matrices = canvas->any_matrix ? canvas->matrices.data() : nullptr;
   skc::DeviceBatch& db = canvas->db;
   db.Reset();  // other draws than the last flush's: their passes are uploaded again
-  int32_t rc = skc::AddStreamCanvas(db.hb, sv);
+  int32_t rc = skc::AddStreamCanvas(db.hb, sv, skc::BuildThreads());
   if (rc) return rc;
   rc = skc::UploadBatch(ctx, db);
   if (rc) return rc;
