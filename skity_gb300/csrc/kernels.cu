@@ -64,10 +64,10 @@ int LaunchGeometry(const DevBatch& b, cudaStream_t stream) {
 
 // Sweeps: one warp per pass, passes taken in the batch's sweep order
 // (longest expected sweeps first, so the long ones do not form the tail).
-// Four forms, each taking the passes SweepForm gives it: register forms for up to 32, 64 and 128 active edges (2 warps
-// per block, each with its RegSharedT block and accumulator in shared
-// memory), then the generic sweep (4 warps per block, state in global
-// memory) for longer lists.
+// Five forms, each taking the passes SweepLaunch gives it: register forms for
+// up to 32, 64, 128 and 256 active edges (2 warps per block, each with its
+// RegSharedT block and accumulator in shared memory), then the generic sweep
+// (4 warps per block, state in global memory) for longer lists.
 constexpr int kSweepWarps = 4;
 constexpr int kRegWarpsMax = 4;  // warps per CTA of the register sweeps: DevBatch::reg_warps
 
@@ -88,7 +88,7 @@ __device__ __forceinline__ uint32_t SweepPassAt(const DevBatch& b, int form, uin
   }
   if (i >= b.n_passes) return b.n_passes;
   const uint32_t p = b.sweep_order ? b.sweep_order[i] : i;
-  return SweepForm(b.geom[p], b.pass_class[p]) == form ? p : b.n_passes;
+  return SweepLaunch(b.geom[p], b.pass_class[p]) == form ? p : b.n_passes;
 }
 
 // Lets the next overlapped launch start once every CTA of this one runs.
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(32 * kRegWarpsMax) k_sweep_reg(DevBatch b) {
       }
     }
   }
-  FinishOverlapped(b.sweep_done ? b.sweep_done + (kForm & 3) : nullptr);
+  FinishOverlapped(b.sweep_done ? b.sweep_done + kForm : nullptr);
 }
 
 // The passes the register forms gave up on, swept with the generic form after
@@ -211,12 +211,13 @@ template <bool kRaw>
 static void LaunchForms(const DevBatch& b, cudaStream_t stream, bool overlap) {
   LaunchOverlapped(k_sweep<kRaw>, dim3((b.n_passes + kSweepWarps - 1) / kSweepWarps),
                    dim3(32 * kSweepWarps), 0, stream, false, b);
+  LaunchRegForm<256, kSweepReg256, kRaw>(b, stream, overlap);
   LaunchRegForm<kRegMaxM, kSweepReg128, kRaw>(b, stream, overlap);
   LaunchRegForm<64, kSweepReg64, kRaw>(b, stream, overlap);
   LaunchRegForm<32, kSweepReg32, kRaw>(b, stream, overlap);
 }
 
-// With b.sweep_done (four zeroed counters) the later forms overlap the
+// With b.sweep_done (a zeroed counter per form) the later forms overlap the
 // earlier ones' tails; without, they run one after the other.
 int LaunchSweep(const DevBatch& b, cudaStream_t stream) {
   if (b.n_passes == 0) return 0;
@@ -226,7 +227,7 @@ int LaunchSweep(const DevBatch& b, cudaStream_t stream) {
   else
     LaunchForms<false>(b, stream, overlap);
   k_sweep_retry<<<64, 32 * kSweepWarps, 0, stream>>>(b);
-  return 5;
+  return kSweepForms + 1;
 }
 
 // ---------------------------------------------------------------------------

@@ -131,10 +131,12 @@ struct PassGeom {
 // The forms' kernels take disjoint passes and depend on nothing the others
 // write, so their launches may overlap.
 constexpr int kRegMaxM = 128;  // the largest active list held in registers
-enum : int { kSweepReg64 = 0, kSweepReg128 = 2, kSweepGeneric = 1, kSweepReg32 = 3 };
-constexpr int kSweepForms = 4;
+enum : int {
+  kSweepReg64 = 0, kSweepReg128 = 2, kSweepGeneric = 1, kSweepReg32 = 3, kSweepReg256 = 4
+};
+constexpr int kSweepForms = 5;
 // pass_class of a pass no sweep form takes (nothing to sweep, or no room)
-constexpr uint8_t kSweepSkip = 4;
+constexpr uint8_t kSweepSkip = 7;
 // The 32-edge form runs last (lightest form) and takes only short passes,
 // so that no long sweep starts at the end of the sweep launches.
 constexpr int kReg32MaxRows = 1100;
@@ -145,6 +147,15 @@ SKC_HD int SweepForm(const PassGeom& g, uint8_t pass_class) {
          : ma <= 64                                     ? kSweepReg64
          : ma <= kRegMaxM                               ? kSweepReg128
                                                         : kSweepGeneric;
+}
+// The launch that sweeps the pass: lists of 129 to 256 edges have a register
+// form of their own.  They are rare (long strokes that cross themselves), but
+// one such pass held a whole render up: of 20,000 paths of 64 verbs on a
+// 2048 x 2048 canvas, 18,395 passes of at most 128 edges took 153 ms to sweep
+// and one pass of 136, on its own warp, 285 in the generic form.
+SKC_HD int SweepLaunch(const PassGeom& g, uint8_t pass_class) {
+  const int form = SweepForm(g, pass_class);
+  return form == kSweepGeneric && pass_class == 0 && g.max_active <= 256 ? kSweepReg256 : form;
 }
 
 struct PassSweep {      // per-pass sweep buffers, set after geometry

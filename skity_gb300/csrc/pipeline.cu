@@ -165,7 +165,7 @@ static int EnqueuePlanned(skity_cuda_context_s* ctx, DeviceBatch& db, cudaStream
       cudaMemsetAsync(db.err.p, 0, 16, s);
       cudaMemsetAsync(db.pass_class.p, 0, std::max<size_t>(np, 1), s);
       cudaMemsetAsync(ctx->span_next.p, 0, 8, s);
-      cudaMemsetAsync(b.sweep_done, 0, 16, s);
+      cudaMemsetAsync(b.sweep_done, 0, 4 * kSweepForms, s);
       cudaMemsetAsync(b.sweep_retry, 0, 4, s);
       {
         int n = LaunchSweep(b, s);
@@ -431,7 +431,7 @@ static int EnqueueDevice(DeviceBatch& db, const DevBatch& b, const DevPlan& q, u
       return LaunchPlan(b, q, s);
     case 2:
       cudaMemsetAsync(b.span_next, 0, 8, s);
-      cudaMemsetAsync(b.sweep_done, 0, 16, s);
+      cudaMemsetAsync(b.sweep_done, 0, 4 * kSweepForms, s);
       cudaMemsetAsync(b.sweep_retry, 0, 4, s);
       return LaunchSweep(b, s);
     case 3:
@@ -815,7 +815,7 @@ static int32_t PlanAndRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool ti
     SKC_TRY(cudaMemsetAsync(db.err.p, 0, 16, s));
     SKC_TRY(cudaMemsetAsync(db.pass_class.p, 0, std::max<size_t>(np, 1), s));
     SKC_TRY(cudaMemsetAsync(ctx->span_next.p, 0, 8, s));
-    SKC_TRY(cudaMemsetAsync(b.sweep_done, 0, 16, s));
+    SKC_TRY(cudaMemsetAsync(b.sweep_done, 0, 4 * kSweepForms, s));
     SKC_TRY(cudaMemsetAsync(b.sweep_retry, 0, 4, s));
     SKC_TRY(cudaEventRecord(ctx->stage[4], s));
     st.kernel_launches += LaunchSweep(b, s);

@@ -261,7 +261,7 @@ __device__ __forceinline__ uint32_t SortKey(const DevBatch& b, const DevPlan& q,
   if (kind == 0) {
     const PassGeom g = b.geom[i];
     const unsigned long long rows = b.sweep[i].bytes ? (unsigned long long)(g.row1 - g.row0) : 0ull;
-    const int form = SweepForm(g, b.pass_class[i]);
+    const int form = SweepLaunch(g, b.pass_class[i]);
     const uint32_t k = WorkBucket<2>(
         rows * (unsigned long long)(1 + (g.max_active > 0 ? g.max_active : 0)), kSweepBuckets);
     return (form < kSweepForms ? (uint32_t)(1 + form) * kSweepBuckets : 0u) + k;

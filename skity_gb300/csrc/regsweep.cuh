@@ -93,6 +93,7 @@ struct RegSharedT {
 static_assert(sizeof(RegSharedT<32>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<64>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<128>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
+static_assert(sizeof(RegSharedT<256>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 
 SKC_HD long long LaneMax64(const Lanes& L, long long v) {
 #ifdef SKC_WARP_LANES

@@ -65,3 +65,16 @@ def test_forms_under_path_clips(gpu_ctx, oracle_lib, teeth, slant, curved):
         scenes.append(b.build())
     for sc, got in zip(scenes, gpu_ctx.render_streams(scenes)):
         assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
+
+
+# at most 256 active edges: two a tooth, and what a slant adds
+@pytest.mark.parametrize("teeth,width,height,slant,curved",
+                         [(65, 513, 24, 0.0, False), (100, 400, 24, 0.4, True),
+                          (127, 700, 20, 0.1, False), (128, 1024, 17, 0.0, True),
+                          (129, 1024, 17, 0.0, False), (150, 3300, 9, 6.0, True),
+                          (300, 900, 12, 3.0, False)])
+@pytest.mark.parametrize("evenodd", [False, True])
+def test_long_lists_match_oracle(gpu_ctx, oracle_lib, teeth, width, height, slant, curved, evenodd):
+    sc = comb_scene(teeth, width, height, slant, curved, evenodd)
+    got = gpu_ctx.render_streams([sc])[0]
+    assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
