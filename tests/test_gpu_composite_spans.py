@@ -44,3 +44,13 @@ def test_spans_match_oracle(gpu_ctx, oracle_lib, width):
     scenes = [bars_scene(width, k) for k in range(3)]
     for sc, got in zip(scenes, gpu_ctx.render_streams(scenes)):
         assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
+
+
+# 36 rows make 64-pixel tiles above; with filler canvases of 1,200, 1,900 and
+# 4,000 rows beside them the tiles are a quarter, half and all of 1,025 wide
+@pytest.mark.parametrize("rows", [1200, 1900, 4000])
+def test_tile_widths_match_oracle(gpu_ctx, oracle_lib, rows):
+    filler = S.SceneBuilder(8, rows).build()
+    scenes = [bars_scene(1025, k) for k in range(3)]
+    for sc, got in zip(scenes, gpu_ctx.render_streams(scenes + [filler])):
+        assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
