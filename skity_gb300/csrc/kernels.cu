@@ -62,14 +62,13 @@ int LaunchGeometry(const DevBatch& b, cudaStream_t stream) {
   return n;
 }
 
-// Sweeps: one warp per pass, passes taken in the batch's sweep order
+// Sweeps, passes taken in the batch's sweep order
 // (longest expected sweeps first, so the long ones do not form the tail).
 // Five forms, each taking the passes SweepLaunch gives it: register forms for
-// up to 32, 64, 128 and 256 active edges (2 warps per block, each with its
-// RegSharedT block and accumulator in shared memory), then the generic sweep
-// (4 warps per block, state in global memory) for longer lists.
+// up to 32, 64, 128 and 256 active edges (two warps a pass, its RegPairT block
+// and accumulator in shared memory), then the generic sweep (4 warps per
+// block, state in global memory) for longer lists.
 constexpr int kSweepWarps = 4;
-constexpr int kRegWarpsMax = 4;  // warps per CTA of the register sweeps: DevBatch::reg_warps
 
 __device__ __forceinline__ uint32_t DynamicSmemBytes() {
   uint32_t v;
@@ -110,29 +109,55 @@ __device__ __forceinline__ void FinishOverlapped(unsigned int* done) {
   }
 }
 
-// What bounds it: instruction issue.  With a step's coverage made inside the
-// step, the kernel was 140 KB of unrolled code, and instruction fetch held it
-// at 26-34 % of the issue slots; walk and emission as two short loops that
-// take turns (regsweep.cuh), one copy of each part and no unrolling are 54 KB
-// and issue 53 %, with fewer instructions a span (105 -> 73).  64 canvases of
-// 50-2,000 paths: 38 -> 15.3 ms; 256 of them: 149 -> 68.  Register caps for
-// more warps (96, 80, 64 registers) are slower: 18.9, 22.7, 27.6 ms.
+// Waits for the other warp of the pair (at most two pairs per CTA; literal
+// barrier numbers, a CTA holds on to as many as its code may name).
+__device__ __forceinline__ void MeetPair(int pair) {
+  if (pair == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+  else asm volatile("bar.sync 2, 64;" ::: "memory");
+}
+
+// Pairs per SM that the registers leave room for.  More pairs hide
+// more latency until the compiler runs out of registers for the walk: of the
+// 32-edge form 11 fit without a cap; 12 / 13 / 15 pairs sweep 64 canvases of
+// 50-2,000 paths in 14.3 / 14.0 / 14.1 ms (11: 15.6), 1,000 paths on 512 x
+// 512, where latency counts, in 1.99 / 2.08 / 2.18 (11: 1.97).
+template <int M>
+constexpr int kPairsPerSm = M == 32 ? 12 : M == 64 ? 10 : 2;
+
+// A pass is swept by two warps: one walks the active list and logs intervals,
+// the other one makes the spans of the log before (SweepPassPair).
+//
+// What bounds it: a pass is a chain of quarter-pixel steps, one after the
+// other, some 2 us each when one warp both walks and emits; large batches are
+// bound by instruction issue.  With a step's coverage made inside the step,
+// the kernel was 140 KB of unrolled code, and instruction fetch held it at
+// 26-34 % of the issue slots; walk and emission as two short loops
+// (regsweep.cuh), one copy of each part and no unrolling are 54 KB and issue
+// 53 %, with fewer instructions a span (105 -> 73): 64 canvases of 50-2,000
+// paths 38 -> 15.5 ms.  The loops on two warps instead of in turns on one:
+// half the chain, and 80 registers instead of 124, so nearly as many passes
+// are in flight.  1,000 paths on 512 x 512 2.71 -> 1.91 ms, 305 long strokes
+// and fills 12.8 -> 8.2, 400 effects draws 2.70 -> 1.99, the 64 canvases
+// 15.5 -> 13.9, 110,000 glyphs 8.4 -> 7.0; 20,000 paths of 64 verbs, most in
+// the 64-edge form, 154 -> 157.
 template <int M, int kForm, bool kRaw>
-__global__ void __launch_bounds__(32 * kRegWarpsMax) k_sweep_reg(DevBatch b) {
+__global__ void __launch_bounds__(128, kPairsPerSm<M> / 2) k_sweep_pair(DevBatch b) {
   extern __shared__ __align__(16) uint8_t reg_smem[];
   AllowNextLaunch();
-  const int w = threadIdx.x >> 5;
-  const uint32_t nw = blockDim.x >> 5;
-  const uint32_t p = SweepPassAt(b, kForm, blockIdx.x * nw + w);
-  if (p < b.n_passes) {
-    if (DynamicSmemBytes() < nw * RegSmemBytes<M>(b.reg_diff_cap)) {  // self-check
+  const int pair = threadIdx.x >> 6;
+  const uint32_t pairs = blockDim.x >> 6;
+  const uint32_t p = SweepPassAt(b, kForm, blockIdx.x * pairs + pair);
+  if (p < b.n_passes) {  // the same for both warps
+    const int32_t diff_cap = PairDiffCap<M>(b.reg_diff_cap);
+    if (DynamicSmemBytes() < pairs * PairSmemBytes<M>(diff_cap)) {  // self-check
       FlagError(b.err, 16);
     } else {
       Lanes L;
       L.lane = threadIdx.x & 31;
-      uint8_t* mine = reg_smem + (size_t)w * RegSmemBytes<M>(b.reg_diff_cap);
-      if (!SweepPassReg<M, kRaw>(b, p, L, (RegSharedT<M>*)mine,
-                           (int32_t*)(mine + sizeof(RegSharedT<M>)), b.reg_diff_cap) &&
+      uint8_t* mine = reg_smem + (size_t)pair * PairSmemBytes<M>(diff_cap);
+      if (!SweepPassPair<M, kRaw>(b, p, L, (threadIdx.x & 32) == 0, (RegPairT<M>*)mine,
+                                  (int32_t*)(mine + sizeof(RegPairT<M>)), diff_cap,
+                                  [pair] { MeetPair(pair); }) &&
           L.leader()) {
         // each pass is taken by one form, so the list holds at most n_passes
         const uint32_t at = b.sweep_retry ? atomicAdd(b.sweep_retry, 1u) : b.n_passes;
@@ -194,13 +219,13 @@ static void LaunchOverlapped(void (*kernel)(Args...), dim3 grid, dim3 block, siz
 
 template <int M, int kForm, bool kRaw>
 static void LaunchRegForm(const DevBatch& b, cudaStream_t stream, bool overlap) {
-  const uint32_t nw = b.reg_warps == 1 || b.reg_warps == 4 ? b.reg_warps : 2;
-  const size_t smem = nw * RegSmemBytes<M>(b.reg_diff_cap);
+  const uint32_t pairs = b.reg_warps == 4 ? 2 : 1;
+  const size_t smem = pairs * PairSmemBytes<M>(PairDiffCap<M>(b.reg_diff_cap));
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_sweep_reg<M, kForm, kRaw>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_sweep_pair<M, kForm, kRaw>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
-  LaunchOverlapped(k_sweep_reg<M, kForm, kRaw>, dim3((b.n_passes + nw - 1) / nw), dim3(32 * nw),
-                   smem, stream, overlap, b);
+  LaunchOverlapped(k_sweep_pair<M, kForm, kRaw>, dim3((b.n_passes + pairs - 1) / pairs),
+                   dim3(64 * pairs), smem, stream, overlap, b);
 }
 
 // The sweep forms in launch order: heaviest first, so the longest sweeps

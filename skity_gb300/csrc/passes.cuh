@@ -401,42 +401,59 @@ template <int M>
 SKC_HD uint64_t RegSmemBytes(int32_t diff_cap) {
   return sizeof(RegSharedT<M>) + 4ull * (uint64_t)diff_cap;
 }
+// Accumulator entries of a pair in shared memory; wider passes keep theirs in
+// their sweep memory.  The 32-edge form has room for some 1,024-pixel passes:
+// with 3,072 entries the pairs of a 4,096-pixel canvas fill the shared memory
+// before the registers (110,000 glyphs: 6.7 ms instead of 6.2); with 640, 400
+// draws on 1204 pixels take 2.75 ms instead of 2.14.
+template <int M>
+SKC_HD int32_t PairDiffCap(int32_t diff_cap) {
+  return M == 32 ? min_(diff_cap, 1156) : diff_cap;
+}
+template <int M>
+SKC_HD uint64_t PairSmemBytes(int32_t diff_cap) {
+  return sizeof(RegPairT<M>) + 4ull * (uint64_t)diff_cap;
+}
 
-// The register sweep of pass p (RegWalk); returns 0 when its active list
-// outgrows the registers.  The accumulator sits in shared memory when it fits.
-template <int M, typename Sink>
-SKC_HD int RunRegSweep(const DevBatch& b, uint32_t p, const PassGeom& g, Sink* sink,
-                       const Lanes& lanes, RegSharedT<M>* sh, int32_t* sdiff, int32_t sdiff_cap) {
-  const PassDesc pd = b.passes[p];
+// The accumulator of a register sweep, zeroed; it sits in shared memory when
+// it fits.
+SKC_HD void InitAcc(const DevBatch& b, uint32_t p, const PassGeom& g, const Lanes& lanes,
+                    int32_t* sdiff, int32_t sdiff_cap, AccState* as) {
   const PassSweep sw = b.sweep[p];
+  as->diff = g.acc_width + 1 <= sdiff_cap
+                 ? sdiff
+                 : SweepMemAt(b.sweepmem + sw.work_off, g.n_edges, g.acc_width).diff;
+#pragma unroll 1
+  for (int i = lanes.lane; i <= g.acc_width; i += Lanes::n) as->diff[i] = 0;
+  as->left = g.acc_left;
+  as->width = g.acc_width;
+  as->y = kNaN32;
+  as->lo = 0x7fffffff;
+  as->hi = -1;
+  as->flushing = false;
+  lanes.sync();
+}
+
+// The walk of pass p (RegWalk); returns 0 when its active list outgrows the
+// registers.
+template <typename Sh, typename Hand>
+SKC_HD int WalkPass(const DevBatch& b, uint32_t p, const PassGeom& g, const Lanes& lanes, Sh* sh,
+                    Hand&& hand) {
+  const PassDesc pd = b.passes[p];
   SliceLayout L;
   L.compute(pd.cap, sizeof(Edge));
   const Edge* S = (const Edge*)(b.scratch + pd.slice_off + L.off[13]);
-  const int n = g.n_edges;
-  int32_t* diff = g.acc_width + 1 <= sdiff_cap
-                      ? sdiff
-                      : SweepMemAt(b.sweepmem + sw.work_off, n, g.acc_width).diff;
-#pragma unroll 1
-  for (int i = lanes.lane; i <= g.acc_width; i += Lanes::n) diff[i] = 0;
-  lanes.sync();
-  AccState as;
-  as.diff = diff;
-  as.left = g.acc_left;
-  as.width = g.acc_width;
-  as.y = kNaN32;
-  as.lo = 0x7fffffff;
-  as.hi = -1;
-  as.flushing = false;
-  return RegWalk(lanes, *sh, S, n, sink, as, g.scan_top, (pd.flags & kPassEvenOdd) != 0,
-                 g.start_y, g.stop_y, g.left_bound, g.right_bound);
+  // rows whose coverage is kept (scan_top is a whole number)
+  return RegWalk(lanes, *sh, S, g.n_edges, (pd.flags & kPassEvenOdd) != 0,
+                 max_((int)g.scan_top, g.row0), g.row1, g.start_y, g.stop_y, g.left_bound, hand);
 }
 
 // Sweep of pass p through the register form of size M (kRaw: the pass may be a
 // path clip's; batches without path clips take the form without that test).
-// Returns false when
-// its active list outgrows M after all: the caller then sweeps the pass with
-// the generic form (SweepPass, which clears the rows the attempt wrote).
-// The generic form is not inlined here, so the register kernels stay small.
+// Returns false when its active list outgrows M after all: the caller then
+// sweeps the pass with the generic form (SweepPass, which clears the rows the
+// attempt wrote).  Walk and emission take turns here: the form for a caller
+// without a second warp (the CPU build of the tests).
 template <int M, bool kRaw = true>
 SKC_HD bool SweepPassReg(const DevBatch& b, uint32_t p, const Lanes& lanes, RegSharedT<M>* sh,
                          int32_t* sdiff, int32_t sdiff_cap) {
@@ -452,9 +469,62 @@ SKC_HD bool SweepPassReg(const DevBatch& b, uint32_t p, const Lanes& lanes, RegS
   lanes.sync();
   PoolSinkT<kRaw> sink;
   InitPoolSink(b, p, g, &sink);
-  if (!RunRegSweep<M>(b, p, g, &sink, lanes, sh, sdiff, sdiff_cap)) {
+  AccState as;
+  InitAcc(b, p, g, lanes, sdiff, sdiff_cap, &as);
+  if (!WalkPass(b, p, g, lanes, sh, [&](int nrec, bool last) {
+        lanes.sync();
+        RegEmit(lanes, *sh, sh->log[0], &sink, as, nrec, g.left_bound, g.right_bound, last);
+        return &sh->log[0];
+      })) {
     lanes.sync();
     return false;
+  }
+  FinishPass(b, p, &sink, lanes);
+  return true;
+}
+
+// The same by two warps (the device's form): one walks and logs, the other
+// emits the log before.  They meet() once a log, when the walker has filled
+// one and the emitter is done with the other.  The emitter returns the pass's
+// result.
+template <int M, bool kRaw, typename Meet>
+SKC_HD bool SweepPassPair(const DevBatch& b, uint32_t p, const Lanes& lanes, bool walker,
+                          RegPairT<M>* sh, int32_t* sdiff, int32_t sdiff_cap, Meet&& meet) {
+  const PassGeom g = b.geom[p];
+  if (g.n_edges <= 0 || g.row1 <= g.row0) {
+    if (!walker) EmptyPass(b, p, lanes);
+    return true;
+  }
+  int buf = 0;
+  if (walker) {
+    auto hand = [&](int nrec, bool last) {
+      if (lanes.leader()) {
+        sh->filled[buf] = nrec;
+        sh->filled[2 + buf] = last;
+      }
+      meet();
+      buf ^= 1;
+      return &sh->log[buf];
+    };
+    if (!WalkPass(b, p, g, lanes, sh, hand)) hand(-1, true);
+    return true;
+  }
+  uint2* rows = b.rowspan + b.sweep[p].rbase;
+#pragma unroll 1
+  for (int r = lanes.lane; r < g.row1 - g.row0; r += Lanes::n) rows[r] = make_uint2(0, 0);
+  lanes.sync();
+  PoolSinkT<kRaw> sink;
+  InitPoolSink(b, p, g, &sink);
+  AccState as;
+  InitAcc(b, p, g, lanes, sdiff, sdiff_cap, &as);
+#pragma unroll 1
+  for (;; buf ^= 1) {
+    meet();
+    const int nrec = sh->filled[buf];
+    const bool last = sh->filled[2 + buf] != 0;
+    if (nrec < 0) return false;
+    RegEmit(lanes, *sh, sh->log[buf], &sink, as, nrec, g.left_bound, g.right_bound, last);
+    if (last) break;
   }
   FinishPass(b, p, &sink, lanes);
   return true;

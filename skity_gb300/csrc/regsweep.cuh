@@ -1,13 +1,13 @@
 // The sweep of sweep.cuh with the active edges held in registers.
 //
 // Same per-step restatement of WalkEdges (src/render/sw/sw_raster.cc:546-677)
-// as LaneSweep, split into two loops that take turns:
+// as LaneSweep, split into two loops, on a warp each (or in turns on one):
 //
 //   the walk (RegWalk) advances the active list step by step and only logs,
 //   per step, one record per coverage interval -- its two edges' x before
 //   and after the step and their dy -- into a shared-memory buffer;
 //
-//   the emission (RegEmit), run whenever the buffer is full, turns the
+//   the emission (RegEmit), run on each buffer the walk has filled, turns the
 //   logged intervals of several rows into spans: a lane per interval for the
 //   set-up (blit_trapezoid_row), then a lane per span.
 //
@@ -26,8 +26,8 @@
 //     recomputed only when the list or a piece changes;
 //   * windings are +-1, so their prefix sums are population counts of two
 //     ballots.
-// A path whose active list would exceed M edges (the form's size) is not swept here
-// (RegWalk returns 0) and goes to LaneSweep.
+// A path whose active list would exceed M edges (the form's size) is not swept
+// here (RegWalk returns 0) and goes to LaneSweep.
 #pragma once
 #include "kernels.cuh"
 #include "sweep.cuh"
@@ -60,40 +60,70 @@ enum : uint32_t {
   kRecReal = 0x800       // after the set-up: spans are direct, not accumulated
 };
 
-// Per-warp shared block of the register sweep for active lists of up to
-// M edges.
+// The interval records of a form, side 0 the left edge, side 1 the right one:
+// x before the step; x after it (left: after the quad-piece update too); dy.
+// The emission overwrites them by its set-ups (ul/ur, ll/lr, lDY/rDY).
 template <int M>
-struct RegSharedT {
+struct RegLogT {
   static constexpr int kRecords = RegRecords(M);
-  static constexpr int kEvents = 2 * M;  // accumulator entries a flush gathers at a time
-  // Interval records, side 0 the left edge, side 1 the right one: x before
-  // the step; x after it (left: after the quad-piece update too); dy.  The
-  // emission overwrites them by its set-ups (ul/ur, ll/lr, lDY/rDY).
   int32_t xa[2][kRecords], xb[2][kRecords], dy[2][kRecords];
   uint32_t meta[kRecords];
+};
+// Edge state by new list position (reorder and insertion), and the sort's
+// keys: x and list position.
+template <int M>
+struct RegListT {
+  int32_t x[M], dx[M], dy[M], low[M], wc[M];
+  int32_t kx[M], kp[M];
+};
+// Accumulator flush: the nonzero entries of the row's difference array, then
+// the runs they start.
+template <int M>
+struct RegRunsT {
+  static constexpr int kEvents = 2 * M;  // entries a flush gathers at a time
+  int32_t pos[kEvents], val[kEvents];
+  int32_t run[kEvents + 2], sat[kEvents + 2];
+};
+
+// Per-warp shared block of the register sweep for active lists of up to
+// M edges.
+template <int M_>
+struct RegSharedT {
+  static constexpr int M = M_;
+  RegLogT<M> log[1];
   int32_t start[32];   // first span of each set-up of the records being emitted
   int32_t q[8][M];     // quad-piece state by quad slot (RegQuad)
   uint8_t free_slot[M];  // quad slots no edge holds
   union {
-    struct {
-      // edge state by new list position (reorder and insertion)
-      int32_t x[M], dx[M], dy[M], low[M], wc[M];
-      // the sort's keys: x and list position
-      int32_t kx[M], kp[M];
-    } p;
-    // accumulator flush (never during a step): the nonzero entries of the
-    // row's difference array, then the runs they start
-    struct {
-      int32_t pos[kEvents], val[kEvents];
-      int32_t run[kEvents + 2], sat[kEvents + 2];
-    } f;
+    RegListT<M> p;  // during a step
+    RegRunsT<M> f;  // between steps
   } u;
+  SKC_HD RegListT<M>& list() { return u.p; }
+  SKC_HD RegRunsT<M>& runs() { return u.f; }
+};
+// The same for a pass swept by two warps, one walking and one emitting: the
+// walk fills one log while the other one is emitted.
+template <int M_>
+struct RegPairT {
+  static constexpr int M = M_;
+  RegLogT<M> log[2];
+  int32_t start[32];
+  int32_t q[8][M];
+  uint8_t free_slot[M];
+  RegListT<M> p;
+  RegRunsT<M> f;
+  int32_t filled[4];  // records of each log (-1: the walk gave up); whether it is the last
+  SKC_HD RegListT<M>& list() { return p; }
+  SKC_HD RegRunsT<M>& runs() { return f; }
 };
 // Host and device must agree on these sizes (the host sizes the launch).
 static_assert(sizeof(RegSharedT<32>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<64>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<128>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
 static_assert(sizeof(RegSharedT<256>) % 16 == 0, "RegSharedT keeps 16-byte alignment");
+static_assert(sizeof(RegPairT<32>) % 16 == 0 && sizeof(RegPairT<64>) % 16 == 0 &&
+                  sizeof(RegPairT<128>) % 16 == 0 && sizeof(RegPairT<256>) % 16 == 0,
+              "RegPairT keeps 16-byte alignment");
 
 SKC_HD long long LaneMax64(const Lanes& L, long long v) {
 #ifdef SKC_WARP_LANES
@@ -116,8 +146,8 @@ SKC_HD unsigned LeMask(const Lanes& L) { return (2u << L.lane) - 1u; }
 // Quad-piece state of an edge at its quad slot: forward-difference position,
 // steps and second differences, the last point (the shift is in the edge's
 // packed word).
-template <int M>
-SKC_HD void RegQuadPut(RegSharedT<M>& sh, int slot, const Edge& e) {
+template <typename Sh>
+SKC_HD void RegQuadPut(Sh& sh, int slot, const Edge& e) {
   sh.q[0][slot] = e.qx;
   sh.q[1][slot] = e.qy;
   sh.q[2][slot] = e.qdx;
@@ -127,8 +157,8 @@ SKC_HD void RegQuadPut(RegSharedT<M>& sh, int slot, const Edge& e) {
   sh.q[6][slot] = e.q_last_x;
   sh.q[7][slot] = e.q_last_y;
 }
-template <int M>
-SKC_HD void RegQuadGet(const RegSharedT<M>& sh, int slot, Edge* e) {
+template <typename Sh>
+SKC_HD void RegQuadGet(const Sh& sh, int slot, Edge* e) {
   e->qx = sh.q[0][slot];
   e->qy = sh.q[1][slot];
   e->qdx = sh.q[2][slot];
@@ -195,23 +225,23 @@ SKC_HD void AccFlushBegin(const Lanes& L, AccState& a) {
 // 103-136): the row's alphas are the saturated prefix sums of the difference
 // array, and a run starts at every entry whose alpha differs from its left
 // neighbour's.  Gathers the next nonzero entries (each is reset to zero) and
-// leaves the runs they complete in sh.u.f.run / sat, each ending where the
+// leaves the runs they complete in f.run / sat, each ending where the
 // next one starts; returns their number.  A run still open waits in `a` for
 // the next call; the flush ends with the touched range.
 template <int M>
-SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
+SKC_HD int AccRuns(const Lanes& L, AccState& a, RegRunsT<M>& f) {
   constexpr int NL = Lanes::n;
   int ne = 0;
 #pragma unroll 1
-  while (a.at < a.hi && ne + NL <= RegSharedT<M>::kEvents) {
+  while (a.at < a.hi && ne + NL <= RegRunsT<M>::kEvents) {
     const int i = a.at + L.lane;
     const int32_t d = i < a.hi ? a.diff[i] : 0;
     const unsigned mask = L.ballot(d != 0);
     if (mask) {
       if (d != 0) {
         const int e = ne + Lanes::popc(mask & L.lt_mask());
-        sh.u.f.pos[e] = i;
-        sh.u.f.val[e] = d;
+        f.pos[e] = i;
+        f.val[e] = d;
         a.diff[i] = 0;
       }
       ne += Lanes::popc(mask);
@@ -221,8 +251,8 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
   int ns = 0;
   if (a.open >= 0) {
     if (L.leader()) {
-      sh.u.f.run[0] = a.open;
-      sh.u.f.sat[0] = a.sat;
+      f.run[0] = a.open;
+      f.sat[0] = a.sat;
     }
     ns = 1;
   }
@@ -231,15 +261,15 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
   for (int eb = 0; eb < ne; eb += NL) {
     const int e = eb + L.lane;
     const bool valid = e < ne;
-    const int32_t incl = LaneScanIncl(L, valid ? sh.u.f.val[e] : 0) + a.sum;
+    const int32_t incl = LaneScanIncl(L, valid ? f.val[e] : 0) + a.sum;
     const int32_t sat = min_(incl, 255);
     const int32_t before = LanePrev(L, sat, a.sat);
     const bool start = valid && sat != before;
     const unsigned starts = L.ballot(start);
     if (start) {
       const int r = ns + Lanes::popc(starts & L.lt_mask());
-      sh.u.f.run[r] = sh.u.f.pos[e];
-      sh.u.f.sat[r] = sat;
+      f.run[r] = f.pos[e];
+      f.sat[r] = sat;
     }
     ns += Lanes::popc(starts);
     a.sum = LaneBcast(L, incl, NL - 1);
@@ -248,7 +278,7 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
   L.sync();
   if (a.at >= a.hi) {  // the row's end closes the last run
     if (L.leader()) {
-      sh.u.f.run[ns] = a.hi;
+      f.run[ns] = a.hi;
       if (a.lo <= a.hi) a.diff[a.hi] = 0;
     }
     a.flushing = false;
@@ -257,7 +287,7 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
     a.y = kNaN32;
   } else if (ns > 0) {
     --ns;
-    a.open = sh.u.f.run[ns];
+    a.open = f.run[ns];
   }
   L.sync();
   return ns;
@@ -271,10 +301,11 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegSharedT<M>& sh) {
 // loop makes the spans of both kinds, a span per lane, so that the code that
 // stores them is there once (the sweep's instruction fetch is its scarcest
 // resource).
-template <int M, typename Sink>
-SKC_HD void RegEmit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as, int nrec,
+template <typename Sh, typename Sink>
+SKC_HD void RegEmit(const Lanes& L, Sh& sh, RegLogT<Sh::M>& lg, Sink* sink, AccState& as, int nrec,
                     Fixed left_clip, Fixed right_clip, bool last) {
   constexpr int NL = Lanes::n;
+  RegRunsT<Sh::M>& f = sh.runs();
   int32_t last_ur = 0, last_lr = 0;  // the previous chunk's last right edge
   // the chunk [lo, lo + nv): this lane's record's row, spans before it and
   // through it; the chunk's row starts and accumulating records
@@ -294,17 +325,17 @@ SKC_HD void RegEmit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as,
       const int i = fi + L.lane;
       y = fy;
       if (i < fn) {
-        const int x0 = sh.u.f.run[i];
+        const int x0 = f.run[i];
         x = as.left + x0;
-        len = sh.u.f.run[i + 1] - x0;
-        al = (uint8_t)sh.u.f.sat[i];
+        len = f.run[i + 1] - x0;
+        al = (uint8_t)f.sat[i];
         kept = al != 0;
       }
       fi += NL;
     } else if (as.flushing) {
       fy = as.y;
       L.sync();
-      fn = AccRuns(L, as, sh);
+      fn = AccRuns(L, as, f);
       fi = 0;
       continue;
     } else if (w < g1) {
@@ -316,14 +347,14 @@ SKC_HD void RegEmit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as,
       const int g = w + L.lane;
       if (g < g1) {
         const int j = before + Lanes::popc(bits & LeMask(L)) - 1;
-        const uint32_t mt = sh.meta[lo + j];
+        const uint32_t mt = lg.meta[lo + j];
         TrapRow q;
-        q.ul = sh.xa[0][lo + j];
-        q.ur = sh.xa[1][lo + j];
-        q.ll = sh.xb[0][lo + j];
-        q.lr = sh.xb[1][lo + j];
-        q.lDY = sh.dy[0][lo + j];
-        q.rDY = sh.dy[1][lo + j];
+        q.ul = lg.xa[0][lo + j];
+        q.ur = lg.xa[1][lo + j];
+        q.ll = lg.xb[0][lo + j];
+        q.lr = lg.xb[1][lo + j];
+        q.lDY = lg.dy[0][lo + j];
+        q.rDY = lg.dy[1][lo + j];
         q.full = (uint8_t)(mt & 0xFF);
         q.real = (mt & kRecReal) != 0;
         y = (int)mt >> 16;
@@ -380,13 +411,13 @@ SKC_HD void RegEmit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as,
       t.lDY = t.rDY = 0;
       L.sync();
       if (valid) {
-        ul = sh.xa[0][i];
-        ll = sh.xb[0][i];
-        t.lDY = sh.dy[0][i];
-        ur = sh.xa[1][i];
-        lr = sh.xb[1][i];
-        t.rDY = sh.dy[1][i];
-        meta = sh.meta[i];
+        ul = lg.xa[0][i];
+        ll = lg.xb[0][i];
+        t.lDY = lg.dy[0][i];
+        ur = lg.xa[1][i];
+        lr = lg.xb[1][i];
+        t.rDY = lg.dy[1][i];
+        meta = lg.meta[i];
       }
       const int32_t pur = LanePrev(L, ur, last_ur), plr = LanePrev(L, lr, last_lr);
       last_ur = LaneBcast(L, ur, NL - 1);
@@ -414,13 +445,13 @@ SKC_HD void RegEmit(const Lanes& L, RegSharedT<M>& sh, Sink* sink, AccState& as,
       L.sync();
       if (spans) {  // the set-ups that make spans, packed from `lo`
         const int j = Lanes::popc(some & L.lt_mask());
-        sh.xa[0][lo + j] = t.ul;
-        sh.xa[1][lo + j] = t.ur;
-        sh.xb[0][lo + j] = t.ll;
-        sh.xb[1][lo + j] = t.lr;
-        sh.dy[0][lo + j] = t.lDY;
-        sh.dy[1][lo + j] = t.rDY;
-        sh.meta[lo + j] = (meta & 0xFFFF00FFu) | (real ? kRecReal : 0u);
+        lg.xa[0][lo + j] = t.ul;
+        lg.xa[1][lo + j] = t.ur;
+        lg.xb[0][lo + j] = t.ll;
+        lg.xb[1][lo + j] = t.lr;
+        lg.dy[0][lo + j] = t.lDY;
+        lg.dy[1][lo + j] = t.rDY;
+        lg.meta[lo + j] = (meta & 0xFFFF00FFu) | (real ? kRecReal : 0u);
         sh.start[j] = excl;
       }
       L.sync();
@@ -466,27 +497,27 @@ SKC_HD void SlotSet(T (&v)[S], int s, T x) {
 
 // Stores an active list by list position for a reorder, then loads it back.
 template <int M>
-SKC_HD void RegStage(RegSharedT<M>& sh, int r, int32_t x, int32_t dx, int32_t dy, int32_t low,
+SKC_HD void RegStage(RegListT<M>& t, int r, int32_t x, int32_t dx, int32_t dy, int32_t low,
                      int32_t wc) {
-  sh.u.p.x[r] = x;
-  sh.u.p.dx[r] = dx;
-  sh.u.p.dy[r] = dy;
-  sh.u.p.low[r] = low;
-  sh.u.p.wc[r] = wc;
+  t.x[r] = x;
+  t.dx[r] = dx;
+  t.dy[r] = dy;
+  t.low[r] = low;
+  t.wc[r] = wc;
 }
 
 template <int M, int S>
-SKC_HD void RegLoad(const Lanes& L, const RegSharedT<M>& sh, int m, int32_t (&x)[S],
+SKC_HD void RegLoad(const Lanes& L, const RegListT<M>& t, int m, int32_t (&x)[S],
                     int32_t (&dx)[S], int32_t (&dy)[S], int32_t (&low)[S], int32_t (&wc)[S]) {
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     const int p = s * Lanes::n + L.lane;
     if (p < m) {
-      x[s] = sh.u.p.x[p];
-      dx[s] = sh.u.p.dx[p];
-      dy[s] = sh.u.p.dy[p];
-      low[s] = sh.u.p.low[p];
-      wc[s] = sh.u.p.wc[p];
+      x[s] = t.x[p];
+      dx[s] = t.dx[p];
+      dy[s] = t.dy[p];
+      low[s] = t.low[p];
+      wc[s] = t.wc[p];
     }
   }
 }
@@ -496,7 +527,7 @@ SKC_HD void RegLoad(const Lanes& L, const RegSharedT<M>& sh, int m, int32_t (&x)
 // against the left edge's predecessor after the reorder (its new predecessor
 // if it survives, else the last processed survivor before it).
 template <int M, int S>
-SKC_HD void RegTrailing(const Lanes& L, RegSharedT<M>& sh, const int32_t (&x)[S],
+SKC_HD void RegTrailing(const Lanes& L, RegLogT<M>& lg, const int32_t (&x)[S],
                         const int32_t (&dx)[S], const int32_t (&low)[S], const int (&off)[S],
                         Fixed next_y, int m, int nr, int nrec, uint32_t meta, Fixed left_clip) {
   constexpr int NL = Lanes::n;
@@ -537,9 +568,9 @@ SKC_HD void RegTrailing(const Lanes& L, RegSharedT<M>& sh, const int32_t (&x)[S]
   const bool tc = wadd(pred_x, kFixed1) >= wsub(xa, iabs_(dxa));
   if (L.leader()) {
     const int at = nrec + nr;
-    sh.xa[1][at] = sh.xb[1][at] = kMaxS32;  // the right clip
-    sh.dy[1][at] = 0;
-    sh.meta[at] = meta | kRecTrailing | (nr == 0 ? kRecFirst : 0u) |
+    lg.xa[1][at] = lg.xb[1][at] = kMaxS32;  // the right clip
+    lg.dy[1][at] = 0;
+    lg.meta[at] = meta | kRecTrailing | (nr == 0 ? kRecFirst : 0u) |
                   (((meta & 0xFF) == 0xFF && tc) ? kRecClose : 0u);
   }
 }
@@ -553,18 +584,18 @@ SKC_HD void RegTrailing(const Lanes& L, RegSharedT<M>& sh, const int32_t (&x)[S]
 // edge's predecessor by a short backward scan, reorders the list and returns
 // whether this lane saw a crossing.
 template <int M, int S>
-SKC_HD bool RegSort(const Lanes& L, RegSharedT<M>& sh, int m, int32_t (&x)[S], int32_t (&dx)[S],
+SKC_HD bool RegSort(const Lanes& L, RegListT<M>& t, int m, int32_t (&x)[S], int32_t (&dx)[S],
                     int32_t (&dy)[S], int32_t (&low)[S], int32_t (&wc)[S]) {
   constexpr int NL = Lanes::n;
-  int32_t* kx = sh.u.p.kx;
-  int32_t* kp = sh.u.p.kp;
+  int32_t* kx = t.kx;
+  int32_t* kp = t.kp;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     const int p = s * NL + L.lane;
     if (p < m) {
       kx[p] = x[s];
       kp[p] = p;
-      sh.u.p.dx[p] = dx[s];
+      t.dx[p] = dx[s];
     }
   }
   L.sync();
@@ -596,42 +627,44 @@ SKC_HD bool RegSort(const Lanes& L, RegSharedT<M>& sh, int m, int32_t (&x)[S], i
     int q = r - 1;
 #pragma unroll 1
     while (q >= 0 && kp[q] > pr) --q;
-    if (q >= 0 && wadd(kx[q], sh.u.p.dx[kp[q]]) > wadd(kx[r], sh.u.p.dx[pr])) cross = true;
+    if (q >= 0 && wadd(kx[q], t.dx[kp[q]]) > wadd(kx[r], t.dx[pr])) cross = true;
   }
   L.sync();
   // rank of each list position, by way of the wc row
 #pragma unroll 1
-  for (int r = L.lane; r < m; r += NL) sh.u.p.wc[kp[r]] = r;
+  for (int r = L.lane; r < m; r += NL) t.wc[kp[r]] = r;
   L.sync();
   int rank[S];
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     const int p = s * NL + L.lane;
-    rank[s] = p < m ? sh.u.p.wc[p] : 0;
+    rank[s] = p < m ? t.wc[p] : 0;
   }
   L.sync();
 #pragma unroll
   for (int s = 0; s < S; ++s)
-    if (s * NL + L.lane < m) RegStage<M>(sh, rank[s], x[s], dx[s], dy[s], low[s], wc[s]);
+    if (s * NL + L.lane < m) RegStage<M>(t, rank[s], x[s], dx[s], dy[s], low[s], wc[s]);
   L.sync();
-  RegLoad<M, S>(L, sh, m, x, dx, dy, low, wc);
+  RegLoad<M, S>(L, t, m, x, dx, dy, low, wc);
   L.sync();
   return cross;
 }
 
-// WalkEdges over the pass's sorted edges W[0, n).  Returns 0 if the active
-// list would exceed M edges.
-template <int M, typename Sink>
-SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink* sink,
-                   AccState& as, float scan_top, bool even_odd, int start_y, int stop_y,
-                   Fixed left_clip, Fixed right_clip) {
+// WalkEdges over the pass's sorted edges W[0, n), logging the intervals of
+// rows [row_lo, row_hi).  hand(records, last) takes a log that is full (or the
+// last one) and returns the log to fill next.  Returns 0 if the active list
+// would exceed M edges.
+template <typename Sh, typename Hand>
+SKC_HD int RegWalk(const Lanes& L, Sh& sh, const Edge* W, int n, bool even_odd, int row_lo,
+                   int row_hi, int start_y, int stop_y, Fixed left_clip, Hand&& hand) {
   constexpr int NL = Lanes::n;
+  constexpr int M = Sh::M;
   constexpr int S = M / NL;
-  constexpr int R = RegSharedT<M>::kRecords;
+  constexpr int R = RegLogT<M>::kRecords;
   constexpr unsigned kFull = NL == 32 ? 0xffffffffu : 1u;
+  RegListT<M>& t = sh.list();
+  RegLogT<M>* lg = &sh.log[0];
   const int winding_mask = even_odd ? 1 : -1;
-  // rows whose coverage is kept (scan_top is a whole number)
-  const int row_lo = max_((int)scan_top, sink->row0), row_hi = sink->row1;
   const Fixed y_stop = IntToFixed(stop_y);
   int32_t x[S], dx[S], dy[S], low[S], wc[S];
   int off[S];  // where the edge logs: side * R + its interval of the step; < 0: it does not
@@ -766,10 +799,10 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
               }
               if (off[s] >= 0) {
                 const int at = off[s] + nrec;
-                (&sh.xa[0][0])[at] = xo[s];
-                (&sh.xb[0][0])[at] = x[s];
-                (&sh.dy[0][0])[at] = dy[s];
-                if (off[s] >= R) sh.meta[at - R] = meta | close | (off[s] == R ? kRecFirst : 0u);
+                (&lg->xa[0][0])[at] = xo[s];
+                (&lg->xb[0][0])[at] = x[s];
+                (&lg->dy[0][0])[at] = dy[s];
+                if (off[s] >= R) lg->meta[at - R] = meta | close | (off[s] == R ? kRecFirst : 0u);
               }
             }
           }
@@ -806,12 +839,12 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
               SlotSet<S>(low, s, e.lower_y);
               SlotSet<S>(wc, s, MakeWc(e.winding, e.curve_count, e.curve_shift, slot));
               const int o = SlotGet<S>(off, s);
-              if (log && o >= 0 && o < R) (&sh.xb[0][0])[o + nrec] = e.x;
+              if (log && o >= 0 && o < R) (&lg->xb[0][0])[o + nrec] = e.x;
             }
           }
         }
         if (SKC_COLD(final_in && log))
-          RegTrailing<M, S>(L, sh, x, dx, low, off, next_y, m, nr, nrec, meta, left_clip);
+          RegTrailing<M, S>(L, *lg, x, dx, low, off, next_y, m, nr, nrec, meta, left_clip);
         if (next_y >= lmin) {
           // ---- the edges that go on, in list order
           unsigned smask[S];
@@ -829,7 +862,7 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
                 const int p = s * NL + L.lane;
                 const unsigned gone = L.ballot(p < m) & ~smask[s];
                 if ((smask[s] >> (NL == 32 ? L.lane : 0)) & 1u)
-                  RegStage<M>(sh, r0 + Lanes::popc(smask[s] & L.lt_mask()), x[s], dx[s], dy[s],
+                  RegStage<M>(t, r0 + Lanes::popc(smask[s] & L.lt_mask()), x[s], dx[s], dy[s],
                               low[s], wc[s]);
                 else if (p < m)
                   sh.free_slot[d0 + Lanes::popc(gone & L.lt_mask())] = (uint8_t)WcSlot(wc[s]);
@@ -840,7 +873,7 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
             n_free = d0;
             m = m2;
             L.sync();
-            RegLoad<M, S>(L, sh, m, x, dx, dy, low, wc);
+            RegLoad<M, S>(L, t, m, x, dx, dy, low, wc);
             L.sync();
           }
         }
@@ -868,7 +901,7 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
         }
         if (L.ballot(inv || crs)) {
           if (L.ballot(inv)) {
-            crs = RegSort<M, S>(L, sh, m, x, dx, dy, low, wc);
+            crs = RegSort<M, S>(L, t, m, x, dx, dy, low, wc);
             changed = true;
           }
           cross = L.ballot(crs) != 0;
@@ -900,11 +933,11 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
         for (int s = 0; s < S; ++s) before[s] = x[s] > x0 ? 1 : 0;
 #pragma unroll 1
         for (int tb = 0; tb < c; tb += NL) {
-          const int t = tb + L.lane;
+          const int te = tb + L.lane;
           Edge e;
           int np = 0;
-          if (t < c) e = W[k + t];
-          const int32_t xt_mine = t < c ? e.x : 0;
+          if (te < c) e = W[k + te];
+          const int32_t xt_mine = te < c ? e.x : 0;
           const int tn = min_(NL, c - tb);
 #pragma unroll 1
           for (int j = 0; j < tn; ++j) {
@@ -921,9 +954,9 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
             }
             if (j == L.lane || NL == 1) np = tb + j + cnt;
           }
-          if (t < c) {
-            const int slot = sh.free_slot[n_free - 1 - t];
-            RegStage<M>(sh, np, e.x, e.dx, e.dy, e.lower_y,
+          if (te < c) {
+            const int slot = sh.free_slot[n_free - 1 - te];
+            RegStage<M>(t, np, e.x, e.dx, e.dy, e.lower_y,
                            MakeWc(e.winding, e.curve_count, e.curve_shift, slot) | kWcNew);
             if (e.curve_count > 0) RegQuadPut(sh, slot, e);
           }
@@ -931,21 +964,21 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
 #pragma unroll
         for (int s = 0; s < S; ++s) {
           const int p = s * NL + L.lane;
-          if (p < m) RegStage<M>(sh, p + before[s], x[s], dx[s], dy[s], low[s], wc[s]);
+          if (p < m) RegStage<M>(t, p + before[s], x[s], dx[s], dy[s], low[s], wc[s]);
         }
         n_free -= c;
         m += c;
         k += c;
         pend_y = k < n ? W[k].upper_y : kMaxS32;
         L.sync();
-        RegLoad<M, S>(L, sh, m, x, dx, dy, low, wc);
+        RegLoad<M, S>(L, t, m, x, dx, dy, low, wc);
         bool cross2 = false;
 #pragma unroll
         for (int s = 0; s < S; ++s) {
           const int p = s * NL + L.lane;
           if (p < m && (wc[s] & kWcNew)) {
             wc[s] &= ~kWcNew;
-            if (p > 0 && wadd(sh.u.p.x[p - 1], sh.u.p.dx[p - 1]) > wadd(x[s], dx[s])) cross2 = true;
+            if (p > 0 && wadd(t.x[p - 1], t.dx[p - 1]) > wadd(x[s], dx[s])) cross2 = true;
           }
         }
         L.sync();
@@ -953,8 +986,7 @@ SKC_HD int RegWalk(const Lanes& L, RegSharedT<M>& sh, const Edge* W, int n, Sink
         changed = true;
       }
     }
-    L.sync();
-    RegEmit(L, sh, sink, as, nrec, left_clip, right_clip, done);
+    lg = hand(nrec, done);
     nrec = 0;
     if (done) break;
   }
