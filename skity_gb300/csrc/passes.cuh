@@ -427,9 +427,10 @@ SKC_HD void InitAcc(const DevBatch& b, uint32_t p, const PassGeom& g, const Lane
   for (int i = lanes.lane; i <= g.acc_width; i += Lanes::n) as->diff[i] = 0;
   as->left = g.acc_left;
   as->width = g.acc_width;
+  as->shift = Lanes::n == 1 ? 0 : 5;
+  while ((g.acc_width >> as->shift) >= 32) ++as->shift;
   as->y = kNaN32;
-  as->lo = 0x7fffffff;
-  as->hi = -1;
+  as->touched = 0;
   as->flushing = false;
   lanes.sync();
 }

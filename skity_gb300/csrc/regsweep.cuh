@@ -198,14 +198,20 @@ SKC_HD void LanePrevOf(const Lanes& L, const int32_t (&v)[S], int s, int32_t* ou
 #endif
 }
 
-// Row accumulator of the sweep (the difference array and its touched range).
+// Row accumulator of the sweep: the difference array, entries 0 .. width, and
+// which of its up to 32 blocks of 1 << shift entries have been added to.  Few
+// entries of a wide row are (two a span): with the range of the touched ones
+// read from end to end, half the reads of 1,000-pixel paths of 64 verbs found
+// nothing, three of four of 2,000-pixel ones (20,000 paths on 2048 x 2048
+// 157 -> 152 ms, long strokes 8.2 -> 7.8, narrow paths as before).
 struct AccState {
   int32_t* diff;
   int left, width;
-  int y;       // row being accumulated (kNaN32: none)
-  int lo, hi;  // touched entries [lo, hi] (this lane's adds; reduced at the flush)
-  // a flush under way: next entry to read, the sum and its saturated value
-  // before it, the run open there
+  int shift;
+  int y;             // row being accumulated (kNaN32: none)
+  uint32_t touched;  // a bit per block (this lane's adds)
+  // a flush under way: blocks to read, entries read of the first of them, the
+  // sum and its saturated value before it, the run open there
   bool flushing;
   int at;
   int32_t sum, sat;
@@ -213,9 +219,8 @@ struct AccState {
 };
 
 SKC_HD void AccFlushBegin(const Lanes& L, AccState& a) {
-  a.lo = LaneMin(L, a.lo);
-  a.hi = LaneMax(L, a.hi);
-  a.at = a.lo;
+  a.touched = LaneOr(L, a.touched);
+  a.at = 0;
   a.sum = a.sat = 0;
   a.open = -1;
   a.flushing = true;
@@ -227,15 +232,15 @@ SKC_HD void AccFlushBegin(const Lanes& L, AccState& a) {
 // neighbour's.  Gathers the next nonzero entries (each is reset to zero) and
 // leaves the runs they complete in f.run / sat, each ending where the
 // next one starts; returns their number.  A run still open waits in `a` for
-// the next call; the flush ends with the touched range.
+// the next call; the last one has alpha 0 (a span's two entries cancel).
 template <int M>
 SKC_HD int AccRuns(const Lanes& L, AccState& a, RegRunsT<M>& f) {
   constexpr int NL = Lanes::n;
   int ne = 0;
 #pragma unroll 1
-  while (a.at < a.hi && ne + NL <= RegRunsT<M>::kEvents) {
-    const int i = a.at + L.lane;
-    const int32_t d = i < a.hi ? a.diff[i] : 0;
+  while (a.touched && ne + NL <= RegRunsT<M>::kEvents) {
+    const int i = ((Lanes::ffs(a.touched) - 1) << a.shift) + a.at + L.lane;
+    const int32_t d = i <= a.width ? a.diff[i] : 0;
     const unsigned mask = L.ballot(d != 0);
     if (mask) {
       if (d != 0) {
@@ -247,6 +252,10 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegRunsT<M>& f) {
       ne += Lanes::popc(mask);
     }
     a.at += NL;
+    if (a.at >> a.shift) {  // the block's end
+      a.at = 0;
+      a.touched &= a.touched - 1;
+    }
   }
   int ns = 0;
   if (a.open >= 0) {
@@ -276,16 +285,11 @@ SKC_HD int AccRuns(const Lanes& L, AccState& a, RegRunsT<M>& f) {
     a.sat = LaneBcast(L, sat, NL - 1);
   }
   L.sync();
-  if (a.at >= a.hi) {  // the row's end closes the last run
-    if (L.leader()) {
-      f.run[ns] = a.hi;
-      if (a.lo <= a.hi) a.diff[a.hi] = 0;
-    }
+  if (!a.touched) {
     a.flushing = false;
-    a.lo = 0x7fffffff;
-    a.hi = -1;
     a.y = kNaN32;
-  } else if (ns > 0) {
+  }
+  if (ns > 0) {
     --ns;
     a.open = f.run[ns];
   }
@@ -365,9 +369,8 @@ SKC_HD void RegEmit(const Lanes& L, Sh& sh, RegLogT<Sh::M>& lg, Sink* sink, AccS
           o0 = max_(o0, 0);
           o1 = min_(o1, as.width);
           if (o0 < o1) {
-            as.lo = min_(as.lo, o0);
-            as.hi = max_(as.hi, o1);
             if (al != 0) {
+              as.touched |= (1u << (o0 >> as.shift)) | (1u << (o1 >> as.shift));
               AtomicAddI32(&as.diff[o0], (int32_t)al);
               AtomicAddI32(&as.diff[o1], -(int32_t)al);
             }
