@@ -88,14 +88,15 @@ struct PoolSinkT : SinkBase<kRawCapable> {
   uint2* rows;                 // (first span, count) per row of [row0, row1)
   uint32_t* err;
   int cur_row;
-  uint64_t row_start, cur, chunk_end;
+  // positions in the pool (it has less than 2^32 spans; meaningless once dead)
+  uint32_t row_start, cur, chunk_end;
   bool dead;
-  uint64_t kept;
+  uint32_t kept;
   unsigned long long frags;
 
   SKC_HD void finish_row(const Lanes& L) {
     if (!dead && cur > row_start && cur_row >= row0 && cur_row < row1 && L.leader())
-      rows[cur_row - row0] = make_uint2((uint32_t)row_start, (uint32_t)(cur - row_start));
+      rows[cur_row - row0] = make_uint2(row_start, cur - row_start);
   }
   SKC_HD void row_begin(const Lanes& L, int y) {
     if (y == cur_row) return;
@@ -105,9 +106,9 @@ struct PoolSinkT : SinkBase<kRawCapable> {
   }
   // Room for `add` more spans after the `written` spans this step already
   // put at cur; returns cur (the row may have moved to a new chunk).
-  SKC_HD uint64_t reserve(const Lanes& L, uint32_t written, uint32_t add) {
-    if (SKC_LIKELY(cur + written + add <= chunk_end)) return cur;
-    const uint64_t have = cur + written - row_start;
+  SKC_HD uint32_t reserve(const Lanes& L, uint32_t written, uint32_t add) {
+    if (SKC_LIKELY(written + add <= chunk_end - cur)) return cur;
+    const uint32_t have = cur + written - row_start;
     if (have + add > chunk) {  // a row larger than a chunk (not expected)
       FlagError(err, 8);
       dead = true;
@@ -126,15 +127,15 @@ struct PoolSinkT : SinkBase<kRawCapable> {
     if (!dead) {
       L.sync();
 #pragma unroll 1
-      for (uint64_t i = L.lane; i < have; i += Lanes::n) pool[c + i] = pool[row_start + i];
+      for (uint32_t i = L.lane; i < have; i += Lanes::n) pool[c + i] = pool[row_start + i];
       L.sync();
     }
-    cur = c + (cur - row_start);
-    row_start = c;
-    chunk_end = c + chunk;
+    cur = (uint32_t)c + (cur - row_start);
+    row_start = (uint32_t)c;
+    chunk_end = row_start + chunk;
     return cur;
   }
-  SKC_HD uint2* span_ptr(uint64_t i) { return dead ? nullptr : pool + i; }
+  SKC_HD uint2* span_ptr(uint32_t i) { return dead ? nullptr : pool + i; }
   // One span per lane (`kept`), rows in increasing order over the lanes, of
   // `len` pixels each: appended in lane order, every row that ends among them
   // entered in the row table, the last one left open.
@@ -142,26 +143,26 @@ struct PoolSinkT : SinkBase<kRawCapable> {
     const unsigned km = L.ballot(kept_);
     if (!km) return;
     const uint32_t cnt = (uint32_t)Lanes::popc(km);
-    const uint64_t at = reserve(L, 0, cnt);
+    const uint32_t at = reserve(L, 0, cnt);
     const unsigned below = km & L.lt_mask();
-    const uint32_t rank = (uint32_t)Lanes::popc(below);
-    uint2* dst = span_ptr(at + rank);
-    if (kept_ && dst) *dst = v;
+    const uint32_t mine = at + (uint32_t)Lanes::popc(below);
+    if (kept_ && !dead) pool[mine] = v;
     const int py = LaneBcast(L, y, below ? 31 - clz_(below) : L.lane);
-    const unsigned heads = L.ballot(kept_ && (below ? py : cur_row) != y);
+    const bool head = kept_ && (below ? py : cur_row) != y;
+    const unsigned heads = L.ballot(head);
     if (heads) {
-      const int first = Lanes::ffs(heads) - 1;
-      const uint64_t end = at + (uint32_t)Lanes::popc(km & ((1u << first) - 1u));
-      if (!dead) {
-        if (L.lane == first && end > row_start && cur_row >= row0 && cur_row < row1)
-          rows[cur_row - row0] = make_uint2((uint32_t)row_start, (uint32_t)(end - row_start));
-        const unsigned later = heads & ~((2u << L.lane) - 1u);
-        if (((heads >> L.lane) & 1u) && later) {
-          const uint32_t next = (uint32_t)Lanes::popc(km & ((1u << (Lanes::ffs(later) - 1)) - 1u));
-          rows[y - row0] = make_uint2((uint32_t)(at + rank), next - rank);
+      const int last = 31 - clz_(heads);
+      if (head && !dead) {
+        // the first one ends the row left open, each but the last is a row
+        if (L.lane == Lanes::ffs(heads) - 1 && mine > row_start && cur_row >= row0 &&
+            cur_row < row1)
+          rows[cur_row - row0] = make_uint2(row_start, mine - row_start);
+        if (L.lane != last) {
+          const unsigned next = heads & ~((2u << L.lane) - 1u);
+          rows[y - row0] = make_uint2(
+              mine, (uint32_t)Lanes::popc(km & ~L.lt_mask() & ((next & (0u - next)) - 1u)));
         }
       }
-      const int last = 31 - clz_(heads);
       cur_row = LaneBcast(L, y, last);
       row_start = at + (uint32_t)Lanes::popc(km & ((1u << last) - 1u));
     }
@@ -282,7 +283,7 @@ struct PoolSinkT : SinkBase<kRawCapable> {
       const int32_t ci = LaneScanIncl(L, cnt);
       const uint32_t total = (uint32_t)LaneBcast(L, ci, Lanes::n - 1);
       if (total) {
-        const uint64_t at = reserve(L, 0, total);
+        const uint32_t at = reserve(L, 0, total);
         uint2* dst = span_ptr(at + (uint32_t)(ci - cnt));
         if (dst) {
           for (int i = 0; i < cnt; ++i) dst[i] = out[i];
@@ -295,7 +296,7 @@ struct PoolSinkT : SinkBase<kRawCapable> {
     if (open_start >= 0) {
       int x = left + open_start, len = hi - open_start;
       if (keep(x, y, len, (uint8_t)open_v)) {
-        const uint64_t at = reserve(L, 0, 1);
+        const uint32_t at = reserve(L, 0, 1);
         if (!dead && L.leader()) pool[at] = pack(x, len, (uint32_t)open_v);
         commit(L, 1, L.leader() ? (unsigned)len : 0u);
       }
@@ -317,7 +318,7 @@ SKC_HD void InitPoolSink(const DevBatch& b, uint32_t p, const PassGeom& g, Sink*
   s->srcover = (pd.flags & kPassSrcOver) != 0;
   s->raw = (pd.flags & kPassRawSpans) != 0;
   s->pool = b.spans;
-  s->cap = b.span_cap;
+  s->cap = b.span_cap < 0xFFFFFFFFull ? b.span_cap : 0xFFFFFFFFull;
   s->next = b.span_next;
   s->chunk = sw.chunk;
   s->rows = b.rowspan + sw.rbase;
@@ -335,7 +336,7 @@ SKC_HD void FinishPass(const DevBatch& b, uint32_t p, Sink* s, const Lanes& L) {
   const unsigned long long frags = LaneSum64(L, s->frags);
   L.sync();
   if (L.leader()) {
-    b.pass_spans[p] = (uint32_t)s->kept;
+    b.pass_spans[p] = s->kept;
     if (b.pass_frags) b.pass_frags[p] = frags;
   }
 }
