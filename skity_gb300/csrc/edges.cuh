@@ -379,17 +379,32 @@ SKC_HD DPath PathTail(const DPath& base, int v, int p, int w) {
 // QuadPathLanes calls regular.  Each contour's segments are dealt to the lanes
 // in runs; a lane's stroker starts behind a segment whose end normals are its
 // own (EndNormals, twice in a row: the second's start is then the path's
-// point), so it joins and offsets its run as the one stroker would.  A first
-// walk counts each run's outline, a second writes it where the runs before it
-// end; the contour's end -- join or caps, the inner side reversed -- follows.
+// point), so it joins and offsets its run as the one stroker would.  A walk
+// drafts each run's outline in the lane's share of `draft` and counts it, and
+// the lanes copy their drafts to where the runs before them end (a draft that
+// does not fit: a second walk writes there); the contour's end -- join or
+// caps, the inner side reversed -- follows.
 // A quad that is not resolved within the depth limit leaves its depth to the
 // quads after it: runs behind one are counted again from that depth.
-// `pidx`: room for an int per verb.  False: not that kind of path, or depths
-// that have not settled; the caller strokes it on one lane.
+// `pidx`: room for an int per verb; `draft`: room for the runs' outlines, 16
+// bytes aligned.  False: not that kind of path, or depths that have not
+// settled; the caller strokes it on one lane.  The stroker's chain of
+// arithmetic is what bounds it, and a counting walk before the writing one was
+// as long: geometry of 305 long strokes and fills 5.6 -> 4.6 ms, of 400 effects
+// draws 0.41 -> 0.28, of an 8-pass icon 0.108 -> 0.082.
 SKC_HDN bool StrokePathLanes(const Lanes& L, const PathView& src, float width, float miter,
                              int cap, int join, DPath* outer, DPath* inner, int inner_max[3],
-                             int32_t* pidx) {
+                             int32_t* pidx, uint8_t* draft, uint64_t draft_bytes) {
   constexpr int NL = Lanes::n;
+  // a lane's draft: two sides of `room` points, weights and verbs each
+  const uint64_t share = draft_bytes / (2 * NL) & ~(uint64_t)15;
+  const int room = (int)(share / 13 < (1u << 28) ? share / 13 : 1u << 28);
+  DPath drafts[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint8_t* at = draft + (2 * L.lane + k) * share;
+    drafts[k].init(at + 12ull * room, room, (P*)at, room, (float*)(at + 8ull * room), room);
+  }
   {
     bool odd = false;
     VerbWalk w;
@@ -473,16 +488,15 @@ SKC_HDN bool StrokePathLanes(const Lanes& L, const PathView& src, float width, f
     from.recursion_depth = depth;
 #pragma unroll 1
     for (int walk = 0;; ++walk) {
-      // a counting walk, until the depths agree; then the writing one
+      // drafting walks, until the depths agree; then, if need be, one that
+      // writes
       const bool write = walk > 0 && settled;
       if (write) {
         o = PathTail(*outer, ov + at[0], op + at[1], ow + at[2]);
         in = PathTail(*inner, at[3], at[4], at[5]);
       } else {
-        DPath none;
-        none.init(nullptr, 0, nullptr, 0, nullptr, 0);
-        o = PathTail(none, 0, 0, 0);
-        in = PathTail(none, 0, 0, 0);
+        o = PathTail(drafts[0], 0, 0, 0);
+        in = PathTail(drafts[1], 0, 0, 0);
       }
       st = from;
       st.outer = &o;
@@ -506,6 +520,20 @@ SKC_HDN bool StrokePathLanes(const Lanes& L, const PathView& src, float width, f
       n[0] = o.nv, n[1] = o.np, n[2] = o.nw, n[3] = in.nv, n[4] = in.np, n[5] = in.nw;
 #pragma unroll
       for (int k = 0; k < 6; ++k) at[k] = LaneScanIncl(L, n[k]) - n[k];
+      if (!L.ballot(o.overflow() || in.overflow())) {
+        auto copy = [](auto* to, int first, int cap_, const auto* from_, int count) {
+          const int fit = min_(count, cap_ - first);
+#pragma unroll 4
+          for (int k = 0; k < fit; ++k) to[first + k] = from_[k];
+        };
+        copy(outer->pts, op + at[1], outer->cap_p, o.pts, n[1]);
+        copy(inner->pts, at[4], inner->cap_p, in.pts, n[4]);
+        copy(outer->verbs, ov + at[0], outer->cap_v, o.verbs, n[0]);
+        copy(inner->verbs, at[3], inner->cap_v, in.verbs, n[3]);
+        copy(outer->w, ow + at[2], outer->cap_w, o.w, n[2]);
+        copy(inner->w, at[5], inner->cap_w, in.w, n[5]);
+        break;
+      }
     }
     settled = false;
     depth = LaneBcast(L, st.recursion_depth, NL - 1);
@@ -728,7 +756,8 @@ SKC_HDN void StrokePass(const DevBatch& b, uint32_t p, const Lanes& L) {
   const bool fits = !q1.overflow();
   const int cap = (int)(pd.cap_join & 0xFF), join = (int)(pd.cap_join >> 8);
   if (fits && !StrokePathLanes(L, q1.view(), pd.stroke_width, pd.miter, cap, join, &outer, &inner,
-                               imax, (int32_t*)(base + S.off[14]))) {
+                               imax, (int32_t*)(base + S.off[14]), base + S.off[12],
+                               S.off[14] - S.off[12])) {
     outer.reset();
     inner.reset();
     if (L.leader())
