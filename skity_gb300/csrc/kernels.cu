@@ -20,9 +20,9 @@
 
 #include <algorithm>
 
-
-#include "passes.cuh"
 #include "clip.cuh"
+#include "overlap.cuh"
+#include "passes.cuh"
 
 namespace skc {
 
@@ -34,6 +34,7 @@ namespace skc {
 // picture of 305 long outlines 32.7 / 5.6, 512x512 of 1,000 fills 0.70 / 0.09.
 constexpr int kGeomWarps = 4;
 __global__ void __launch_bounds__(32 * kGeomWarps) k_stroke(DevBatch b) {
+  AllowNextLaunch();
   const uint32_t i = blockIdx.x * kGeomWarps + (threadIdx.x >> 5);
   if (i >= b.n_list) return;
   Lanes L;
@@ -41,25 +42,28 @@ __global__ void __launch_bounds__(32 * kGeomWarps) k_stroke(DevBatch b) {
   StrokePass(b, b.pass_list ? b.pass_list[i] : i, L);
 }
 
+// May overlap k_stroke: only the stroked passes need it to be done, and the
+// work queued behind this kernel sees both done.
 __global__ void __launch_bounds__(32 * kGeomWarps) k_edges(DevBatch b) {
   __shared__ SortShared sh[kGeomWarps];
   const uint32_t i = blockIdx.x * kGeomWarps + (threadIdx.x >> 5);
-  if (i >= b.n_list) return;
-  Lanes L;
-  L.lane = threadIdx.x & 31;
-  EdgesPass(b, b.pass_list ? b.pass_list[i] : i, L, &sh[threadIdx.x >> 5]);
+  if (i < b.n_list) {
+    const uint32_t p = b.pass_list ? b.pass_list[i] : i;
+    Lanes L;
+    L.lane = threadIdx.x & 31;
+    if (b.passes[p].flags & kPassStroke) WaitLaunchBefore();
+    EdgesPass(b, p, L, &sh[threadIdx.x >> 5]);
+  }
+  WaitLaunchBefore();
 }
 
 int LaunchGeometry(const DevBatch& b, cudaStream_t stream) {
   if (b.n_list == 0) return 0;
   const uint32_t grid = (b.n_list + kGeomWarps - 1) / kGeomWarps;
-  int n = 1;
-  if (b.any_stroke) {
-    k_stroke<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
-    n++;
-  }
-  k_edges<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
-  return n;
+  if (b.any_stroke) k_stroke<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
+  LaunchOverlapped(k_edges, dim3(grid), dim3(32 * kGeomWarps), 0, stream,
+                   b.any_stroke && b.sweep_done, b);
+  return b.any_stroke ? 2 : 1;
 }
 
 // Sweeps, passes taken in the batch's sweep order
@@ -88,11 +92,6 @@ __device__ __forceinline__ uint32_t SweepPassAt(const DevBatch& b, int form, uin
   if (i >= b.n_passes) return b.n_passes;
   const uint32_t p = b.sweep_order ? b.sweep_order[i] : i;
   return SweepLaunch(b.geom[p], b.pass_class[p]) == form ? p : b.n_passes;
-}
-
-// Lets the next overlapped launch start once every CTA of this one runs.
-__device__ __forceinline__ void AllowNextLaunch() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // End of a sweep kernel that may have overlapped the one before it: the
@@ -197,26 +196,6 @@ __global__ void __launch_bounds__(32 * kSweepWarps) k_sweep(DevBatch b) {
   FinishOverlapped(b.sweep_done ? b.sweep_done + kSweepGeneric : nullptr);
 }
 
-// Launch with programmatic stream serialization: the kernel may start as
-// soon as every CTA of the kernel before it has started (and signalled, at
-// its beginning), so it fills the SMs that kernel's tail leaves idle.  The
-// sweep forms take disjoint passes and read nothing the others write.
-template <typename... Args>
-static void LaunchOverlapped(void (*kernel)(Args...), dim3 grid, dim3 block, size_t smem,
-                             cudaStream_t stream, bool overlap, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int M, int kForm, bool kRaw>
 static void LaunchRegForm(const DevBatch& b, cudaStream_t stream, bool overlap) {
   const uint32_t pairs = b.reg_warps == 4 ? 2 : 1;
@@ -228,9 +207,10 @@ static void LaunchRegForm(const DevBatch& b, cudaStream_t stream, bool overlap) 
                    dim3(64 * pairs), smem, stream, overlap, b);
 }
 
-// The sweep forms in launch order: heaviest first, so the longest sweeps
-// start at once and each later (lighter) form fills the SMs the earlier ones'
-// tails leave idle.  kRaw: the batch has path clips, whose passes keep raw
+// The sweep forms in launch order: heaviest first, so the longest sweeps start
+// at once and each later (lighter) form fills the SMs the earlier ones' tails
+// leave idle.  They may overlap: they take disjoint passes and read nothing
+// the others write.  kRaw: the batch has path clips, whose passes keep raw
 // spans.
 template <bool kRaw>
 static void LaunchForms(const DevBatch& b, cudaStream_t stream, bool overlap) {

@@ -274,7 +274,8 @@ struct PlanStatus {  // zeroed before each render, read back after it
   // the passes of sweep form f are [form_end[f + 1], form_end[f]) of the sweep
   // order (the forms' keys sort in descending order)
   uint32_t form_end[kSweepForms + 1];
-  uint32_t pad;
+  unsigned long long span_used;  // spans the sweeps asked the pool for
+  uint32_t err[4];               // DevBatch::err
 };
 
 struct BandSeg {   // a pass-bin segment: the passes [p0, p1) of the band's canvas

@@ -371,7 +371,7 @@ static int32_t PrepareDevice(skity_cuda_context_s* ctx, DeviceBatch& db, DevBatc
   b.rowspan = db.rowspan.as<uint2>();
   b.pass_spans = db.pass_spans.as<uint32_t>();
   b.pass_frags = db.pass_frags.as<unsigned long long>();
-  b.err = db.err.as<uint32_t>();
+  b.err = db.plan_st.as<PlanStatus>()->err;
   b.pass_class = db.pass_class.as<uint8_t>();
   uint32_t maxw = 1;
   for (const CanvasDesc& cd : hb.canvases) maxw = std::max(maxw, cd.w);
@@ -442,18 +442,13 @@ static int EnqueueDevice(DeviceBatch& db, const DevBatch& b, const DevPlan& q, u
         }
       }
       cudaMemsetAsync(q.st, 0, sizeof(PlanStatus), s);
-      cudaMemsetAsync(b.err, 0, 16, s);
       return LaunchGeometry(b, s);
     case 1:
       return LaunchPlan(b, q, s);
     case 2:
-      cudaMemsetAsync(b.span_next, 0, 8, s);
-      cudaMemsetAsync(b.sweep_done, 0, 4 * kSweepForms, s);
-      cudaMemsetAsync(b.sweep_retry, 0, 4, s);
       return LaunchSweep(b, s);
     case 3:
       if (!q.n_temp) return 0;
-      cudaMemsetAsync(b.task_next, 0, 4, s);
       return LaunchComposite(b, q.tasks_out + q.n_main, q.n_temp, db.chunk, db.cfg.ctas_per_sm,
                              num_sms, b.task_next, s);
     case 4:
@@ -461,7 +456,6 @@ static int EnqueueDevice(DeviceBatch& db, const DevBatch& b, const DevPlan& q, u
       return LaunchBlur(b, db.temps.as<uint32_t>(), (uint32_t)hb.temp_canvases.size(),
                         hb.max_temp_h, hb.max_temp_w, hb.max_temp_style, s);
     default: {
-      cudaMemsetAsync(b.task_next + 1, 0, 4, s);
       int n = LaunchComposite(b, q.tasks_out, q.n_main, db.chunk, db.cfg.ctas_per_sm, num_sms,
                               b.task_next + 1, s);
       return n + LaunchPlanStats(b, q, s);
@@ -548,13 +542,11 @@ static int32_t DeviceRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool tim
     SKC_TRY(cudaEventRecord(ctx->ev1, s));
     SKC_TRY(cudaGetLastError());
     PlanStatus ps;
-    uint32_t err = 0;
-    unsigned long long used = 0;
     SKC_TRY(cudaMemcpyAsync(&ps, q.st, sizeof ps, cudaMemcpyDeviceToHost, s));
-    SKC_TRY(cudaMemcpyAsync(&err, b.err, 4, cudaMemcpyDeviceToHost, s));
-    SKC_TRY(cudaMemcpyAsync(&used, b.span_next, 8, cudaMemcpyDeviceToHost, s));
     SKC_TRY(cudaStreamSynchronize(s));
     st.host_syncs++;
+    const uint32_t err = ps.err[0];
+    const unsigned long long used = ps.span_used;
     if (err) {
       std::fprintf(stderr, "skity_cuda: device self-check failed (code %u)\n", err);
       return SKITY_CUDA_ERROR_DEVICE;

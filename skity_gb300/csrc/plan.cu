@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "overlap.cuh"
 #include "sweep.cuh"
 
 namespace skc {
@@ -70,9 +71,20 @@ __device__ __forceinline__ uint32_t WorkBucket(unsigned long long c, uint32_t bu
   return k < buckets ? k : buckets - 1u;
 }
 
+// The counters of the sweeps and the compositors behind the plan.
+__device__ __forceinline__ void ClearCounters(const DevBatch& b) {
+  *b.span_next = 0;
+  b.sweep_retry[0] = 0;
+  for (int k = 0; k < kSweepForms; ++k) b.sweep_done[k] = 0;
+  b.task_next[0] = b.task_next[1] = 0;
+}
+
 __global__ void __launch_bounds__(kPlanThreads) k_plan_sizes(DevBatch b, DevPlan q) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= b.n_passes) return;
+  if (p == 0) ClearCounters(b);
   const PassGeom g = b.geom[p];
   if (g.status != 0) {
     atomicOr(&q.st->flags, kPlanGeomOverflow);
@@ -90,6 +102,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan_sizes(DevBatch b, DevPlan
 __global__ void __launch_bounds__(kScanThreads)
     k_scan2(unsigned long long* a, unsigned long long* c, uint32_t n, unsigned long long* ta,
             unsigned long long* tc) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   __shared__ unsigned long long wa[32], wc[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   unsigned long long carry_a = 0, carry_c = 0;
@@ -156,6 +170,8 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 
 __global__ void __launch_bounds__(kPlanThreads) k_plan_place(DevBatch b, DevPlan q) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < b.n_passes) {
     const PassGeom g = b.geom[p];
@@ -196,6 +212,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan_place(DevBatch b, DevPlan
 }
 
 __global__ void __launch_bounds__(32 * kBinWarps) k_bin_count(DevPlan q) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   const uint32_t seg = blockIdx.x * kBinWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (seg >= q.n_segs) return;
@@ -214,6 +232,8 @@ __global__ void __launch_bounds__(32 * kBinWarps) k_bin_count(DevPlan q) {
 }
 
 __global__ void __launch_bounds__(32 * kBinWarps) k_bin_fill(DevPlan q) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   const uint32_t seg = blockIdx.x * kBinWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (seg >= q.n_segs) return;
@@ -277,6 +297,8 @@ __device__ __forceinline__ uint32_t SortKey(const DevBatch& b, const DevPlan& q,
 // hist[(nb - 1 - key) * nblocks + block] = items of the block with that key
 __global__ void __launch_bounds__(kSortThreads)
     k_sort_hist(DevBatch b, DevPlan q, int kind, uint32_t n, uint32_t nb) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   __shared__ uint32_t h[kMaxSortKeys];
   for (uint32_t k = threadIdx.x; k < nb; k += kSortThreads) h[k] = 0;
   __syncthreads();
@@ -295,6 +317,8 @@ __global__ void __launch_bounds__(kSortThreads)
 
 __global__ void __launch_bounds__(kSortThreads)
     k_sort_place(DevPlan q, int kind, uint32_t n, uint32_t nb) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   __shared__ uint32_t cur[kMaxSortKeys];
   for (uint32_t k = threadIdx.x; k < nb; k += kSortThreads)
     cur[k] = (uint32_t)q.sort_hist[(unsigned long long)(nb - 1 - k) * gridDim.x + blockIdx.x];
@@ -339,8 +363,11 @@ __device__ __forceinline__ unsigned long long WarpSum64(unsigned long long v) {
 }
 
 __global__ void __launch_bounds__(kPlanThreads) k_plan_stats(DevBatch b, DevPlan q) {
+  WaitLaunchBefore();
+  AllowNextLaunch();
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long spans = 0, edges = 0, f[4] = {0, 0, 0, 0};
+  if (p == 0) q.st->span_used = *b.span_next;
   if (p < b.n_passes) {
     const PassGeom g = b.geom[p];
     if (g.status == 0 && g.n_edges > 0) edges = (unsigned long long)g.n_edges;
@@ -366,14 +393,21 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan_stats(DevBatch b, DevPlan
 
 inline unsigned Blocks(uint64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
+// The plan's kernels are a few us each, one after the other: each is launched
+// while the one before runs, and waits for it inside.
+template <typename... Args>
+void LaunchNext(void (*kernel)(Args...), unsigned blocks, int threads, cudaStream_t s, Args... args) {
+  LaunchOverlapped(kernel, dim3(blocks), dim3(threads), 0, s, true, args...);
+}
+
 int LaunchSort(const DevBatch& b, const DevPlan& q, int kind, uint32_t n, uint32_t nb,
                cudaStream_t s) {
   const unsigned blocks = Blocks(n, kSortItems);
-  k_sort_hist<<<blocks, kSortThreads, 0, s>>>(b, q, kind, n, nb);
-  k_scan2<<<1, kScanThreads, 0, s>>>(q.sort_hist, nullptr, blocks * nb,
-                                      kind == 0 ? &q.st->sort_total[0] : &q.st->sort_total[1],
-                                      nullptr);
-  k_sort_place<<<blocks, kSortThreads, 0, s>>>(q, kind, n, nb);
+  unsigned long long* const none = nullptr;
+  LaunchNext(k_sort_hist, blocks, kSortThreads, s, b, q, kind, n, nb);
+  LaunchNext(k_scan2, 1, kScanThreads, s, q.sort_hist, none, blocks * nb,
+             kind == 0 ? &q.st->sort_total[0] : &q.st->sort_total[1], none);
+  LaunchNext(k_sort_place, blocks, kSortThreads, s, q, kind, n, nb);
   return 3;
 }
 
@@ -381,17 +415,20 @@ int LaunchSort(const DevBatch& b, const DevPlan& q, int kind, uint32_t n, uint32
 
 int LaunchPlan(const DevBatch& b, const DevPlan& q, cudaStream_t s) {
   const uint32_t np = b.n_passes;
+  unsigned long long* const none = nullptr;
   int n = 0;
   if (np) {
     k_plan_sizes<<<Blocks(np, kPlanThreads), kPlanThreads, 0, s>>>(b, q);
-    k_scan2<<<1, kScanThreads, 0, s>>>(q.a, q.r, np, &q.st->sweep_need, &q.st->rows_need);
-    k_plan_place<<<Blocks(np, kPlanThreads), kPlanThreads, 0, s>>>(b, q);
+    LaunchNext(k_scan2, 1, kScanThreads, s, q.a, q.r, np, &q.st->sweep_need, &q.st->rows_need);
+    LaunchNext(k_plan_place, Blocks(np, kPlanThreads), kPlanThreads, s, b, q);
     n += 3 + LaunchSort(b, q, 0, np, kSweepKeys, s);
+  } else {
+    cudaMemsetAsync(b.task_next, 0, 8, s);
   }
   if (q.n_segs) {
-    k_bin_count<<<Blocks(q.n_segs, kBinWarps), 32 * kBinWarps, 0, s>>>(q);
-    k_scan2<<<1, kScanThreads, 0, s>>>(q.seg_cnt, nullptr, q.n_segs, &q.st->bins_need, nullptr);
-    k_bin_fill<<<Blocks(q.n_segs, kBinWarps), 32 * kBinWarps, 0, s>>>(q);
+    LaunchNext(k_bin_count, Blocks(q.n_segs, kBinWarps), 32 * kBinWarps, s, q);
+    LaunchNext(k_scan2, 1, kScanThreads, s, q.seg_cnt, none, q.n_segs, &q.st->bins_need, none);
+    LaunchNext(k_bin_fill, Blocks(q.n_segs, kBinWarps), 32 * kBinWarps, s, q);
     n += 3;
   }
   const uint32_t nt = q.n_main + q.n_temp;
@@ -401,7 +438,7 @@ int LaunchPlan(const DevBatch& b, const DevPlan& q, cudaStream_t s) {
 
 int LaunchPlanStats(const DevBatch& b, const DevPlan& q, cudaStream_t s) {
   if (!b.n_passes) return 0;
-  k_plan_stats<<<Blocks(b.n_passes, kPlanThreads), kPlanThreads, 0, s>>>(b, q);
+  LaunchNext(k_plan_stats, Blocks(b.n_passes, kPlanThreads), kPlanThreads, s, b, q);
   return 1;
 }
 
