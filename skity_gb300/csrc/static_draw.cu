@@ -34,7 +34,9 @@
 
 #include <atomic>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 
 #include "../../include/skity_cuda.h"
 #include "batch.h"
@@ -56,14 +58,21 @@ struct StaticDesc {  // the descriptor block at the start of the scratch
   CanvasDesc canvas;
   Brush brush[2];
   PassGeom geom[2];
-  PassSweep sweep[2];
-  PassComp comp[2];
-  uint32_t err;
-  uint32_t pass_spans[2];
-  uint8_t pass_class[8];
-  unsigned long long pass_frags[2];
-  unsigned long long span_next;
-  uint32_t sweep_retry[3];  // DevBatch::sweep_retry: a count, then at most two passes
+  // what the sweeps start from, written in one copy
+  struct Sweeps {
+    PassSweep sweep[2];
+    PassComp comp[2];
+    uint32_t pass_spans[2];
+    uint8_t pass_class[8];
+    unsigned long long pass_frags[2];
+    uint32_t sweep_retry[3];  // DevBatch::sweep_retry: a count, then at most two passes
+    uint32_t sweep_done[kSweepForms];
+    // the self-check word and the pool use, read back in one copy
+    struct Check {
+      unsigned long long span_next;
+      uint32_t err;
+    } check;
+  } s;
 };
 static_assert(sizeof(StaticDesc) <= kDescBytes, "descriptor block");
 static_assert(sizeof(P) == 8, "points are copied as float pairs");
@@ -99,6 +108,8 @@ inline uint64_t Align256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
 constexpr int kStaticCompWarps = 4;
 __global__ void __launch_bounds__(32 * kStaticCompWarps)
     k_static_composite(DevBatch b, uint32_t p, uint8_t* pixels, size_t row_bytes) {
+  // a failed self-check, or spans that did not fit: no pixel is written
+  if (*b.err != 0 || *b.span_next > b.span_cap) return;
   const int lane = threadIdx.x & 31;
   const PassComp pc = b.comp[p];
   const int y = pc.row0 + (int)(blockIdx.x * kStaticCompWarps + (threadIdx.x >> 5));
@@ -137,9 +148,9 @@ int32_t Err(cudaError_t e) {
 // sized and swept before any of them is composited, so a draw that does not
 // fit the scratch, or whose sweep fails its device self-check, leaves the
 // caller's canvas untouched.  `pd[i]` arrive with their initial capacities;
-// the path copy already sits at `path_off`.
-int32_t StaticDraw(uint8_t* base, uint64_t path_off, uint64_t slice_off0, PassDesc* pd,
-                   const Brush* br, uint32_t npass, const DrawDesc& dd, const CanvasDesc& cd,
+// `head`: the descriptor's place and the path, copied to the scratch's start.
+int32_t StaticDraw(uint8_t* base, uint8_t* head, uint64_t path_off, uint64_t path_bytes,
+                   uint64_t slice_off0, PassDesc* pd, const Brush* br, uint32_t npass, const DrawDesc& dd, const CanvasDesc& cd,
                    uint8_t* pixels, size_t row_bytes, cudaStream_t st) {
   StaticDesc* dev = (StaticDesc*)base;
   DevBatch b;
@@ -150,14 +161,15 @@ int32_t StaticDraw(uint8_t* base, uint64_t path_off, uint64_t slice_off0, PassDe
   b.n_passes = npass;
   b.canvases = &dev->canvas;
   b.geom = dev->geom;
-  b.sweep = dev->sweep;
-  b.pass_spans = dev->pass_spans;
-  b.pass_frags = dev->pass_frags;
-  b.err = &dev->err;
-  b.comp = dev->comp;
+  b.sweep = dev->s.sweep;
+  b.pass_spans = dev->s.pass_spans;
+  b.pass_frags = dev->s.pass_frags;
+  b.err = &dev->s.check.err;
+  b.sweep_done = dev->s.sweep_done;
+  b.comp = dev->s.comp;
   b.brushes = dev->brush;
-  b.pass_class = dev->pass_class;
-  b.sweep_retry = dev->sweep_retry;
+  b.pass_class = dev->s.pass_class;
+  b.sweep_retry = dev->s.sweep_retry;
   b.pixels = pixels;
   b.n_list = npass;
   for (uint32_t i = 0; i < npass; ++i) b.any_stroke |= pd[i].flags & kPassStroke;
@@ -189,7 +201,9 @@ int32_t StaticDraw(uint8_t* base, uint64_t path_off, uint64_t slice_off0, PassDe
     if (slices_end > kStaticScratchBytes) return SKITY_CUDA_ERROR_SCRATCH_LIMIT;
     h.draw = dd;
     h.canvas = cd;
-    cudaError_t e = cudaMemcpyAsync(dev, &h, sizeof h, cudaMemcpyHostToDevice, st);
+    std::memcpy(head, &h, sizeof h);
+    cudaError_t e = cudaMemcpyAsync(dev, head, attempt == 0 ? path_off + path_bytes : sizeof h,
+                                    cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return Err(e);
     LaunchGeometry(b, st);
     e = cudaGetLastError();
@@ -209,10 +223,10 @@ int32_t StaticDraw(uint8_t* base, uint64_t path_off, uint64_t slice_off0, PassDe
 
   // sweep memory and row tables of every pass after the slices, then one
   // span pool (the rest of the scratch) shared by the passes
-  PassSweep sw[2];
-  PassComp pc[2];
-  std::memset(sw, 0, sizeof sw);
-  std::memset(pc, 0, sizeof pc);
+  StaticDesc::Sweeps init;
+  std::memset(&init, 0, sizeof init);
+  PassSweep* sw = init.sweep;
+  PassComp* pc = init.comp;
   uint64_t sweep_total = 0, rows_total = 0;
   uint32_t chunk_max = 0;
   bool any = false;
@@ -246,45 +260,25 @@ int32_t StaticDraw(uint8_t* base, uint64_t path_off, uint64_t slice_off0, PassDe
   b.rowspan = (uint2*)(base + rows_off);
   b.spans = (uint2*)(base + spans_off);
   b.span_cap = span_cap;
-  b.span_next = &dev->span_next;
+  b.span_next = &dev->s.check.span_next;
 
-  cudaError_t e = cudaMemcpyAsync(dev->sweep, sw, sizeof(PassSweep) * npass,
-                                  cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dev->comp, pc, sizeof(PassComp) * npass, cudaMemcpyHostToDevice, st);
-  // empty rows read as (0, 0); the flag, the sweep forms and the pool
-  // allocator start clear
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.rowspan, 0, sizeof(uint2) * rows_total, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&dev->err, 0, sizeof(uint32_t), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dev->pass_class, 0, sizeof dev->pass_class, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&dev->span_next, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dev->sweep_retry, 0, sizeof dev->sweep_retry, st);
+  cudaError_t e = cudaMemcpyAsync(&dev->s, &init, sizeof init, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return Err(e);
   LaunchSweep(b, st);
-  // the sweeps' self-check word and pool use, both read before any pixel is
-  // written
-  struct {
-    uint32_t err;
-    unsigned long long used;
-  } chk = {0, 0};
-  e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&chk.used, &dev->span_next, sizeof chk.used, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&chk.err, &dev->err, sizeof chk.err, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return Err(e);
-  if (chk.err) return SKITY_CUDA_ERROR_DEVICE;
-  if (chk.used > span_cap) return SKITY_CUDA_ERROR_SCRATCH_LIMIT;
   for (uint32_t i = 0; i < npass; ++i) {
     const int nrows = pc[i].row1 - pc[i].row0;
     if (nrows <= 0) continue;
     const unsigned grid = (unsigned)((nrows + kStaticCompWarps - 1) / kStaticCompWarps);
     k_static_composite<<<grid, 32 * kStaticCompWarps, 0, st>>>(b, i, pixels, row_bytes);
   }
+  StaticDesc::Sweeps::Check chk = {0, 0};
   e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&chk, &dev->s.check, sizeof chk, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  return Err(e);
+  if (e != cudaSuccess) return Err(e);
+  if (chk.err) return SKITY_CUDA_ERROR_DEVICE;
+  return chk.span_next > span_cap ? SKITY_CUDA_ERROR_SCRATCH_LIMIT : SKITY_CUDA_SUCCESS;
 }
 
 int32_t DrawStatic(uint8_t* base, uint8_t* pixels, uint32_t width, uint32_t height,
@@ -297,14 +291,13 @@ int32_t DrawStatic(uint8_t* base, uint8_t* pixels, uint32_t width, uint32_t heig
   const uint64_t path_bytes = Align256(nv) + Align256(8ull * np) + Align256(4ull * nw);
   const uint64_t slice_off0 = Align256(path_off + path_bytes);
   if (slice_off0 > kStaticScratchBytes) return SKITY_CUDA_ERROR_SCRATCH_LIMIT;
-  cudaError_t e = cudaMemcpyAsync(base + path_off, path->verbs, nv, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && np)
-    e = cudaMemcpyAsync(base + path_off + Align256(nv), path->points, 8ull * np,
-                        cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && nw)
-    e = cudaMemcpyAsync(base + path_off + Align256(nv) + Align256(8ull * np), path->conic_weights,
-                        4ull * nw, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return Err(e);
+  std::unique_ptr<uint8_t[]> head(new (std::nothrow) uint8_t[path_off + path_bytes]);
+  if (!head) return SKITY_CUDA_ERROR_OUT_OF_HOST_MEMORY;
+  std::memcpy(head.get() + path_off, path->verbs, nv);
+  if (np) std::memcpy(head.get() + path_off + Align256(nv), path->points, 8ull * np);
+  if (nw)
+    std::memcpy(head.get() + path_off + Align256(nv) + Align256(8ull * np), path->conic_weights,
+                4ull * nw);
 
   DrawDesc dd;
   dd.v0 = 0;
@@ -352,7 +345,7 @@ int32_t DrawStatic(uint8_t* base, uint8_t* pixels, uint32_t width, uint32_t heig
     if (need_fill) pass(false);
     if (need_stroke) pass(true);
   }
-  return StaticDraw(base, path_off, slice_off0, pd, br, npass, dd, cd, pixels, row_bytes, st);
+  return StaticDraw(base, head.get(), path_off, path_bytes, slice_off0, pd, br, npass, dd, cd, pixels, row_bytes, st);
 }
 
 }  // namespace
