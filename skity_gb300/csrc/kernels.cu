@@ -30,11 +30,12 @@ namespace skc {
 // quads, edges and sort.  With the whole chain on one thread, packed 1 to 32
 // passes a warp, it was the batch's longest passes' serial chains, and half of
 // a stroke's was double arithmetic (1/64 of the float rate).  Before / after:
-// the 20,000-path scene 36.4 / 6.8 ms, 64 canvases of fills 3.3 / 0.84, a
-// picture of 305 long outlines 32.7 / 5.6, 512x512 of 1,000 fills 0.70 / 0.09.
+// the 20,000-path scene 36.4 / 5.7 ms, 64 canvases of fills 3.3 / 0.84, a
+// picture of 305 long outlines 32.7 / 4.6, 512x512 of 1,000 fills 0.70 / 0.09.
+// (k_edges overlapping k_stroke, stroked passes alone waiting for it, is
+// slower: 6.3 ms for the scene, and 2.58 instead of 2.13 for 110,000 glyphs.)
 constexpr int kGeomWarps = 4;
 __global__ void __launch_bounds__(32 * kGeomWarps) k_stroke(DevBatch b) {
-  AllowNextLaunch();
   const uint32_t i = blockIdx.x * kGeomWarps + (threadIdx.x >> 5);
   if (i >= b.n_list) return;
   Lanes L;
@@ -42,28 +43,25 @@ __global__ void __launch_bounds__(32 * kGeomWarps) k_stroke(DevBatch b) {
   StrokePass(b, b.pass_list ? b.pass_list[i] : i, L);
 }
 
-// May overlap k_stroke: only the stroked passes need it to be done, and the
-// work queued behind this kernel sees both done.
 __global__ void __launch_bounds__(32 * kGeomWarps) k_edges(DevBatch b) {
   __shared__ SortShared sh[kGeomWarps];
   const uint32_t i = blockIdx.x * kGeomWarps + (threadIdx.x >> 5);
-  if (i < b.n_list) {
-    const uint32_t p = b.pass_list ? b.pass_list[i] : i;
-    Lanes L;
-    L.lane = threadIdx.x & 31;
-    if (b.passes[p].flags & kPassStroke) WaitLaunchBefore();
-    EdgesPass(b, p, L, &sh[threadIdx.x >> 5]);
-  }
-  WaitLaunchBefore();
+  if (i >= b.n_list) return;
+  Lanes L;
+  L.lane = threadIdx.x & 31;
+  EdgesPass(b, b.pass_list ? b.pass_list[i] : i, L, &sh[threadIdx.x >> 5]);
 }
 
 int LaunchGeometry(const DevBatch& b, cudaStream_t stream) {
   if (b.n_list == 0) return 0;
   const uint32_t grid = (b.n_list + kGeomWarps - 1) / kGeomWarps;
-  if (b.any_stroke) k_stroke<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
-  LaunchOverlapped(k_edges, dim3(grid), dim3(32 * kGeomWarps), 0, stream,
-                   b.any_stroke && b.sweep_done, b);
-  return b.any_stroke ? 2 : 1;
+  int n = 1;
+  if (b.any_stroke) {
+    k_stroke<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
+    n++;
+  }
+  k_edges<<<grid, 32 * kGeomWarps, 0, stream>>>(b);
+  return n;
 }
 
 // Sweeps, passes taken in the batch's sweep order
