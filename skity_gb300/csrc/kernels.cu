@@ -315,6 +315,13 @@ struct BrushHead {
   uint32_t kind, blend, solid, global_alpha;
 };
 
+// The spans of a pass row are one dependent load behind its row entry; those
+// of 32 passes start on their way to the L2 at once (64 canvases of 50-2,000
+// paths: 3.52 -> 3.28 ms; spans in registers two passes ahead instead: 3.56).
+__device__ __forceinline__ void PrefetchL2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // How a pass's pixels are made.
 //   solid:    a src-over fill without a colour filter: the span's colour is
 //             made once a span, and a pixel is one PMSrcOver.  FastBlend's
@@ -504,6 +511,8 @@ __device__ __forceinline__ void CompositeTile(const DevBatch& b, const RowTask& 
       bh.solid = q.solid;
       bh.global_alpha = q.global_alpha;
     }
+    if (rs.y != 0) PrefetchL2(b.spans + rs.x);
+    if (rs.y > 16) PrefetchL2(b.spans + rs.x + 16);
     uint32_t mask = __ballot_sync(0xffffffffu, rs.y != 0);
     // the first 32 spans of a pass are loaded while the pass before is blended
     auto first_spans = [&](uint32_t m) {
