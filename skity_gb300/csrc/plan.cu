@@ -55,7 +55,7 @@ __device__ __forceinline__ void PassNeeds(const PassGeom& g, unsigned long long*
 // Sort key of a work estimate: 0 for no work, else 2^kBits buckets per octave
 // (1 + 2^kBits floor(log2 c) + the next kBits bits of c), at most `buckets` -
 // 1: the tile order below is by work to within about 9% (3 bits), the sweep
-// order to within 19% (2 bits), ties in index order.
+// order to within 19% (2 bits).
 constexpr uint32_t kSortBuckets = 512;    // of a work estimate, tiles
 constexpr uint32_t kSweepBuckets = 128;   // of a work estimate, sweeps
 // the sweep order's keys: kSweepBuckets per form, the forms in the order of
@@ -261,12 +261,12 @@ __global__ void __launch_bounds__(32 * kBinWarps) k_bin_fill(DevPlan q) {
   }
 }
 
-// ---- stable descending bucket sort (sweep order and tile order) ----------
-// Items are sorted by their key, heaviest first, items of equal key in index
-// order: a counting sort over blocks of kSortItems items -- per-block key
-// histograms, one prefix sum over (key descending, block), then each block
-// places its items, warp by warp, ranking equal keys inside a warp with
-// __match_any_sync.
+// ---- descending bucket sort (sweep order and tile order) -------------------
+// Items are sorted by their key, heaviest first: a counting sort over blocks
+// of kSortItems items -- per-block key histograms, one prefix sum over (key
+// descending, block), then each block places its items, equal keys in any
+// order (it is an order of work, no pixel depends on it; keeping the items in
+// index order, the warps in turns, made plans of small batches 21 us longer).
 constexpr uint32_t kMaxSortKeys = 2 * kSortBuckets;
 static_assert(kSweepKeys <= kMaxSortKeys, "shared histograms");
 constexpr int kSortThreads = 256;
@@ -331,28 +331,13 @@ __global__ void __launch_bounds__(kSortThreads)
         (uint32_t)q.sort_hist[(unsigned long long)(nb - 1 - key) * gridDim.x];
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
   const uint32_t i0 = blockIdx.x * kSortItems;
-  for (uint32_t base = 0; base < (uint32_t)kSortItems; base += kSortThreads) {
-    const uint32_t i = i0 + base + threadIdx.x;
-    const bool valid = i < n;
-    const uint32_t key = valid ? q.sort_keys[i] : 0xFFFFFFFFu;
-    // warps of the round in order, so equal keys keep their index order
-    for (int ww = 0; ww < kSortThreads / 32; ++ww) {
-      if (w == ww) {
-        const uint32_t peers = __match_any_sync(0xffffffffu, key);
-        if (valid) {
-          const uint32_t rank = __popc(peers & lt);
-          const uint32_t pos = cur[key] + rank;
-          if (kind == 0) q.sweep_order[pos] = i;
-          else q.tasks_out[pos] = q.tasks_in[i];
-          __syncwarp(peers);
-          if ((peers >> lane) == 1u) cur[key] += __popc(peers);  // the group's last lane
-        }
-      }
-      __syncthreads();
-    }
+  for (uint32_t j = threadIdx.x; j < kSortItems; j += kSortThreads) {
+    const uint32_t i = i0 + j;
+    if (i >= n) break;
+    const uint32_t pos = atomicAdd(&cur[q.sort_keys[i]], 1u);
+    if (kind == 0) q.sweep_order[pos] = i;
+    else q.tasks_out[pos] = q.tasks_in[i];
   }
 }
 
