@@ -1847,6 +1847,33 @@ inline uint64_t PlanPathClips(HostBatch& hb, const std::vector<PassGeom>& geom,
   return rbase;
 }
 
+// The states with rows, by generation: those without a parent, then those
+// whose parent is one of the generation before, and so on.
+inline void PlanClipGens(const HostBatch& hb, std::vector<uint32_t>& order,
+                         std::vector<ClipGen>& gens) {
+  const std::vector<ClipStateDesc>& states = hb.clip_states;
+  std::vector<uint32_t> gen(states.size());
+  gens.clear();
+  for (size_t k = 0; k < states.size(); ++k) {  // a parent comes before its children
+    const ClipStateDesc& st = states[k];
+    gen[k] = st.parent ? gen[st.parent - 1] + 1 : 0;
+    if (st.y1 <= st.y0) continue;
+    if (gen[k] >= gens.size()) gens.resize(gen[k] + 1, ClipGen{0, 0, 0});
+    gens[gen[k]].count++;
+    gens[gen[k]].rows = std::max(gens[gen[k]].rows, (uint32_t)(st.y1 - st.y0));
+  }
+  uint32_t n = 0;
+  for (ClipGen& g : gens) {
+    g.first = n;
+    n += g.count;
+  }
+  order.resize(n);
+  std::vector<uint32_t> at;
+  for (const ClipGen& g : gens) at.push_back(g.first);
+  for (size_t k = 0; k < states.size(); ++k)
+    if (states[k].y1 > states[k].y0) order[at[gen[k]]++] = (uint32_t)k + 1;
+}
+
 // The order in which the sweeps take the passes: longest expected sweep
 // first (rows times the bound of the active list), so that the long sweeps
 // start early instead of forming the tail of the launch.

@@ -70,7 +70,8 @@ struct DeviceBatch {
   RasterConfig cfg;
   DevBuf task_next;  // persistent compositor's counters
   DevBuf retry;      // DevBatch::sweep_retry
-  DevBuf clip_states, clip_flags, clip_rows, clip_items;  // path clips
+  DevBuf clip_states, clip_flags, clip_rows, clip_items, clip_order;  // path clips
+  std::vector<ClipGen> clip_gens;
   // device planning (batches without path clips): status, per-pass scan
   // arrays and band ranges, bin segments, the tiles (main then temp) and
   // their sorted copy; capacities of the plan's buffers

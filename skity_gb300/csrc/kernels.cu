@@ -576,37 +576,42 @@ int LaunchComposite(const DevBatch& b, const RowTask* tasks, uint32_t n_tasks, u
 }
 
 // ---------------------------------------------------------------------------
-// Path clips (clip.cuh): each clip state's span rows, one launch per state
-// in order (a state reads its parent's rows and whether the parent's list
-// is empty, known only once the parent's launch is complete), then the rows
-// of the draws under a clip, one thread per (pass, row).
+// Path clips (clip.cuh): the clip states' span rows, a thread a row, one
+// launch per generation (a state reads its parent's rows and whether the
+// parent's list is empty, known only once the parent's launch is complete;
+// with a launch per state, 24 states in groups of three took 0.4 ms longer),
+// then the rows of the draws under a clip, one thread per (pass, row).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_clip_state(DevBatch b, uint32_t k, int32_t y0, int32_t y1) {
-  const int32_t y = y0 + (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (y >= y1) return;
+constexpr int kClipThreads = 128;
+__global__ void __launch_bounds__(kClipThreads) k_clip_state(DevBatch b, const uint32_t* states) {
+  const uint32_t k = states[blockIdx.y];
+  const ClipStateDesc& st = b.clip_states[k - 1];
+  const int32_t y = st.y0 + (int32_t)(blockIdx.x * kClipThreads + threadIdx.x);
+  if (y >= st.y1) return;
   int32_t order[kClipRowCap];
   ClipStateStage(b, k, y, order);
 }
 
-__global__ void __launch_bounds__(128) k_clip_apply(DevBatch b) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kClipThreads) k_clip_apply(DevBatch b) {
+  const uint32_t i = blockIdx.x * kClipThreads + threadIdx.x;
   if (i >= b.n_clip_items) return;
   int32_t order[kClipRowCap];
   ClipApplyStage(b, i, order);
 }
 
-int LaunchPathClips(const DevBatch& b, const ClipStateDesc* states, uint32_t n_states,
+int LaunchPathClips(const DevBatch& b, const uint32_t* order, const ClipGen* gens, size_t n_gens,
                     cudaStream_t stream) {
   int launches = 0;
-  for (uint32_t k = 1; k <= n_states; ++k) {
-    const ClipStateDesc& st = states[k - 1];
-    if (st.y1 <= st.y0) continue;
-    const uint32_t rows = (uint32_t)(st.y1 - st.y0);
-    k_clip_state<<<(rows + 127) / 128, 128, 0, stream>>>(b, k, st.y0, st.y1);
-    launches++;
+  for (size_t g = 0; g < n_gens; ++g) {
+    for (uint32_t at = 0; at < gens[g].count; at += 65535) {
+      const dim3 grid((gens[g].rows + kClipThreads - 1) / kClipThreads,
+                      std::min(gens[g].count - at, 65535u));
+      k_clip_state<<<grid, kClipThreads, 0, stream>>>(b, order + gens[g].first + at);
+      launches++;
+    }
   }
   if (b.n_clip_items) {
-    k_clip_apply<<<(b.n_clip_items + 127) / 128, 128, 0, stream>>>(b);
+    k_clip_apply<<<(b.n_clip_items + kClipThreads - 1) / kClipThreads, kClipThreads, 0, stream>>>(b);
     launches++;
   }
   return launches;

@@ -64,6 +64,11 @@ struct ClipStateDesc {
   uint32_t rbase;       // first entry of its rows in DevBatch::clip_rows
 };
 
+struct ClipGen {  // path-clip states that depend on none of each other
+  uint32_t first, count;  // their places in the order of the states by generation
+  uint32_t rows;          // most rows of one of them
+};
+
 struct DrawDesc {  // a Path inside the batch's verb/point/weight arrays
   uint32_t v0, nv, p0, np, w0, nw;
 };
@@ -318,8 +323,9 @@ constexpr int32_t kRegDiffMax = 3072;
 // number of launches made
 int LaunchGeometry(const DevBatch& b, cudaStream_t stream);
 int LaunchSweep(const DevBatch& b, cudaStream_t stream);
-// the path-clip stages after the sweeps; states: the host copy of b.clip_states
-int LaunchPathClips(const DevBatch& b, const ClipStateDesc* states, uint32_t n_states,
+// the path-clip stages after the sweeps; order: the states with rows (1-based)
+// by generation, on the device; gens: its generations
+int LaunchPathClips(const DevBatch& b, const uint32_t* order, const ClipGen* gens, size_t n_gens,
                     cudaStream_t stream);
 // ctas_per_sm > 0: a persistent grid of ctas_per_sm CTAs per SM taking row
 // tiles from `counter` (zeroed before the launch); 0: one warp per tile.

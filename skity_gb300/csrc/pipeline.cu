@@ -188,7 +188,7 @@ static int EnqueuePlanned(skity_cuda_context_s* ctx, DeviceBatch& db, cudaStream
         int n = LaunchSweep(b, s);
         if (b.n_clip_states || b.n_clip_items) {
           cudaMemsetAsync(b.clip_flags, 0, 8 * (size_t)std::max<uint32_t>(b.n_clip_states, 1), s);
-          n += LaunchPathClips(b, hb.clip_states.data(), b.n_clip_states, s);
+          n += LaunchPathClips(b, db.clip_order.as<uint32_t>(), db.clip_gens.data(), db.clip_gens.size(), s);
         }
         return n;
       }
@@ -767,6 +767,9 @@ static int32_t PlanAndRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool ti
   if (clip_state_rows >= 0xFFFFFFFFull || clip_items.size() >= 0xFFFFFFFFull)
     return SKITY_CUDA_ERROR_OUT_OF_DEVICE_MEMORY;
   if (!hb.clip_states.empty()) SKC_TRY(Upload(db.clip_states, hb.clip_states, s));
+  std::vector<uint32_t> clip_order;
+  PlanClipGens(hb, clip_order, db.clip_gens);
+  if (!clip_order.empty()) SKC_TRY(Upload(db.clip_order, clip_order, s));
   SKC_TRY(db.clip_flags.ensure(8 * std::max<size_t>(hb.clip_states.size(), 1)));
   SKC_TRY(db.clip_rows.ensure(8 * std::max<uint64_t>(clip_state_rows, 1)));
   if (!clip_items.empty()) SKC_TRY(Upload(db.clip_items, clip_items, s));
@@ -830,7 +833,7 @@ static int32_t PlanAndRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool ti
     st.kernel_launches += LaunchSweep(b, s);
     if (b.n_clip_states || b.n_clip_items) {  // the path-clip stages use the span pool too
       SKC_TRY(cudaMemsetAsync(b.clip_flags, 0, 8 * (size_t)std::max<uint32_t>(b.n_clip_states, 1), s));
-      st.kernel_launches += LaunchPathClips(b, hb.clip_states.data(), b.n_clip_states, s);
+      st.kernel_launches += LaunchPathClips(b, db.clip_order.as<uint32_t>(), db.clip_gens.data(), db.clip_gens.size(), s);
     }
     SKC_TRY(cudaEventRecord(ctx->stage[5], s));
     SKC_TRY(cudaGetLastError());
