@@ -546,51 +546,53 @@ SKC_HD uint64_t StackBlurMul(int32_t r) {
   return ((1ull << StackBlurShr(r)) + d - 1) / d;
 }
 
-// Blur one line of n pixels (stride in pixels) from src into dst. v_bug
-// reproduces the vertical pass's out_sum initialisation (slots 0 and 3 from
-// slot 1, sw_stack_blur.cc:175-179).
-SKC_HDN void BlurLine(const uint8_t* src, uint8_t* dst, int n, size_t stride, int r, bool v_bug) {
+// Blur one channel of a line of n pixels (`step` bytes apart) from src into
+// dst (`out_step` bytes apart), both at the channel's first byte.  out0: the pixel value that the
+// out_sum starts from -- the channel's own first one, or, in the vertical
+// pass, slot 1's for slots 0 and 3 (sw_stack_blur.cc:175-179).  Sums are
+// modulo the reference's 64 bits; Sum = int32_t where they stay below 2^31.
+template <typename Sum>
+SKC_HD void BlurChannelSums(const uint8_t* __restrict__ src, size_t step,
+                            uint8_t* __restrict__ dst, size_t out_step, int n, int r, int out0) {
   const int rp1 = r + 1;
   const int nm1 = n - 1;
-  const uint64_t sum_factor = (uint64_t)(rp1 * (rp1 + 1) / 2);
-  const uint64_t mul = StackBlurMul(r);
+  const int64_t mul = (int64_t)StackBlurMul(r);
   const int shr = StackBlurShr(r);
-  auto px = [&](int i, int c) -> uint64_t { return src[(size_t)i * stride * 4 + c]; };
-  uint64_t sum[4], in_sum[4], out_sum[4];
-  for (int c = 0; c < 4; ++c) {
-    uint64_t p0 = px(0, c);
-    sum[c] = p0 * sum_factor;
-    out_sum[c] = p0 * rp1;
-    in_sum[c] = 0;
-  }
-  if (v_bug) {
-    out_sum[0] = px(0, 1) * rp1;
-    out_sum[3] = px(0, 1) * rp1;
-  }
+  auto px = [&](int i) -> Sum { return (Sum)src[(size_t)i * step]; };
+  Sum sum = px(0) * (Sum)(rp1 * (rp1 + 1) / 2), in_sum = 0, out_sum = (Sum)out0 * (Sum)rp1;
+#pragma unroll 4
   for (int i = 1; i <= r; ++i) {
-    int k = min_(i, nm1);
-    for (int c = 0; c < 4; ++c) {
-      uint64_t v = px(k, c);
-      sum[c] += v * (uint64_t)(rp1 - i);
-      in_sum[c] += v;
-    }
+    const Sum v = px(min_(i, nm1));
+    sum += v * (Sum)(rp1 - i);
+    in_sum += v;
   }
+#pragma unroll 4
   for (int i = 0; i < n; ++i) {
-    uint8_t* o = dst + (size_t)i * stride * 4;
-    int kout = max_(i - r, 0), kin = min_(i + rp1, nm1), kmid = min_(i + 1, nm1);
-    for (int c = 0; c < 4; ++c) {
-      o[c] = (uint8_t)((sum[c] * mul) >> shr);
-      sum[c] -= out_sum[c];
-      out_sum[c] -= px(kout, c);
-      in_sum[c] += px(kin, c);
-      sum[c] += in_sum[c];
-      uint64_t vm = px(kmid, c);
-      out_sum[c] += vm;
-      in_sum[c] -= vm;
-    }
+    const Sum out = px(max_(i - r, 0)), in = px(min_(i + rp1, nm1)), mid = px(min_(i + 1, nm1));
+    // the low bits of the 64-bit product, whichever sign the sum has
+    dst[(size_t)i * out_step] = (uint8_t)(((int64_t)sum * mul) >> shr);
+    in_sum += in;
+    sum += in_sum - out_sum;
+    out_sum += mid - out;
+    in_sum -= mid;
   }
 }
+SKC_HD void BlurChannel(const uint8_t* src, size_t step, uint8_t* dst, size_t out_step, int n,
+                        int r, int out0) {
+  // a wrong start of out_sum is off by at most 255 (r + 1), on every pixel
+  if ((int64_t)(n + r + 1) * 255 * (r + 1) < (1ll << 31))
+    BlurChannelSums<int32_t>(src, step, dst, out_step, n, r, out0);
+  else
+    BlurChannelSums<int64_t>(src, step, dst, out_step, n, r, out0);
+}
 
+// Blur one line of n pixels (stride in pixels) from src into dst (v: the
+// vertical pass).
+SKC_HDN void BlurLine(const uint8_t* src, uint8_t* dst, int n, size_t stride, int r, bool v) {
+  for (int c = 0; c < 4; ++c)
+    BlurChannel(src + c, 4 * stride, dst + c, 4 * stride, n, r,
+                src[v && (c == 0 || c == 3) ? 1 : c]);
+}
 
 // Scalar composite of one row task (CPU execution of the pipeline; the GPU
 // runs the warp-parallel form in kernels.cu with identical per-pixel order).
