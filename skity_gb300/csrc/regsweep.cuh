@@ -710,7 +710,10 @@ SKC_HD int RegWalk(const Lanes& L, Sh& sh, const Edge* W, int n, bool even_odd, 
   bool final_in = false;
   Fixed lmin = kMaxS32, lnext = kMaxS32;
   bool cross = false, changed = true;
-  int nrec = 0;
+  // records to log before the hand-over: few at first, so that the emission of
+  // a short pass does not wait for a full log (110,000 glyphs 6.99 -> 6.82 ms,
+  // 64 canvases of fills 13.46 -> 13.39)
+  int nrec = 0, limit = min_(R, 16);
   L.sync();
 
 #pragma unroll 1
@@ -755,7 +758,7 @@ SKC_HD int RegWalk(const Lanes& L, Sh& sh, const Edge* W, int n, bool even_odd, 
         lnext = LaneMin(L, l1);
         changed = false;
       }
-      if (nrec + K > R) break;  // the buffer is full: emit, then take the step
+      if (nrec + K > limit && nrec > 0) break;  // full: emit, then take the step
       Fixed nny = min_(lnext, pend_y);
       if (cross) nny = min_(nny, y + (kFixed1 >> kAccuracy));
       cross = false;
@@ -990,6 +993,7 @@ SKC_HD int RegWalk(const Lanes& L, Sh& sh, const Edge* W, int n, bool even_odd, 
       }
     }
     lg = hand(nrec, done);
+    limit = min_(R, 2 * limit);
     nrec = 0;
     if (done) break;
   }
