@@ -153,31 +153,31 @@ def issue_roofline(st, frame_ms, composite_ms, clk, sms):
 
 
 # The sweep stage's counters per emitted span, from an ncu capture of the
-# 256-canvas workload's first 64 canvases (profiles/k_sweep_reg_config3_64canvases.md):
-# warp instructions executed and DRAM bytes (read + write) of the five sweep
-# launches of one render (17.440 G instructions, 1.854 GB) over the
+# 256-canvas workload's first 64 canvases (profiles/k_sweep_pair_config3_64canvases.md):
+# warp instructions executed and DRAM bytes (read + write) of the six sweep
+# launches of one render (11.616 G instructions, 1.569 GB) over the
 # 165,827,810 spans they emit.  Multiplied by the spans of the timed render
 # (the units one launch processes) they give the per-render figures.
-SWEEP_PER_SPAN = {"warp_inst": 105.17, "dram_bytes": 11.18}
+SWEEP_PER_SPAN = {"warp_inst": 70.05, "dram_bytes": 9.46}
 
 
 def sweep_roofline(st, sweep_ms, clk, sms, hbm_peak, hbm_kind):
     """Roofline of the dominant kernel, the AAA sweep.  It is neither
-    HBM- nor tensor-bound: one warp per path walks the path's rows in order,
+    HBM- nor tensor-bound: two warps per path walk the path's rows in order,
     so its bound is instruction issue (SMs x 4 schedulers x 1 warp
     instruction per cycle at the sampled SM clock).  achieved = the sweep's
     warp instructions per render (ncu count per span x the render's spans)
     / the sweep stage's CUDA-event time; traffic = its DRAM bytes per render
     (ncu, scaled the same way).  Beside it, the HBM view: the sweep's
-    algorithmic bytes (84-byte edges read and written, 8-byte spans
+    algorithmic bytes (76-byte edges read and written, 8-byte spans
     written) over the same time against the measured copy bandwidth."""
     mhz = clk.get("sm_mhz") or 2070.0
     spans, edges = st["spans"], st["edges"]
-    alg = spans * 8 + edges * 84 * 2
+    alg = spans * 8 + edges * 76 * 2
     hbm = {"algorithmic_bytes": alg, "achieved_gbs": alg / (sweep_ms / 1e3) / 1e9,
            "peak_gbs": hbm_peak, "peak_source": hbm_kind}
     hbm["frac"] = hbm["achieved_gbs"] / hbm_peak
-    out = {"kernel": "sweep (k_sweep_reg<32/64/128>, k_sweep, k_sweep_retry)", "sweep_ms": sweep_ms, "hbm": hbm}
+    out = {"kernel": "sweep (k_sweep_pair<32/64/128/256>, k_sweep, k_sweep_retry)", "sweep_ms": sweep_ms, "hbm": hbm}
     if SWEEP_PER_SPAN["warp_inst"]:
         inst = SWEEP_PER_SPAN["warp_inst"] * spans
         peak = sms * 4 * mhz * 1e6 / 1e9
