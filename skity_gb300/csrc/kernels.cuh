@@ -176,6 +176,9 @@ struct PassComp {       // per-pass data the compositor reads
   uint32_t brush;
 };
 
+// What walking a row's spans costs a compositor tile, in pixels of its width.
+constexpr uint32_t kTileSpans = 219;
+
 struct RowTask {
   uint32_t canvas, y, x0, x1;
 };

@@ -63,25 +63,11 @@ static int32_t UploadDevicePlanInputs(skity_cuda_context_s* ctx, DeviceBatch& db
   return SKITY_CUDA_SUCCESS;
 }
 
-// Width of a compositor row tile: the configured width at most, less when the
-// canvases have too few rows to give every warp of the chip a tile (152 SMs x
-// 24 warps).  A tile is one warp's serial work, so one canvas of 512 rows left
-// most warps idle; but every tile of a row walks all of the row's spans, so
-// not narrower than 64 pixels nor more tiles than that.  1,000 paths on 512 x
-// 512: 1.16 -> 0.78 ms; 400 draws on 1204 x 803: 1.11 -> 0.75.  Half the tiles
-// 0.83 and 0.83, twice as many 0.79 and 0.84 (and 17.9 -> 20.4 ms of 3,000
-// paths on 2048 x 2048, which 3,648 tiles leave as it was).
-static uint32_t TileWidth(const HostBatch& hb, uint32_t tile_w) {
-  constexpr uint64_t kTiles = 3648;
-  uint32_t maxw = 1;
-  uint64_t rows = 0;
-  for (uint32_t c : hb.main_canvases) {
-    maxw = std::max(maxw, hb.canvases[c].w);
-    rows += hb.canvases[c].h;
-  }
-  const uint64_t pieces = std::max<uint64_t>(1, (kTiles + rows - 1) / std::max<uint64_t>(rows, 1));
-  const uint32_t even = (uint32_t)std::max<uint64_t>(64, ((maxw + pieces - 1) / pieces + 31) & ~31ull);
-  return std::min(maxw, std::min(even, std::max<uint32_t>(32, std::min<uint32_t>(tile_w, 2048))));
+// The compositor's row tiles of the batch.
+static void BuildTiles(DeviceBatch& db) {
+  const uint32_t max_w = std::max<uint32_t>(32, std::min<uint32_t>(db.cfg.tile_w, 2048));
+  db.chunk = std::max(BuildBalancedTasks(db.hb, db.hb.main_canvases, max_w, db.h_tasks_main),
+                      BuildBalancedTasks(db.hb, db.hb.temp_canvases, max_w, db.h_tasks_temp));
 }
 
 int32_t UploadBatch(skity_cuda_context_s* ctx, DeviceBatch& db) {
@@ -116,9 +102,7 @@ int32_t UploadBatch(skity_cuda_context_s* ctx, DeviceBatch& db) {
     SKC_TRY(Upload(db.srgb_tables, tables, s));
   }
   SKC_TRY(Upload(db.temps, hb.temp_canvases, s));
-  db.chunk = TileWidth(hb, db.cfg.tile_w);
-  BuildRowTasks(hb, hb.main_canvases, db.chunk, db.h_tasks_main);
-  BuildRowTasks(hb, hb.temp_canvases, db.chunk, db.h_tasks_temp);
+  BuildTiles(db);
   SKC_TRY(Upload(db.tasks_main, db.h_tasks_main, s));
   SKC_TRY(Upload(db.tasks_temp, db.h_tasks_temp, s));
   if (int32_t rc = UploadDevicePlanInputs(ctx, db)) return rc;
@@ -142,9 +126,7 @@ int32_t ApplyConfig(skity_cuda_context_s* ctx, DeviceBatch& db, const RasterConf
   db.cfg = cfg;
   db.n_bands = AssignBands(hb, cfg.band_shift);
   SKC_TRY(Upload(db.canvases, hb.canvases, s));
-  db.chunk = TileWidth(hb, cfg.tile_w);
-  BuildRowTasks(hb, hb.main_canvases, db.chunk, db.h_tasks_main);
-  BuildRowTasks(hb, hb.temp_canvases, db.chunk, db.h_tasks_temp);
+  BuildTiles(db);
   if (int32_t rc = UploadDevicePlanInputs(ctx, db)) return rc;
   for (auto& g : db.graphs) {
     if (g) cudaGraphExecDestroy(g);

@@ -274,8 +274,9 @@ constexpr int kSortItems = 2048;
 
 // Key of item i: kind 0 the sweep of pass i (its form, then rows x (1 +
 // active-list bound): each form's launch takes its own passes, longest first,
-// so no warp of a CTA waits out a pass of another form), kind 1 compositor tile i (passes in its band's bin + 1) x its width; the
-// temp canvases' tiles (i >= n_main) sort after every main tile.
+// so no warp of a CTA waits out a pass of another form), kind 1 compositor
+// tile i (passes in its band's bin + 1) x (its width + kTileSpans); the temp
+// canvases' tiles (i >= n_main) sort after every main tile.
 __device__ __forceinline__ uint32_t SortKey(const DevBatch& b, const DevPlan& q, int kind,
                                             uint32_t i) {
   if (kind == 0) {
@@ -290,7 +291,7 @@ __device__ __forceinline__ uint32_t SortKey(const DevBatch& b, const DevPlan& q,
   const CanvasDesc& cd = b.canvases[t.canvas];
   const uint32_t band = cd.band0 + (t.y >> b.band_shift);
   const unsigned long long n = q.band_off[band + 1] - q.band_off[band];
-  const uint32_t k = WorkBucket<3>((n + 1ull) * (unsigned long long)(t.x1 - t.x0), kSortBuckets);
+  const uint32_t k = WorkBucket<3>((n + 1ull) * (unsigned long long)(t.x1 - t.x0 + kTileSpans), kSortBuckets);
   return i < q.n_main ? kSortBuckets + k : k;
 }
 

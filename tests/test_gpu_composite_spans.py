@@ -46,11 +46,17 @@ def test_spans_match_oracle(gpu_ctx, oracle_lib, width):
         assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
 
 
-# 36 rows make 64-pixel tiles above; with filler canvases of 1,200, 1,900 and
-# 4,000 rows beside them the tiles are a quarter, half and all of 1,025 wide
-@pytest.mark.parametrize("rows", [1200, 1900, 4000])
+# The canvases above are the whole batch and take 64-pixel tiles; beside a
+# filler of more work (60 draws on so many rows) theirs are wider, up to all of
+# their 1,025 pixels
+@pytest.mark.parametrize("rows", [4, 40, 400, 4000])
 def test_tile_widths_match_oracle(gpu_ctx, oracle_lib, rows):
-    filler = S.SceneBuilder(8, rows).build()
-    scenes = [bars_scene(1025, k) for k in range(3)]
-    for sc, got in zip(scenes, gpu_ctx.render_streams(scenes + [filler])):
+    b = S.SceneBuilder(900, rows)
+    for k in range(60):
+        p = S.default_paint()
+        p["fill_color"] = (0.1, 0.2, 0.3, 0.5)
+        b.draw_path([S.MOVE, S.LINE, S.LINE, S.LINE, S.CLOSE],
+                    [(0, 0), (900 - k, 0.5), (900 - k, rows), (3.3 * k, rows)], p)
+    scenes = [bars_scene(1025, k) for k in range(3)] + [b.build()]
+    for sc, got in zip(scenes, gpu_ctx.render_streams(scenes)):
         assert oracle_lib.compare(got, oracle_lib.render(sc)[0])["bad_pixels"] == 0
