@@ -3,19 +3,20 @@
 //   k_stroke     1 warp / pass   : stroked passes: Path -> QuadPath -> outline
 //   k_edges      1 warp / pass   : Path (or outline) -> QuadPath -> fixed-point
 //                                  edges -> introsort
-//   k_sweep_*    1 warp / pass   : analytic-AA sweep (register form, generic
-//                                  form for very long active lists) writing
-//                                  each row's spans contiguously into the
-//                                  span pool
+//   k_sweep_pair 2 warps / pass  : analytic-AA sweep, one walking, the other
+//   k_sweep      1 warp / pass     one writing each row's spans contiguously
+//                                  into the span pool; the generic form for
+//                                  very long active lists
 //   k_composite  1 warp / row tile: replays the spans of the row band's
 //                                  passes in draw order into a shared-memory
 //                                  tile, then writes the tile back
-//   k_blur_h/_v  1 thread / row / column of each blur temp canvas: StackBlur
+//   k_blur_h/_v  1 thread / channel of a row / column of each blur temp
+//                                  canvas: StackBlur
 //
 // The stroker and the sweeps are inherently sequential per path (the
 // reference's scanline sweep carries state across rows), so the parallelism
 // there is across paths; compositing is parallel across rows and, inside a row,
-// across pixels with a fixed lane per pixel column (no cross-lane hazards).
+// across the pixels of disjoint spans.
 #include <cuda_runtime.h>
 
 #include <algorithm>
