@@ -17,6 +17,13 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (GB300)")
 
 
+# A directory without the reference's sources is no checkout: the tests that
+# need one skip themselves where it does not exist.
+_reference = os.environ.get("SKITY_REFERENCE", "/root/reference")
+if not os.path.isdir(os.path.join(_reference, "src")):
+    os.environ["SKITY_REFERENCE"] = os.path.join(_reference, "src")
+
+
 def _cuda_include():
     for d in ("/usr/local/cuda/include", "/usr/local/cuda/targets/sbsa-linux/include",
               "/usr/local/cuda/targets/x86_64-linux/include"):
