@@ -283,9 +283,10 @@ __global__ void __launch_bounds__(32 * kCompWarps, kCompMinBlocks)
     k_composite(DevBatch b, const RowTask* __restrict__ tasks, uint32_t n_tasks, uint32_t chunk,
                 unsigned int* counter) {
   extern __shared__ __align__(16) uint8_t reg_smem[];
-  // a device plan that fell short: the host grows its buffers and renders
-  // again, so nothing is composited from it
-  if (b.plan && b.plan->flags) return;
+  // a device plan that fell short, or sweeps that ran out of span pool: the
+  // host grows the buffers and renders again, so nothing is composited (a
+  // canvas that keeps its pixels would get the spans there are twice)
+  if (b.plan && (b.plan->flags || *b.span_next > b.span_cap)) return;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   uint8_t* mine = reg_smem + (size_t)wib * CompWarpSmem(chunk);

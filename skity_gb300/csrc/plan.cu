@@ -408,7 +408,8 @@ int LaunchPlan(const DevBatch& b, const DevPlan& q, cudaStream_t s) {
     LaunchNext(k_scan2, 1, kScanThreads, s, q.a, q.r, np, &q.st->sweep_need, &q.st->rows_need);
     LaunchNext(k_plan_place, Blocks(np, kPlanThreads), kPlanThreads, s, b, q);
     n += 3 + LaunchSort(b, q, 0, np, kSweepKeys, s);
-  } else {
+  } else {  // what ClearCounters clears and the compositors read
+    cudaMemsetAsync(b.span_next, 0, 8, s);
     cudaMemsetAsync(b.task_next, 0, 8, s);
   }
   if (q.n_segs) {
