@@ -15,7 +15,6 @@
 #include <cstring>
 #include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -258,9 +257,10 @@ inline void RunParts(unsigned threads, uint32_t parts, F&& body) {
     }
   };
   std::vector<std::thread> pool;
-  try {
+  try {  // no thread or no memory for one: those there are take all parts
+    pool.reserve(threads);
     for (unsigned t = 1; t < threads; ++t) pool.emplace_back(work);
-  } catch (const std::system_error&) {
+  } catch (...) {
   }
   work();
   for (auto& t : pool) t.join();
