@@ -1928,6 +1928,13 @@ inline void SweepOrder(const std::vector<PassGeom>& geom, std::vector<uint32_t>&
   std::stable_sort(order.begin(), order.end(),
                    [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
 }
+// The geometry slice of a pass at `at` in the scratch; returns its end.
+inline uint64_t PlaceSlice(PassDesc& pd, uint64_t at) {
+  SliceLayout L;
+  L.compute(pd.cap, sizeof(Edge));
+  pd.slice_off = at;
+  return at + L.bytes;
+}
 // Grow the capacities of a pass whose geometry overflowed.
 inline void GrowCaps(PassDesc& pd, const PassGeom& g) {
   bool stroke = (pd.flags & kPassStroke) != 0;

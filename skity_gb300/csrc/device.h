@@ -41,6 +41,16 @@ struct DevBuf {
   T* as() const { return (T*)p; }
 };
 
+// `v` to the start of `d`, grown to hold it.
+template <typename T>
+cudaError_t Upload(DevBuf& d, const std::vector<T>& v, cudaStream_t s) {
+  cudaError_t e = d.ensure(std::max<size_t>(v.size() * sizeof(T), 16));
+  if (e != cudaSuccess || v.empty()) return e;
+  return cudaMemcpyAsync(d.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s);
+}
+
+int32_t CudaErr(cudaError_t e);
+
 struct Context;
 
 // Launch shape of the compositor and the granularity of its pass bins
@@ -123,8 +133,45 @@ struct DeviceBatch {
     keep_pixels = false;
     uploaded = false;
     slices_dirty = true;
+    slices_end = 0;
     cap_sweep = cap_rows = cap_bins = 0;
     stats = skity_cuda_stats{};
+  }
+  // Lays the passes' geometry slices out in `scratch`, one behind the other,
+  // unless they stand, with room behind them for those that outgrow their
+  // estimate.  Every renderer that keeps them for the next one does it here:
+  // GrowSlices goes on where they end.
+  int32_t LayoutSlices(uint64_t budget, cudaStream_t s) {
+    if (!slices_dirty) return SKITY_CUDA_SUCCESS;
+    uint64_t total = 0;
+    for (PassDesc& pd : hb.passes) total = PlaceSlice(pd, total);
+    if (budget && total > budget) return SKITY_CUDA_ERROR_OUT_OF_DEVICE_MEMORY;
+    uint64_t want = total + total / 32 + (1u << 20);
+    if (budget) want = std::max(total, std::min(want, budget));
+    cudaError_t e = scratch.ensure(want);
+    if (e == cudaSuccess) e = Upload(passes, hb.passes, s);
+    if (e != cudaSuccess) return CudaErr(e);
+    slices_dirty = false;
+    slices_end = total;
+    return SKITY_CUDA_SUCCESS;
+  }
+  // The passes whose geometry (h_geom) outgrew their slices get new ones
+  // behind the others, and only they (`todo`) are to run again; without room
+  // there, all slices are to be laid out again (slices_dirty).
+  int32_t GrowSlices(std::vector<uint32_t>& todo, cudaStream_t s) {
+    uint64_t end = slices_end;
+    for (uint32_t p = 0; p < (uint32_t)hb.passes.size(); ++p) {
+      if (!h_geom[p].status) continue;
+      GrowCaps(hb.passes[p], h_geom[p]);
+      end = PlaceSlice(hb.passes[p], end);
+      todo.push_back(p);
+    }
+    slices_dirty = true;
+    if (end > scratch.cap) return SKITY_CUDA_SUCCESS;
+    if (cudaError_t e = Upload(passes, hb.passes, s)) return CudaErr(e);
+    slices_dirty = false;
+    slices_end = end;
+    return SKITY_CUDA_SUCCESS;
   }
   std::vector<PassGeom> h_geom;
   skity_cuda_stats stats{};
@@ -156,7 +203,6 @@ struct skity_cuda_context_s {
 
 namespace skc {
 
-int32_t CudaErr(cudaError_t e);
 // Parses scene streams into the batch's host description.
 int32_t BuildFromStreams(DeviceBatch& db, uint32_t count, const uint8_t* const* streams,
                          const size_t* bytes);

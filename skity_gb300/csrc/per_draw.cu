@@ -176,22 +176,7 @@ int32_t RenderPerDraw(skity_cuda_context_s* ctx, DeviceBatch& db) {
   uint64_t cap_rows = 2ull * maxh;
   DevBuf status, sweepmem, rowspan;
   for (int attempt = 0; attempt < 8; ++attempt) {
-    if (db.slices_dirty) {
-      uint64_t total = 0;
-      for (uint32_t i = 0; i < np; ++i) {
-        SliceLayout L;
-        L.compute(hb.passes[i].cap, sizeof(Edge));
-        hb.passes[i].slice_off = total;
-        total += L.bytes;
-      }
-      if (ctx->budget && total > ctx->budget) return SKITY_CUDA_ERROR_OUT_OF_DEVICE_MEMORY;
-      SKC_TRY_RC(db.scratch.ensure(std::max<uint64_t>(total, 16)));
-      SKC_TRY_RC(db.passes.ensure(npm * sizeof(PassDesc)));
-      if (np)
-        SKC_TRY_RC(cudaMemcpyAsync(db.passes.p, hb.passes.data(), np * sizeof(PassDesc),
-                                   cudaMemcpyHostToDevice, s));
-      db.slices_dirty = false;
-    }
+    if (int32_t rc = db.LayoutSlices(ctx->budget, s)) return rc;
     SKC_TRY_RC(db.geom.ensure(npm * sizeof(PassGeom)));
     SKC_TRY_RC(db.sweep.ensure(npm * sizeof(PassSweep)));
     SKC_TRY_RC(db.comp.ensure(npm * sizeof(PassComp)));

@@ -43,13 +43,6 @@ int32_t CudaErr(cudaError_t e) {
     if (_e != cudaSuccess) return CudaErr(_e);     \
   } while (0)
 
-template <typename T>
-static cudaError_t Upload(DevBuf& d, const std::vector<T>& v, cudaStream_t s) {
-  cudaError_t e = d.ensure(std::max<size_t>(v.size() * sizeof(T), 16));
-  if (e != cudaSuccess || v.empty()) return e;
-  return cudaMemcpyAsync(d.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s);
-}
-
 // Inputs of the device planner that depend only on the canvases, their
 // passes and the raster config: the compositor's tiles (main canvases, then
 // the temp canvases) and the pass-bin segments.
@@ -281,23 +274,7 @@ static int32_t PrepareDevice(skity_cuda_context_s* ctx, DeviceBatch& db, DevBatc
   cudaStream_t s = ctx->stream;
   const uint32_t np = (uint32_t)hb.passes.size();
   const size_t npm = std::max<size_t>(np, 1);
-  if (db.slices_dirty) {
-    uint64_t total = 0;
-    for (uint32_t i = 0; i < np; ++i) {
-      SliceLayout L;
-      L.compute(hb.passes[i].cap, sizeof(Edge));
-      hb.passes[i].slice_off = total;
-      total += L.bytes;
-    }
-    if (ctx->budget && total > ctx->budget) return SKITY_CUDA_ERROR_OUT_OF_DEVICE_MEMORY;
-    // with room behind the slices for those that outgrow their estimate
-    uint64_t want = total + total / 32 + (1u << 20);
-    if (ctx->budget) want = std::max(total, std::min(want, ctx->budget));
-    SKC_TRY(db.scratch.ensure(want));
-    SKC_TRY(Upload(db.passes, hb.passes, s));
-    db.slices_dirty = false;
-    db.slices_end = total;
-  }
+  if (int32_t rc = db.LayoutSlices(ctx->budget, s)) return rc;
   SKC_TRY(db.geom.ensure(npm * sizeof(PassGeom)));
   SKC_TRY(db.sweep.ensure(npm * sizeof(PassSweep)));
   SKC_TRY(db.comp.ensure(npm * sizeof(PassComp)));
@@ -565,27 +542,11 @@ static int32_t DeviceRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool tim
     todo.clear();
     all = false;
     if (ps.flags & kPlanGeomOverflow) {
-      // the passes that outgrew their slices get new ones behind the others,
-      // and only they run again; without room there, all slices move
       db.h_geom.resize(np);
       SKC_TRY(cudaMemcpy(db.h_geom.data(), db.geom.p, (size_t)np * sizeof(PassGeom),
                          cudaMemcpyDeviceToHost));
-      uint64_t end = db.slices_end;
-      for (uint32_t p = 0; p < np; ++p) {
-        if (!db.h_geom[p].status) continue;
-        GrowCaps(hb.passes[p], db.h_geom[p]);
-        SliceLayout L;
-        L.compute(hb.passes[p].cap, sizeof(Edge));
-        hb.passes[p].slice_off = end;
-        end += L.bytes;
-        todo.push_back(p);
-      }
-      if (end <= db.scratch.cap) {
-        db.slices_end = end;
-        SKC_TRY(Upload(db.passes, hb.passes, s));
-      } else {
-        all = db.slices_dirty = true;
-      }
+      if (int32_t grow_rc = db.GrowSlices(todo, s)) return grow_rc;
+      all = db.slices_dirty;
     }
     if (ps.sweep_need > db.cap_sweep) db.cap_sweep = ps.sweep_need + ps.sweep_need / 8;
     if (ps.rows_need > db.cap_rows) db.cap_rows = ps.rows_need + ps.rows_need / 8;
@@ -671,12 +632,7 @@ static int32_t PlanAndRender(skity_cuda_context_s* ctx, DeviceBatch& db, bool ti
   SKC_TRY(db.geom.ensure(std::max<size_t>(np, 1) * sizeof(PassGeom)));
   for (int attempt = 0; attempt < 8 && !todo.empty(); ++attempt) {
     uint64_t total = 0;
-    for (uint32_t i = 0; i < np; ++i) {
-      SliceLayout L;
-      L.compute(hb.passes[i].cap, sizeof(Edge));
-      hb.passes[i].slice_off = total;
-      total += L.bytes;
-    }
+    for (PassDesc& pd : hb.passes) total = PlaceSlice(pd, total);
     if (ctx->budget && total > ctx->budget) return SKITY_CUDA_ERROR_OUT_OF_DEVICE_MEMORY;
     SKC_TRY(db.scratch.ensure(std::max<uint64_t>(total, 16)));
     SKC_TRY(Upload(db.passes, hb.passes, s));
