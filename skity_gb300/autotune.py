@@ -3,15 +3,16 @@
 The pixels never depend on the configuration (skity_cuda_raster_config);
 only the time does.  The searched space:
 
-* row-tile width in pixels {128, 256, 512, 1024, 2048} -- the compositor gives each
-  warp one canvas row segment, so a tile is (width x 1 row) and its width,
-  a multiple of the 32 lanes, is the shape parameter;
+* widest row tile in pixels {128, 256, 512, 1024, 2048} -- the compositor gives
+  each warp one canvas row segment, so a tile is (width x 1 row); tiles that
+  would be more than a warp's share of the batch's work are narrower anyway
+  (skity_cuda_raster_config), so widths above the widest of those time alike;
 * persistent CTAs per SM {1, 2, 4, 6, 8} (the grid is that many CTAs per SM,
   pulling tiles from a work counter in most-work-first order);
 * pass-bin granularity: bands of {8, 16, 32} rows;
-* warps per CTA of the register-resident AAA sweeps {1, 2, 4} (one pass a
-  warp; fewer warps a CTA spread a batch's few long passes over more SMs,
-  more warps share one CTA's launch and shared-memory carve-out).
+* warps per CTA of the register-resident AAA sweeps {2, 4} (two warps a pass;
+  one pass a CTA spreads a batch's few long passes over more SMs, two share
+  one CTA's launch and shared-memory carve-out; 1 is the launch of 2).
 
 Tile width x CTAs per SM are swept together on the compositing time, then
 the band height with the best pair on the same time, then the sweep's warps
@@ -29,7 +30,7 @@ import os
 TILE_WIDTHS = (128, 256, 512, 1024, 2048)
 CTAS_PER_SM = (1, 2, 4, 6, 8)
 BAND_ROWS = (8, 16, 32)
-SWEEP_WARPS = (1, 2, 4)
+SWEEP_WARPS = (2, 4)
 
 
 def cache_path() -> str:
