@@ -15,6 +15,7 @@
 #include <cstring>
 #include <exception>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -265,6 +266,17 @@ inline void RunParts(unsigned threads, uint32_t parts, F&& body) {
   work();
   for (auto& t : pool) t.join();
   if (thrown) std::rethrow_exception(thrown);
+}
+
+// The status of `build`, out of host memory as one: the C entries let no
+// exception out.
+template <typename F>
+inline int32_t BuildStatus(F&& build) {
+  try {
+    return build();
+  } catch (const std::bad_alloc&) {
+    return SKITY_CUDA_ERROR_OUT_OF_HOST_MEMORY;
+  }
 }
 
 // Host threads for a stream of `verbs` verbs: 16384 verbs (0.4 to 0.6 ms of

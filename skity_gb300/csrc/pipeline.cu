@@ -863,7 +863,8 @@ static unsigned BuildThreads() {
 
 int32_t BuildFromStreams(DeviceBatch& db, uint32_t count, const uint8_t* const* streams,
                                 const size_t* bytes) {
-  return BuildStreams(db.hb, count, streams, bytes, BuildThreads());
+  return BuildStatus(
+      [&] { return BuildStreams(db.hb, count, streams, bytes, BuildThreads()); });
 }
 
 int32_t ReadCanvas(skity_cuda_context_s* ctx, DeviceBatch& db, uint32_t index, uint8_t* out,
@@ -2095,7 +2096,8 @@ SKITY_CUDA_API int32_t skity_cuda_canvas_flush(skity_cuda_canvas canvas) {
   sv.matrices = canvas->any_matrix ? canvas->matrices.data() : nullptr;
   skc::DeviceBatch& db = canvas->db;
   db.Reset();  // other draws than the last flush's: their passes are uploaded again
-  int32_t rc = skc::AddStreamCanvas(db.hb, sv, skc::BuildThreads());
+  int32_t rc =
+      skc::BuildStatus([&] { return skc::AddStreamCanvas(db.hb, sv, skc::BuildThreads()); });
   if (rc) return rc;
   rc = skc::UploadBatch(ctx, db);
   if (rc) return rc;
