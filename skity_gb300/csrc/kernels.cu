@@ -171,7 +171,10 @@ __global__ void __launch_bounds__(128, kPairsPerSm<M> / 2) k_sweep_pair(DevBatch
 }
 
 // The passes the register forms gave up on, swept with the generic form after
-// every register form has finished (a plain launch after them).
+// every register form has finished (a plain launch after them).  The last CTA
+// marks the plan of a render whose sweeps ran out of span pool: the compositor
+// then has one word to look at (reading the pool's counter there changed its
+// register allocation: 1,500 paths with gradients 3.72 -> 3.82 ms).
 __global__ void __launch_bounds__(32 * kSweepWarps) k_sweep_retry(DevBatch b) {
   if (!b.sweep_retry) return;
   const uint32_t n = min(b.sweep_retry[0], b.n_passes);
@@ -180,6 +183,14 @@ __global__ void __launch_bounds__(32 * kSweepWarps) k_sweep_retry(DevBatch b) {
   L.lane = threadIdx.x & 31;
   for (uint32_t i = blockIdx.x * kSweepWarps + (threadIdx.x >> 5); i < n; i += nw)
     SweepPass(b, b.sweep_retry[1 + i], L);
+  if (!b.plan) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(b.sweep_done + kSweepForms, 1u) == gridDim.x - 1 &&
+        *(volatile unsigned long long*)b.span_next > b.span_cap)
+      atomicOr(&b.plan->flags, (uint32_t)kPlanSpans);
+  }
 }
 
 template <bool kRaw>
@@ -286,7 +297,7 @@ __global__ void __launch_bounds__(32 * kCompWarps, kCompMinBlocks)
   // a device plan that fell short, or sweeps that ran out of span pool: the
   // host grows the buffers and renders again, so nothing is composited (a
   // canvas that keeps its pixels would get the spans there are twice)
-  if (b.plan && (b.plan->flags || *b.span_next > b.span_cap)) return;
+  if (b.plan && b.plan->flags) return;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   uint8_t* mine = reg_smem + (size_t)wib * CompWarpSmem(chunk);

@@ -225,8 +225,8 @@ struct DevBatch {
   uint32_t* sweep_retry;     // [0]: passes the register sweeps gave up on (zeroed before the
                              // sweeps), [1, n_passes]: their indices
   unsigned int* task_next;   // persistent compositor's work counters (temp, main)
-  unsigned int* sweep_done;  // per sweep form, CTAs finished (zeroed before the sweeps);
-                             // null: the forms' launches do not overlap
+  unsigned int* sweep_done;  // per sweep form, then k_sweep_retry's, CTAs finished (zeroed
+                             // before the sweeps); null: the forms' launches do not overlap
   // path clips
   const ClipStateDesc* clip_states;  // [n_clip_states]
   uint32_t n_clip_states;
@@ -239,7 +239,7 @@ struct DevBatch {
   uint32_t any_general;
   // device-planned renders: the plan's status (null for host-planned
   // ones); the compositor writes nothing when a plan buffer fell short
-  const struct PlanStatus* plan;
+  struct PlanStatus* plan;
 };
 
 // Spans per pool chunk for a pass: a power of two holding any one row of it.
@@ -267,6 +267,7 @@ enum : uint32_t {
   kPlanSweepMem = 2,      // sweep memory short
   kPlanRows = 4,          // row-span table short
   kPlanBins = 8,          // pass bins short
+  kPlanSpans = 16,        // span pool short (known after the sweeps)
 };
 
 struct PlanStatus {  // zeroed before each render, read back after it

@@ -108,7 +108,7 @@ int32_t UploadBatch(skity_cuda_context_s* ctx, DeviceBatch& db) {
   for (const HostBatch::ImageUpload& u : hb.image_uploads)  // the draws' images
     SKC_TRY(cudaMemcpyAsync(db.pixels.as<uint8_t>() + u.off, u.bytes.data(), u.bytes.size(),
                             cudaMemcpyHostToDevice, s));
-  SKC_TRY(db.task_next.ensure(32));
+  SKC_TRY(db.task_next.ensure(4 * (2 + kSweepForms + 1)));
   db.uploaded = true;
   return SKITY_CUDA_SUCCESS;
 }
@@ -292,7 +292,7 @@ static int32_t PrepareDevice(skity_cuda_context_s* ctx, DeviceBatch& db, DevBatc
   SKC_TRY(db.band_off.ensure(((size_t)db.n_bands + 1) * 4));
   const size_t nt = db.h_tasks_main.size() + db.h_tasks_temp.size();
   SKC_TRY(db.tasks_sorted.ensure(std::max<size_t>(nt, 1) * sizeof(RowTask)));
-  SKC_TRY(db.task_next.ensure(32));
+  SKC_TRY(db.task_next.ensure(4 * (2 + kSweepForms + 1)));
   SKC_TRY(ctx->span_next.ensure(8));
   {
     // bucket sorts: a key per item, 1024 counts per block of 2048 items

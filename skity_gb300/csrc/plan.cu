@@ -75,7 +75,7 @@ __device__ __forceinline__ uint32_t WorkBucket(unsigned long long c, uint32_t bu
 __device__ __forceinline__ void ClearCounters(const DevBatch& b) {
   *b.span_next = 0;
   b.sweep_retry[0] = 0;
-  for (int k = 0; k < kSweepForms; ++k) b.sweep_done[k] = 0;
+  for (int k = 0; k <= kSweepForms; ++k) b.sweep_done[k] = 0;
   b.task_next[0] = b.task_next[1] = 0;
 }
 
@@ -408,8 +408,7 @@ int LaunchPlan(const DevBatch& b, const DevPlan& q, cudaStream_t s) {
     LaunchNext(k_scan2, 1, kScanThreads, s, q.a, q.r, np, &q.st->sweep_need, &q.st->rows_need);
     LaunchNext(k_plan_place, Blocks(np, kPlanThreads), kPlanThreads, s, b, q);
     n += 3 + LaunchSort(b, q, 0, np, kSweepKeys, s);
-  } else {  // what ClearCounters clears and the compositors read
-    cudaMemsetAsync(b.span_next, 0, 8, s);
+  } else {
     cudaMemsetAsync(b.task_next, 0, 8, s);
   }
   if (q.n_segs) {

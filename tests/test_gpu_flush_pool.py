@@ -50,7 +50,7 @@ def test_every_draw_lands_once(gpu_ctx, oracle_lib, draws, blend, blur, short):
 
 
 def test_empty_canvases_in_a_new_context(gpu_ctx):
-    """Nothing to sweep: the pool's counter is clear all the same."""
+    """A plan without passes falls short of nothing, in a context without a pool."""
     ctx = Context(0)
     scenes = [S.SceneBuilder(40 + i, 30, clear=(1.0, 0.5, 0.0, 1.0)).build() for i in range(3)]
     for _ in range(2):
