@@ -1,8 +1,9 @@
 // The geometry of one pass on one warp: Path -> QuadPath (-> stroke ->
 // QuadPath) -> bounds -> fixed-point edges -> sort, with the lanes on
-// different verbs, edges and sort positions.  Every stage gives what the
-// one-thread functions of geom.cuh and raster.cuh give (on the CPU the lanes
-// are one thread); only the stroker walks its path in order, on one lane.
+// different verbs, runs of a contour's segments, edges and sort positions.
+// Every stage gives what the one-thread functions of geom.cuh, stroke.cuh and
+// raster.cuh give (on the CPU the lanes are one thread); paths that are not
+// regular (RegularVerb) go through those on one lane.
 #pragma once
 #include "kernels.cuh"
 #include "stroke.cuh"

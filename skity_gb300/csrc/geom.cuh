@@ -423,8 +423,9 @@ SKC_HD double CubicQuadCountD(const P c[4]) {
   P d = mkP(p2x2.x - p1x2.x, p2x2.y - p1x2.y);
   float err = d.x * d.x + d.y * d.y;
   // The ceiling is known from a float power unless that is close to a whole
-  // number (double arithmetic runs at 1/64 of the float rate): exp2f and
-  // log2f are within 4e-7 of it for these exponents.
+  // number (double arithmetic runs at 1/64 of the float rate): by way of exp2f
+  // and log2f it is within 2e-6 of it (a unit in the last place of a logarithm
+  // of up to 65 is 8e-6, a sixth of that in the exponent), against a slack of 1e-4.
   if (err > 1e-20f && err < 1e20f) {
     const float v = exp2f(log2f(err * (float)(1.0 / max_hypot2)) * (1.0f / 6.0f));
     const float c = ceil_(v), slack = 1e-4f * c;

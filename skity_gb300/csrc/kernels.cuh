@@ -132,7 +132,8 @@ struct PassGeom {
 
 // Which sweep form takes pass p: the register form for up to 32, 64 or 128
 // active edges, or the generic form, by the geometry's bound of the active
-// list (PassGeom::max_active); pass_class != 0 forces the generic form.
+// list (PassGeom::max_active).  A pass_class other than 0 is the form itself
+// (kSweepGeneric) or kSweepSkip.  SweepLaunch adds the form for 129 to 256.
 // The forms' kernels take disjoint passes and depend on nothing the others
 // write, so their launches may overlap.
 constexpr int kRegMaxM = 128;  // the largest active list held in registers
@@ -215,8 +216,8 @@ struct DevBatch {
   const uint32_t* pass_list;  // passes to (re)run in the geometry kernels
   uint32_t n_list;
   uint32_t any_stroke;  // a pass is stroked: the stroker's kernel runs
-  uint8_t* pass_class;  // sweep form per pass: 0 register sweep, 1 generic
-  int32_t reg_diff_cap; // accumulator entries per warp in shared memory
+  uint8_t* pass_class;  // per pass: 0 (the form by its bound), a form, or kSweepSkip
+  int32_t reg_diff_cap; // accumulator entries per pass in shared memory
   const uint32_t* band_off;  // per band: first entry in bins (one past the end follows)
   const uint32_t* bins;      // pass indices, per band in draw order
   const uint32_t* sweep_order;  // passes in the order the sweeps take them (null: index order)
@@ -318,9 +319,9 @@ int LaunchPlan(const DevBatch& b, const DevPlan& q, cudaStream_t stream);
 // Work totals of the render into the plan status.
 int LaunchPlanStats(const DevBatch& b, const DevPlan& q, cudaStream_t stream);
 
-// Shared memory of one register-sweep warp: its RegSharedT block, then an
-// accumulator of reg_diff_cap entries (passes with wider accumulators keep
-// theirs in the pass's sweep memory).
+// Shared memory of a pass in a register form: the pair's RegPairT block, then
+// an accumulator of up to reg_diff_cap entries (PairDiffCap; passes with wider
+// accumulators keep theirs in the pass's sweep memory).
 constexpr int32_t kRegDiffMax = 3072;
 
 // kernel launchers (kernels.cu); all launch on `stream` and return the
@@ -340,6 +341,5 @@ int LaunchComposite(const DevBatch& b, const RowTask* tasks, uint32_t n_tasks, u
 // runs only when one is not kNormal)
 int LaunchBlur(const DevBatch& b, const uint32_t* temp_canvases, uint32_t n_temp,
                uint32_t max_h, uint32_t max_w, uint32_t max_style, cudaStream_t stream);
-int LaunchClearCanvases(const DevBatch& b, const uint32_t* canvases, uint32_t n, cudaStream_t stream);
 
 }  // namespace skc

@@ -6,8 +6,8 @@
 //   k_plan_place    1 thread / pass : PassSweep, PassComp, sweep form, band
 //                                     range
 //   k_sort_*        sweep order     : passes by sweep form, then by expected
-//                                     sweep length, longest first (stable
-//                                     bucket sort)
+//                                     sweep length, longest first (bucket
+//                                     sort)
 //   k_bin_count     1 warp / segment: passes meeting a band (warp ballots)
 //   k_scan2         1 block         : segment offsets
 //   k_bin_fill      1 warp / segment: the bins, draw order kept by ballot ranks
@@ -58,8 +58,8 @@ __device__ __forceinline__ void PassNeeds(const PassGeom& g, unsigned long long*
 // order to within 19% (2 bits).
 constexpr uint32_t kSortBuckets = 512;    // of a work estimate, tiles
 constexpr uint32_t kSweepBuckets = 128;   // of a work estimate, sweeps
-// the sweep order's keys: kSweepBuckets per form, the forms in the order of
-// kFormRank (the passes no form takes last)
+// the sweep order's keys: kSweepBuckets per form, the higher form numbers
+// first and the passes no form takes last
 constexpr uint32_t kSweepKeys = (kSweepForms + 1) * kSweepBuckets;
 template <uint32_t kBits>
 __device__ __forceinline__ uint32_t WorkBucket(unsigned long long c, uint32_t buckets) {
